@@ -831,6 +831,8 @@ kz_status kz_scene_build(kz_scene* s) {
 
     cudaStream_t st = s->stream;
     KZ_TRY(upload(s->nodes, out.nodes, st));
+    kz::launch_pack_nodes(s->nodes.as<uint4>(), out.n_nodes, st);
+    KZ_CUDA(cudaGetLastError());
     KZ_TRY(upload(s->tris, out.tris, st));
     KZ_TRY(upload(s->geom_offset, goff, st));
     KZ_TRY(upload(s->geom_light, glight, st));

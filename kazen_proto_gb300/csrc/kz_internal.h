@@ -169,6 +169,8 @@ struct BatchCounters {
 };
 
 // ---- launchers (kz_kernels.cu) -------------------------------------------
+// Nodes as the builder writes them to the layout the traversal reads, in place.
+void launch_pack_nodes(uint4* nodes, uint32_t n, cudaStream_t st);
 // `next` is a zeroed 64-bit fetch counter for the persistent kernel.
 void launch_intersect_closest(const DevScene& s, const kz_ray* rays, uint64_t n, kz_hits hits,
                               unsigned long long* next, uint32_t* status, cudaStream_t st);

@@ -110,12 +110,6 @@ __device__ __forceinline__ void warp_count(uint32_t a, uint32_t b, unsigned long
     }
 }
 
-// Leaf triangles of the persistent kernels tested warp-wide
-// (persistent_rays_shared) rather than per lane (persistent_rays).
-#ifndef KZ_SHARE_LEAVES
-#define KZ_SHARE_LEAVES 1
-#endif
-
 // Shared memory of the persistent traversal loops: the closest-hit loop's
 // first stack entries and warp-shared leaf arrays, and the any-hit loop's
 // leaf arrays (blocks of 256 threads). A kernel that runs both loops one
@@ -126,6 +120,7 @@ struct ClosestSmem {
     unsigned long long key[256];
     uint32_t rec[256];
     float4 vwdt[256];
+    uint4 ent[kClosestSteps * 256];
 };
 // KZ_ANY_SMEM_STACK: the any-hit loop's first stack entries in shared memory
 // (off: the terrain frame's shadow stage measured 29.1 ms with 4 or 8 entries
@@ -137,14 +132,17 @@ struct AnySmem {
     float4 ray[2 * 256];
     unsigned long long key[256];
     uint32_t rec[256];
+    uint4 ent[kAnySteps * 256];
 #if KZ_ANY_SMEM_STACK > 0 && KZ_ANY_SMEM_STACK < KZ_WIDE_STACK
     uint2 stack[KZ_ANY_SMEM_STACK * 256];
 #endif
 };
 
-// Closest hit of ray k through persistent_rays: load(k, r, tmax) sets the
-// ray up, store(k, hit) writes the result; m is the block's shared memory.
-// `s` is the lane's scene; load may repoint it per ray (batched jobs: kOwnScene).
+// Closest hit of ray k through persistent_rays_shared: load(k, r, tmax) sets
+// the ray up, store(k, hit) writes the result; m is the block's shared memory.
+// `s` is the lane's scene; load may repoint it per ray (batched jobs:
+// kOwnScene). The fetch-counting variant keeps one node per step, so that its
+// counts are those of a sequential traversal.
 template <bool kCount, bool kOwnScene, typename Ctr, typename Load, typename Store>
 __device__ __forceinline__ void persistent_closest_in(ClosestSmem& m, DevScene& s, Ctr n, Ctr* next,
                                                       uint32_t* status, Load load, Store store, uint32_t& dn,
@@ -156,59 +154,38 @@ __device__ __forceinline__ void persistent_closest_in(ClosestSmem& m, DevScene& 
     uint2 stack_lm[kWideStack];
     const LocalStack stack{stack_lm};
 #endif
-#if KZ_SHARE_LEAVES
-    const LeafShare sh{m.ray, m.key, m.rec, m.vwdt};
-    ClosestState c;
+    constexpr int K = kCount ? 1 : kClosestSteps;
+    const LeafShare sh{m.ray, m.key, m.rec, m.vwdt, m.ent};
+    AnyState c;
     TRay r;
-    float tmax = 0.f;
-    uint32_t octp = 0;
+    WideDir dir;
+    float tmax = 0.f, tcur = 0.f;
     Ctr ray = 0;
-    persistent_rays_shared(
+    persistent_rays_shared<K>(
         n, next, kTraceRefill,
         [&](Ctr k) {
             ray = k;
             load(k, r, tmax);
-            octp = wide_octant(r);
-            closest_begin(c, tmax);
+            dir = wide_dir(r);
+            any_begin(c);
+            tcur = tmax;
             publish_ray(sh, r);
+            best_begin(sh, tmax);
         },
-        [&](uint32_t& tbits, uint32_t& tbase) {
-            return closest_node<kCount>(s, r, octp, c, stack, tbits, tbase, dn, dt);
+        [&](LeafGroup& lg) {
+            if (visit_node<kCount>(s, r, dir, tcur, c, stack, lg, dn) < 0) return -1;
+            if (kCount) dt += __popc(lg.bits);
+            return group_pop(c, stack);
         },
-        [&](uint32_t tbits, uint32_t tbase) { closest_leaves<kOwnScene>(sh, s.tris, tbits, tbase, c); },
+        [&](const LeafGroup(&g)[K]) { closest_leaves<kOwnScene>(sh, s.tris, g, tcur); },
         [&](int rc) {
-            if (rc == 0) rc = group_pop(c, stack);
             if (rc == 0) return false;
             HitRec h;
-            closest_finish(c, rc > 0, tmax, h);
+            best_finish(sh, rc > 0, tmax, h);
             if (rc < 0) set_status(status, KZ_ERR_STACK);
             store(ray, h);
             return true;
         });
-#else
-    ClosestState c;
-    TRay r;
-    float tmax = 0.f;
-    uint32_t octp = 0;
-    Ctr ray = 0;
-    persistent_rays(
-        n, next, kTraceRefill,
-        [&](Ctr k) {
-            ray = k;
-            load(k, r, tmax);
-            octp = wide_octant(r);
-            closest_begin(c, tmax);
-        },
-        [&]() {
-            const int rc = closest_step<kCount>(s, r, octp, c, stack, dn, dt);
-            if (rc == 0) return false;
-            HitRec h;
-            closest_finish(c, rc > 0, tmax, h);
-            if (rc < 0) set_status(status, KZ_ERR_STACK);
-            store(ray, h);
-            return true;
-        });
-#endif
 }
 
 // The same with the block's own static shared memory.
@@ -231,33 +208,35 @@ __device__ __forceinline__ void persistent_any_in(AnySmem& m, DevScene& s, Ctr n
     uint2 stack_lm[kWideStack];
     const LocalStack stack{stack_lm};
 #endif
-    const LeafShare sh{m.ray, m.key, m.rec, nullptr};
+    constexpr int K = kCount ? 1 : kAnySteps;
+    const LeafShare sh{m.ray, m.key, m.rec, nullptr, m.ent};
     AnyState c;
     TRay r;
+    WideDir dir;
     float tmax = 0.f;
-    uint32_t octp = 0;
     Ctr ray = 0;
     bool hit = false;
-    persistent_rays_shared(
+    persistent_rays_shared<K>(
         n, next, kAnyRefill,
         [&](Ctr k) {
             ray = k;
             load(k, r, tmax);
-            octp = wide_octant(r);
+            dir = wide_dir(r);
             any_begin(c);
             publish_ray(sh, r);
             publish_tmax(sh, tmax);
         },
-        [&](uint32_t& tbits, uint32_t& tbase) {
-            return any_node<kCount>(s, r, octp, tmax, c, stack, tbits, tbase, dn, dt);
+        [&](LeafGroup& lg) {
+            if (visit_node<kCount>(s, r, dir, tmax, c, stack, lg, dn) < 0) return -1;
+            return group_pop(c, stack);
         },
-        [&](uint32_t tbits, uint32_t tbase) {
-            const uint32_t hits = any_leaves<kOwnScene>(sh, s.tris, tbits, tbase);
+        [&](const LeafGroup(&g)[K]) {
+            const uint32_t hits = any_leaves<kOwnScene>(sh, s.tris, g);
             hit = hits != 0u;
-            if (kCount) dt += any_tested(tbits, hits);
+            if (kCount) dt += any_tested(g[0].bits, hits);
         },
         [&](int rc) {
-            if (rc == 0) rc = hit ? 2 : group_pop(c, stack);
+            if (hit && rc >= 0) rc = 2;
             if (rc == 0) return false;
             done(ray, rc);
             return true;

@@ -13,6 +13,31 @@
 namespace kz {
 namespace {
 
+// A node of the builder's layout (kz_bvh.h) to the traversal's (WideAxis,
+// kz_traverse.cuh), in place; the same boxes, children and records.
+__global__ void k_pack_nodes(uint4* nodes, uint32_t n) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    uint4* p = nodes + (size_t)i * 5;
+    const uint4 h0 = p[0], h1 = p[1];
+    uint32_t valid = 0;
+#pragma unroll
+    for (int s = 0; s < 8; ++s) {
+        const uint32_t m = ((s < 4 ? h1.z : h1.w) >> (8 * (s & 3))) & 0xFFu;
+        if (!((h0.w >> (24 + s)) & 1u)) valid |= (m >> 5) << (3 * s);
+    }
+    const auto scale = [&](int a) { return (((h0.w >> (8 * a)) & 0xFFu) + 15u) << 7; };
+    p[0].w = scale(0) | scale(1) << 16;
+    p[1].z = valid | (h0.w & 0xFF000000u);
+    p[1].w = scale(2);
+#pragma unroll
+    for (int a = 2; a < 5; ++a) {
+        const uint4 q = p[a];  // low planes of slots 0-3, 4-7, high planes of slots 0-3, 4-7
+        p[a] = make_uint4(__byte_perm(q.x, q.z, 0x5140), __byte_perm(q.x, q.z, 0x7362),
+                          __byte_perm(q.y, q.w, 0x5140), __byte_perm(q.y, q.w, 0x7362));
+    }
+}
+
 // kz_intersect_any: rays (o, tmin, d, tmax) in, an occlusion byte out.
 __global__ void __launch_bounds__(256, KZ_TRACE_MINB) k_intersect_any_persistent(DevScene s,
                                                                                  const kz_ray* __restrict__ rays,
@@ -149,7 +174,6 @@ __global__ void __launch_bounds__(256, KZ_TRACE_MINB) k_trace_shadow_persistent(
             if (nee) nee[rb + (tag & 15u)].n.w = 1.f;
         }
     };
-#if KZ_SHARE_LEAVES
     persistent_any<kCount>(
         s, ctr->n_shadow, &ctr->shadow_next,
         [&](uint32_t k, TRay& r, float& tmax) {
@@ -162,37 +186,8 @@ __global__ void __launch_bounds__(256, KZ_TRACE_MINB) k_trace_shadow_persistent(
             if (rc == 1) unoccluded(ray);
         },
         dn, dt);
-#else
-    uint2 stack_lm[kWideStack];
-    const LocalStack stack{stack_lm};
-    AnyState c;
-    TRay r;
-    float tmax = 0.f;
-    uint32_t octp = 0, ray = 0;
-    persistent_rays(
-        ctr->n_shadow, &ctr->shadow_next, kTraceRefill,
-        [&](uint32_t k) {
-            ray = k;
-            const float4 o = sq.o4[k], d = sq.d4[k];
-            r = make_tray(xyz(o), xyz(d), kRayEps);
-            tmax = o.w;
-            octp = wide_octant(r);
-            any_begin(c);
-        },
-        [&]() {
-            const int rc = any_step<kCount>(s, r, octp, tmax, c, stack, dn, dt);
-            if (rc == 0) return false;
-            if (rc < 0) set_status(&ctr->status, KZ_ERR_STACK);
-            if (rc == 1) unoccluded(ray);
-            return true;
-        });
-#endif
     if (kCount) warp_count(dn, dt, &ctr->fetch[2]);
 }
-
-// Training samples from the records of a guided pass: every valid vertex
-// whose integrand estimate L*f*cos is positive, weighted by its luminance
-// over the pdf the direction was sampled with.
 
 __global__ void __launch_bounds__(256, KZ_TRACE_MINB) k_trace_paths_batch(const DevJob* __restrict__ jobs, PathSoA p,
                                                                           DevCounters* ctr) {
@@ -207,6 +202,10 @@ __global__ void __launch_bounds__(256, KZ_TRACE_MINB) k_trace_shadow_batch(const
 }
 
 }  // namespace
+
+void launch_pack_nodes(uint4* nodes, uint32_t n, cudaStream_t st) {
+    if (n) k_pack_nodes<<<grid_for(n, 256), 256, 0, st>>>(nodes, n);
+}
 
 void launch_intersect_closest(const DevScene& s, const kz_ray* rays, uint64_t n, kz_hits hits,
                               unsigned long long* next, uint32_t* status, cudaStream_t st) {

@@ -13,8 +13,8 @@
 //    non-coherent loads), in the manner of H. Ylitie, T. Karras, S. Laine,
 //    "Efficient Incoherent Ray Traversal on GPUs Through Compressed Wide
 //    BVHs", HPG 2017: one node test yields a 32-bit mask of inner children
-//    (in an octant-derived near-first order) and leaf triangles; a stack of
-//    (child base, mask) groups in local memory.
+//    (visited in an octant-derived near-first order) and leaf triangles; a
+//    stack of (child base, mask) groups in local memory.
 // Box distances are widened by a margin above their rounding error (see
 // wide_axis), so no box holding a hit at t <= t_best is culled.
 #pragma once
@@ -59,41 +59,15 @@ __device__ __forceinline__ TRay make_tray(f3 o, f3 d, float tmin) {
     return r;
 }
 
-__device__ __forceinline__ float pick(float4 v, int k) { return k == 0 ? v.x : (k == 1 ? v.y : v.z); }
-
-// Watertight test against a triangle record; t, u, v valid when it returns true.
-__device__ __forceinline__ bool tri_test(const TRay& r, float4 a, float4 b, float4 c, float& t, float& bu, float& bv) {
-    const float okx = comp(r.o, r.kx), oky = comp(r.o, r.ky), okz = comp(r.o, r.kz);
-    const float Akx = pick(a, r.kx) - okx, Aky = pick(a, r.ky) - oky, Akz = pick(a, r.kz) - okz;
-    const float Bkx = pick(b, r.kx) - okx, Bky = pick(b, r.ky) - oky, Bkz = pick(b, r.kz) - okz;
-    const float Ckx = pick(c, r.kx) - okx, Cky = pick(c, r.ky) - oky, Ckz = pick(c, r.kz) - okz;
-    const float Ax = Akx - r.Sx * Akz, Ay = Aky - r.Sy * Akz;
-    const float Bx = Bkx - r.Sx * Bkz, By = Bky - r.Sy * Bkz;
-    const float Cx = Ckx - r.Sx * Ckz, Cy = Cky - r.Sy * Ckz;
-    float U = Cx * By - Cy * Bx;
-    float V = Ax * Cy - Ay * Cx;
-    float W = Bx * Ay - By * Ax;
-    if (U == 0.f || V == 0.f || W == 0.f) {
-        U = (float)((double)Cx * (double)By - (double)Cy * (double)Bx);
-        V = (float)((double)Ax * (double)Cy - (double)Ay * (double)Cx);
-        W = (float)((double)Bx * (double)Ay - (double)By * (double)Ax);
-    }
-    if ((U < 0.f || V < 0.f || W < 0.f) && (U > 0.f || V > 0.f || W > 0.f)) return false;
-    const float det = U + V + W;
-    if (det == 0.f) return false;
-    const float T = U * (r.Sz * Akz) + V * (r.Sz * Bkz) + W * (r.Sz * Ckz);
-    t = T / det;
-    bu = V / det;
-    bv = W / det;
-    return true;
-}
+// The component whose bit is set in a pair of bits (0: x, 1: y; neither: z).
+__device__ __forceinline__ float pick_bits(float4 v, uint32_t k) { return (k & 1u) ? v.x : ((k & 2u) ? v.y : v.z); }
 
 // The per-ray terms of the watertight test: the origin in the permuted axes
 // (kx, ky, kz), the shear and the ray's lower bound.
 struct TriRay {
     float okx, oky, okz, tmin;
     float Sx, Sy, Sz;
-    int kx, ky, kz;
+    uint32_t axes;  // pick_bits pairs of kx (bits 0-1), ky (2-3), kz (4-5)
 };
 
 __device__ __forceinline__ TriRay tri_ray(const TRay& r) {
@@ -105,20 +79,20 @@ __device__ __forceinline__ TriRay tri_ray(const TRay& r) {
     q.Sx = r.Sx;
     q.Sy = r.Sy;
     q.Sz = r.Sz;
-    q.kx = r.kx;
-    q.ky = r.ky;
-    q.kz = r.kz;
+    q.axes = (r.kx == 2 ? 0u : 1u << r.kx) | (r.ky == 2 ? 0u : 4u << r.ky) | (r.kz == 2 ? 0u : 16u << r.kz);
     return q;
 }
 
-// The same test with the barycentric divisions left to the caller:
-// u = V / det, v = W / det for the hit that is kept.
+// Watertight test against a triangle record; t is valid when it returns true.
+// The barycentric divisions are left to the caller: u = V / det, v = W / det
+// for the hit that is kept.
 __device__ __forceinline__ bool tri_test_t(const TriRay& r, float4 a, float4 b, float4 c, float& t, float& V_,
                                            float& W_, float& det_) {
     const float okx = r.okx, oky = r.oky, okz = r.okz;
-    const float Akx = pick(a, r.kx) - okx, Aky = pick(a, r.ky) - oky, Akz = pick(a, r.kz) - okz;
-    const float Bkx = pick(b, r.kx) - okx, Bky = pick(b, r.ky) - oky, Bkz = pick(b, r.kz) - okz;
-    const float Ckx = pick(c, r.kx) - okx, Cky = pick(c, r.ky) - oky, Ckz = pick(c, r.kz) - okz;
+    const uint32_t kx = r.axes, ky = r.axes >> 2, kz = r.axes >> 4;
+    const float Akx = pick_bits(a, kx) - okx, Aky = pick_bits(a, ky) - oky, Akz = pick_bits(a, kz) - okz;
+    const float Bkx = pick_bits(b, kx) - okx, Bky = pick_bits(b, ky) - oky, Bkz = pick_bits(b, kz) - okz;
+    const float Ckx = pick_bits(c, kx) - okx, Cky = pick_bits(c, ky) - oky, Ckz = pick_bits(c, kz) - okz;
     const float Ax = Akx - r.Sx * Akz, Ay = Aky - r.Sy * Akz;
     const float Bx = Bkx - r.Sx * Bkz, By = Bky - r.Sy * Bkz;
     const float Cx = Ckx - r.Sx * Ckz, Cy = Cky - r.Sy * Ckz;
@@ -163,113 +137,125 @@ struct HitRec {
 // rounding and no box holding a hit at t <= t_best is culled. An overflowing
 // A or b turns the axis' distances into NaN, which the min/max below ignore:
 // such an axis culls nothing.
+// The device's copy of a node (pack_nodes, kz_trace.cu) holds the same boxes
+// with the fields arranged so that a slot costs no decoding:
+//   w0..w2   p
+//   w3       the x and y scales 2^(E+15) as the upper halves of their floats
+//   w4, w5   first inner child, first triangle record
+//   w6       bits 0-23: triangle k of leaf slot s at bit 3 s + k; bits 24-31
+//            the inner-slot mask
+//   w7       the z scale's upper half (bits 0-15)
+//   w8..w19  per axis 4 words, word j: low and high plane bytes of slot 2 j,
+//            then of slot 2 j + 1
+// A slot that is hit sets its three triangle bits and its inner bit with one
+// constant; an AND with w6 then keeps what the node holds. The near and far
+// byte of a word are picked by the byte permute's own selector, which the
+// ray's direction signs fix.
 struct WideAxis {
     float A, Bn, Bf;
-    uint32_t n0, n1, f0, f1;  // near / far plane bytes (slots 0-3, 4-7)
+    uint4 q;
 };
 
-__device__ __forceinline__ WideAxis wide_axis(float p, uint32_t e, float o, float inv, uint4 q) {
+__device__ __forceinline__ WideAxis wide_axis(float p, float scale, float o, float inv, uint4 q) {
     WideAxis ax;
-    ax.A = __uint_as_float((e + 15u) << 23) * inv;
+    ax.A = scale * inv;
     const float b = (p - o) * inv;
     const float B = b - ax.A;
     const float d = (fabsf(b) + fabsf(ax.A) * 0.03125f) * 1.52587890625e-05f;
     ax.Bn = B - d;
     ax.Bf = B + d;
-    const bool neg = inv < 0.f;  // entering through the high plane
-    ax.n0 = neg ? q.z : q.x;
-    ax.n1 = neg ? q.w : q.y;
-    ax.f0 = neg ? q.x : q.z;
-    ax.f1 = neg ? q.y : q.w;
+    ax.q = q;
     return ax;
 }
 
-template <int kSlot>
-__device__ __forceinline__ float wide_t(const WideAxis& ax, bool near_plane) {
-    const uint32_t w = near_plane ? (kSlot < 4 ? ax.n0 : ax.n1) : (kSlot < 4 ? ax.f0 : ax.f1);
-    const float f = __uint_as_float(__byte_perm(w, 0x3F800000u, 0x7604u | ((kSlot & 3) << 4)));
-    return fmaf(f, ax.A, near_plane ? ax.Bn : ax.Bf);
-}
-
-// KZ_MINMAX3: the slot test's entry / exit distances through three-input
-// min.f32 / max.f32 (sm_100 and later; bit-identical to the fminf / fmaxf
-// chains on every combination of NaN, infinities, signed zeros, denormals and
-// finite values). Measured on the terrain frame: 1,764 against 1,778
-// Mpaths*bounces/s for the chains, which take the ray's bound first.
-#ifndef KZ_MINMAX3
-#define KZ_MINMAX3 0
-#endif
-__device__ __forceinline__ float max3f(float a, float b, float c) {
-#if KZ_MINMAX3
-    float r;
-    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-    return r;
-#else
-    return fmaxf(fmaxf(a, b), c);
-#endif
-}
-__device__ __forceinline__ float min3f(float a, float b, float c) {
-#if KZ_MINMAX3
-    float r;
-    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-    return r;
-#else
-    return fminf(fminf(a, b), c);
-#endif
-}
+// Per-ray constants of the node test and of the visiting order.
+struct WideDir {
+    uint32_t sx, sy, sz;  // byte-permute selectors of the near plane of even slots
+    uint32_t p2, p1, p0;  // inner bits (24-31) visited first at each level of the octant order
+};
 
 template <int kSlot>
-__device__ __forceinline__ void wide_slot(const WideAxis& X, const WideAxis& Y, const WideAxis& Z, uint32_t meta,
+__device__ __forceinline__ float wide_t(const WideAxis& ax, uint32_t sel, bool near_plane) {
+    const uint32_t w = kSlot < 2 ? ax.q.x : kSlot < 4 ? ax.q.y : kSlot < 6 ? ax.q.z : ax.q.w;
+    const uint32_t k = (sel ^ (near_plane ? 0u : 0x10u)) | ((kSlot & 1) ? 0x20u : 0u);
+    return fmaf(__uint_as_float(__byte_perm(w, 0x3F800000u, k)), ax.A, near_plane ? ax.Bn : ax.Bf);
+}
+
+// Two-input minima and maxima on purpose: with the three-input forms, or the
+// planes in packed FP32 pairs, the trace stage of the terrain frame took 86.7
+// and 86.9 ms against 82.2 (fewer instructions, but more registers than the
+// 64 that keep 32 warps on an SM).
+template <int kSlot>
+__device__ __forceinline__ void wide_slot(const WideAxis& X, const WideAxis& Y, const WideAxis& Z, const WideDir& dir,
                                           float tmin, float tcur, uint32_t& hits) {
-    const float tn = max3f(fmaxf(wide_t<kSlot>(X, true), tmin), wide_t<kSlot>(Y, true), wide_t<kSlot>(Z, true));
-    const float tf = min3f(fminf(wide_t<kSlot>(X, false), tcur), wide_t<kSlot>(Y, false), wide_t<kSlot>(Z, false));
-    const uint32_t m = (meta >> (8 * (kSlot & 3))) & 0xFFu;
-    if (tn <= tf) hits |= (m >> 5) << (m & 31u);
+    const float tn = fmaxf(fmaxf(fmaxf(wide_t<kSlot>(X, dir.sx, true), tmin), wide_t<kSlot>(Y, dir.sy, true)),
+                           wide_t<kSlot>(Z, dir.sz, true));
+    const float tf = fminf(fminf(fminf(wide_t<kSlot>(X, dir.sx, false), tcur), wide_t<kSlot>(Y, dir.sy, false)),
+                           wide_t<kSlot>(Z, dir.sz, false));
+    if (tn <= tf) hits |= (7u << (3 * kSlot)) | (1u << (24 + kSlot));
 }
 
-// Tests the 8 child boxes of a node. Returns the hit mask: bits 24-31 the
-// inner children in visiting order (bit 31 first), bits 0-23 the triangles
-// (relative to tri_base) of the leaves hit.
-__device__ __forceinline__ uint32_t wide_node(const uint4* __restrict__ np, const TRay& r, uint32_t octp, float tcur,
-                                              uint32_t& child_base, uint32_t& tri_base, uint32_t& imask) {
+// Leaf triangles pending for a warp-wide test: bits of the node's triangle
+// mask that are hit, the mask itself (a triangle's record is the base plus
+// its rank in the mask) and the base.
+struct LeafGroup {
+    uint32_t bits, valid, base;
+};
+
+__device__ __forceinline__ uint32_t leaf_record(uint32_t base, uint32_t valid, uint32_t bit) {
+    return base + __popc(valid & ((1u << bit) - 1u));
+}
+
+// Tests the 8 child boxes of a node: the inner children hit (bits 24-31, with
+// the inner-slot mask in bits 0-7) and the triangles of the leaves hit.
+__device__ __forceinline__ uint32_t wide_node(const uint4* __restrict__ np, const TRay& r, const WideDir& dir,
+                                              float tcur, uint32_t& child_base, LeafGroup& lg) {
     const uint4 h0 = __ldg(np), h1 = __ldg(np + 1);
     const uint4 qx = __ldg(np + 2), qy = __ldg(np + 3), qz = __ldg(np + 4);
-    child_base = h1.x;
-    tri_base = h1.y;
-    imask = h0.w >> 24;
-    const WideAxis X = wide_axis(__uint_as_float(h0.x), h0.w & 0xFFu, r.o.x, r.inv.x, qx);
-    const WideAxis Y = wide_axis(__uint_as_float(h0.y), (h0.w >> 8) & 0xFFu, r.o.y, r.inv.y, qy);
-    const WideAxis Z = wide_axis(__uint_as_float(h0.z), (h0.w >> 16) & 0xFFu, r.o.z, r.inv.z, qz);
-    // inner slots carry 24 + slot in their low bits; XOR the ray's octant in
-    // so that the nearest octant lands on bit 31
-    uint32_t m0 = h1.z, m1 = h1.w;
-    m0 ^= ((m0 >> 4) & (m0 >> 3) & 0x01010101u) * octp;
-    m1 ^= ((m1 >> 4) & (m1 >> 3) & 0x01010101u) * octp;
+    const WideAxis X = wide_axis(__uint_as_float(h0.x), __uint_as_float(h0.w << 16), r.o.x, r.inv.x, qx);
+    const WideAxis Y = wide_axis(__uint_as_float(h0.y), __uint_as_float(h0.w & 0xFFFF0000u), r.o.y, r.inv.y, qy);
+    const WideAxis Z = wide_axis(__uint_as_float(h0.z), __uint_as_float(h1.w << 16), r.o.z, r.inv.z, qz);
     uint32_t hits = 0;
-    wide_slot<0>(X, Y, Z, m0, r.tmin, tcur, hits);
-    wide_slot<1>(X, Y, Z, m0, r.tmin, tcur, hits);
-    wide_slot<2>(X, Y, Z, m0, r.tmin, tcur, hits);
-    wide_slot<3>(X, Y, Z, m0, r.tmin, tcur, hits);
-    wide_slot<4>(X, Y, Z, m1, r.tmin, tcur, hits);
-    wide_slot<5>(X, Y, Z, m1, r.tmin, tcur, hits);
-    wide_slot<6>(X, Y, Z, m1, r.tmin, tcur, hits);
-    wide_slot<7>(X, Y, Z, m1, r.tmin, tcur, hits);
-    return hits;
+    wide_slot<0>(X, Y, Z, dir, r.tmin, tcur, hits);
+    wide_slot<1>(X, Y, Z, dir, r.tmin, tcur, hits);
+    wide_slot<2>(X, Y, Z, dir, r.tmin, tcur, hits);
+    wide_slot<3>(X, Y, Z, dir, r.tmin, tcur, hits);
+    wide_slot<4>(X, Y, Z, dir, r.tmin, tcur, hits);
+    wide_slot<5>(X, Y, Z, dir, r.tmin, tcur, hits);
+    wide_slot<6>(X, Y, Z, dir, r.tmin, tcur, hits);
+    wide_slot<7>(X, Y, Z, dir, r.tmin, tcur, hits);
+    hits &= h1.z;
+    child_base = h1.x;
+    lg.bits = hits & 0x00FFFFFFu;
+    lg.valid = h1.z & 0x00FFFFFFu;
+    lg.base = h1.y;
+    return (hits & 0xFF000000u) | (h1.z >> 24);
 }
 
-// XOR mask that maps a slot to its visiting rank: 7 for the octant the ray
-// enters first (slot bits set on the axes whose direction is negative).
-__device__ __forceinline__ uint32_t wide_octant(const TRay& r) {
-    return 7u ^ ((r.inv.x < 0.f ? 1u : 0u) | (r.inv.y < 0.f ? 2u : 0u) | (r.inv.z < 0.f ? 4u : 0u));
+// A ray visits its inner children in the order of slot ^ m, largest first,
+// with m = 7 for the octant it enters first (slot bits set on the axes whose
+// direction is negative): at each level the half its direction enters first.
+__device__ __forceinline__ WideDir wide_dir(const TRay& r) {
+    const bool nx = r.inv.x < 0.f, ny = r.inv.y < 0.f, nz = r.inv.z < 0.f;
+    WideDir d;
+    d.sx = nx ? 0x7614u : 0x7604u;
+    d.sy = ny ? 0x7614u : 0x7604u;
+    d.sz = nz ? 0x7614u : 0x7604u;
+    d.p2 = nz ? 0xF0000000u : 0x0F000000u;
+    d.p1 = ny ? 0xCC000000u : 0x33000000u;
+    d.p0 = nx ? 0xAA000000u : 0x55000000u;
+    return d;
 }
 
 // Next inner child of a node group (base, bits): bits 24-31 the remaining
-// hits in visiting order, bits 0-7 the node's inner-slot mask.
-__device__ __forceinline__ uint32_t wide_pop_child(uint32_t base, uint32_t& bits, uint32_t octp) {
-    const uint32_t pos = 31u - __clz(bits);
-    bits ^= 1u << pos;
-    const uint32_t slot = (pos - 24u) ^ octp;
-    return base + __popc(bits & ((1u << slot) - 1u));
+// hits by slot, bits 0-7 the node's inner-slot mask.
+__device__ __forceinline__ uint32_t wide_pop_child(uint32_t base, uint32_t& bits, const WideDir& dir) {
+    uint32_t m = bits & 0xFF000000u;
+    if (m & dir.p2) m &= dir.p2;
+    if (m & dir.p1) m &= dir.p1;
+    if (m & dir.p0) m &= dir.p0;  // one bit is left
+    bits ^= m;
+    return base + __popc(bits & ((m >> 24) - 1u));
 }
 
 // Traversal stack of node groups: a per-thread local array (LocalStack), or
@@ -295,8 +281,8 @@ struct SplitStack {
 
 // Closest-hit traversal state, advanced one node at a time (closest_step) so
 // that persistent kernels can interleave rays; trace_closest runs it to the
-// end. The barycentric divisions are deferred to closest_finish (the same
-// IEEE divisions as tri_test, for the kept hit only).
+// end. The barycentric divisions are deferred to closest_finish (for the kept
+// hit only).
 struct ClosestState {
     float t, V, W, det;
     uint32_t prim;
@@ -324,21 +310,20 @@ __device__ __forceinline__ void closest_begin(ClosestState& c, float tmax) {
 // visited than the tree holds, or a record index is out of range (a corrupt
 // node array).
 template <bool kCount, typename Stack>
-__device__ __forceinline__ int closest_step(const DevScene& s, const TRay& r, uint32_t octp, ClosestState& c,
+__device__ __forceinline__ int closest_step(const DevScene& s, const TRay& r, const WideDir& dir, ClosestState& c,
                                             const Stack& stack, uint32_t& nnode, uint32_t& ntri) {
-    const uint32_t node = wide_pop_child(c.gbase, c.gbits, octp);
+    const uint32_t node = wide_pop_child(c.gbase, c.gbits, dir);
     if (c.gbits > 0x00FFFFFFu) {
         if (c.sp >= kWideStack) return -1;
         stack.put(c.sp++, make_uint2(c.gbase, c.gbits));
     }
     if (++c.visits > s.n_nodes || node >= s.n_nodes) return -1;
-    uint32_t tri_base, imask;
-    const uint32_t hm = wide_node(s.nodes + (size_t)node * 5, r, octp, c.t, c.gbase, tri_base, imask);
+    LeafGroup lg;
+    c.gbits = wide_node(s.nodes + (size_t)node * 5, r, dir, c.t, c.gbase, lg);
     if (kCount) ++nnode;
-    c.gbits = (hm & 0xFF000000u) | imask;
-    uint32_t tbits = hm & 0x00FFFFFFu;
+    uint32_t tbits = lg.bits;
     while (tbits) {
-        const uint32_t rec = tri_base + (__ffs(tbits) - 1);
+        const uint32_t rec = leaf_record(lg.base, lg.valid, __ffs(tbits) - 1);
         tbits &= tbits - 1u;
         if (rec >= s.n_tris) return -1;
         const float4* tp = s.tris + (size_t)rec * 3;
@@ -385,13 +370,13 @@ __device__ __forceinline__ void closest_finish(const ClosestState& c, bool ok, f
 template <bool kCount>
 __device__ bool trace_closest(const DevScene& s, const TRay& r, float tmax, HitRec& h, uint32_t& nnode,
                               uint32_t& ntri) {
-    const uint32_t octp = wide_octant(r);
+    const WideDir dir = wide_dir(r);
     uint2 stack[kWideStack];
     ClosestState c;
     closest_begin(c, tmax);
     int rc;
     do {
-        rc = closest_step<kCount>(s, r, octp, c, LocalStack{stack}, nnode, ntri);
+        rc = closest_step<kCount>(s, r, dir, c, LocalStack{stack}, nnode, ntri);
     } while (rc == 0);
     closest_finish(c, rc > 0, tmax, h);
     return rc > 0;
@@ -414,21 +399,20 @@ __device__ __forceinline__ void any_begin(AnyState& c) {
 // One node of an any-hit query in (tmin, tmax]: 0 while nodes remain, 1 no
 // hit (complete), 2 hit, -1 abort (as closest_step).
 template <bool kCount, typename Stack>
-__device__ __forceinline__ int any_step(const DevScene& s, const TRay& r, uint32_t octp, float tmax, AnyState& c,
+__device__ __forceinline__ int any_step(const DevScene& s, const TRay& r, const WideDir& dir, float tmax, AnyState& c,
                                         const Stack& stack, uint32_t& nnode, uint32_t& ntri) {
-    const uint32_t node = wide_pop_child(c.gbase, c.gbits, octp);
+    const uint32_t node = wide_pop_child(c.gbase, c.gbits, dir);
     if (c.gbits > 0x00FFFFFFu) {
         if (c.sp >= kWideStack) return -1;
         stack.put(c.sp++, make_uint2(c.gbase, c.gbits));
     }
     if (++c.visits > s.n_nodes || node >= s.n_nodes) return -1;
-    uint32_t tri_base, imask;
-    const uint32_t hm = wide_node(s.nodes + (size_t)node * 5, r, octp, tmax, c.gbase, tri_base, imask);
+    LeafGroup lg;
+    c.gbits = wide_node(s.nodes + (size_t)node * 5, r, dir, tmax, c.gbase, lg);
     if (kCount) ++nnode;
-    c.gbits = (hm & 0xFF000000u) | imask;
-    uint32_t tbits = hm & 0x00FFFFFFu;
+    uint32_t tbits = lg.bits;
     while (tbits) {
-        const uint32_t rec = tri_base + (__ffs(tbits) - 1);
+        const uint32_t rec = leaf_record(lg.base, lg.valid, __ffs(tbits) - 1);
         tbits &= tbits - 1u;
         if (rec >= s.n_tris) return -1;
         const float4* tp = s.tris + (size_t)rec * 3;
@@ -450,13 +434,13 @@ __device__ __forceinline__ int any_step(const DevScene& s, const TRay& r, uint32
 template <bool kCount>
 __device__ bool trace_any(const DevScene& s, const TRay& r, float tmax, bool& overflow, uint32_t& nnode,
                           uint32_t& ntri) {
-    const uint32_t octp = wide_octant(r);
+    const WideDir dir = wide_dir(r);
     uint2 stack[kWideStack];
     AnyState c;
     any_begin(c);
     int rc;
     do {
-        rc = any_step<kCount>(s, r, octp, tmax, c, LocalStack{stack}, nnode, ntri);
+        rc = any_step<kCount>(s, r, dir, tmax, c, LocalStack{stack}, nnode, ntri);
     } while (rc == 0);
     overflow = rc < 0;
     return rc == 2;
@@ -464,36 +448,54 @@ __device__ bool trace_any(const DevScene& s, const TRay& r, float tmax, bool& ov
 
 // ---- warp-shared leaf tests ---------------------------------------------------
 //
-// In the persistent kernels a traversal step is split into a node part (the
-// lane's node test; its leaf triangles are left pending), a warp-wide part in
-// which all 32 lanes, busy or idle, test the pending (ray, triangle) pairs of
-// the whole warp, 32 at a time, and a pop of the next node group. A per-lane
+// In the persistent kernels a traversal step is split into a node part
+// (a few node tests per lane; the leaf triangles they hit are left
+// pending) and a warp-wide part in which all 32 lanes, busy or idle, test the
+// pending (ray, triangle) pairs of the whole warp, 32 at a time. A per-lane
 // triangle loop would run for the warp's largest leaf count with a few lanes
 // active; sharing the pairs spreads them over the warp.
 //
+// What bounds these loops is the issue rate (ncu, terrain frame: 79 % of the
+// issue slots, ALU pipe 69 %), so the split follows the instructions: one node
+// test a step leaves some 12 pairs for 32 lanes, two or three fill them. The
+// nodes of a step cull against the bound of the step before, which costs a
+// few visits more than it saves only from four on. Trace + shadow stages of
+// the terrain frame at 1 / 2 / 3 / 4 nodes a step: 132.6 / 105.0 / 102.2 /
+// 104.5 ms (135.7 before, with decoded slots and a searched pair list); any hit
+// on 2^24 incoherent rays at 2 / 3: 5.23 / 5.52 ms (6.31 before), closest hit
+// 8.63 at both (11.19 before).
+//
 // Each lane publishes its ray (TriRay) in shared memory when it starts one.
-// The closest hit of a step is exact and independent of which lane tested
-// what: candidates are combined by a 64-bit atomicMin of (t in a total order,
-// global triangle id) on the owner's slot, the lexicographic minimum that the
+// The closest hit is exact and independent of which lane tested what:
+// candidates are combined by a 64-bit atomicMin of (t in a total order, global
+// triangle id) on the owner's slot, the lexicographic minimum that the
 // sequential loop keeps (smaller t, then smaller id), then the lane whose
 // candidate won writes its record, its unrounded t and the barycentric terms.
+#ifndef KZ_CLOSEST_STEPS
+#define KZ_CLOSEST_STEPS 3
+#endif
+#ifndef KZ_ANY_STEPS
+#define KZ_ANY_STEPS 2
+#endif
+constexpr int kClosestSteps = KZ_CLOSEST_STEPS, kAnySteps = KZ_ANY_STEPS;
+
 struct LeafShare {
-    float4* ray;              // [2 * 256]: (okx, oky, okz, tmin), (Sx, Sy, Sz, kx | ky << 2 | kz << 4)
+    float4* ray;              // [2 * 256]: (okx, oky, okz, tmin), (Sx, Sy, Sz, axes)
     unsigned long long* key;  // [256] closest: best (t, id); any hit: tmax bits
     uint32_t* rec;            // [256] closest: record of the best; any hit: mask of the triangles hit
     float4* vwdt;             // [256] closest: V, W, det, t of the best
+    uint4* ent;               // [steps * 256] pending groups of a warp: bits, valid, base, start | lane << 16
 };
 
 __device__ __forceinline__ void publish_ray(const LeafShare& sh, const TRay& r) {
     const TriRay q = tri_ray(r);
     sh.ray[2 * threadIdx.x] = make_float4(q.okx, q.oky, q.okz, q.tmin);
     sh.ray[2 * threadIdx.x + 1] =
-        make_float4(q.Sx, q.Sy, q.Sz, __uint_as_float((uint32_t)q.kx | ((uint32_t)q.ky << 2) | ((uint32_t)q.kz << 4)));
+        make_float4(q.Sx, q.Sy, q.Sz, __uint_as_float(q.axes));
 }
 
 __device__ __forceinline__ TriRay shared_ray(const LeafShare& sh, uint32_t slot) {
     const float4 a = sh.ray[2 * slot], b = sh.ray[2 * slot + 1];
-    const uint32_t k = __float_as_uint(b.w);
     TriRay q;
     q.okx = a.x;
     q.oky = a.y;
@@ -502,9 +504,7 @@ __device__ __forceinline__ TriRay shared_ray(const LeafShare& sh, uint32_t slot)
     q.Sx = b.x;
     q.Sy = b.y;
     q.Sz = b.z;
-    q.kx = (int)(k & 3u);
-    q.ky = (int)((k >> 2) & 3u);
-    q.kz = (int)((k >> 4) & 3u);
+    q.axes = __float_as_uint(b.w);
     return q;
 }
 
@@ -525,64 +525,88 @@ __device__ __forceinline__ uint32_t nth_set_bit(uint32_t m, uint32_t k) {
     return pos;
 }
 
-// Assignment of pair p (0 <= p < total) of a warp whose lanes hold cnt pairs
-// each (inclusive prefix incl): the owner lane and the owner's bit. Every
-// lane must call it (full-warp shuffles).
-struct LeafPair {
-    uint32_t owner, bit, rec;
-};
-__device__ __forceinline__ LeafPair leaf_pair(uint32_t p, uint32_t incl, uint32_t cnt, uint32_t tbits, uint32_t tbase) {
-    uint32_t o = 0;
+// The pending pairs of a warp as one list: lane by lane, group by group, bit
+// by bit. publish_groups writes each non-empty group with the position of its
+// first pair; pair p then belongs to the group with the largest start <= p,
+// found as the rank of p in a bit mask of the starts (one warp-wide OR and one
+// population count, instead of a search).
+template <int K>
+__device__ __forceinline__ uint32_t publish_groups(const LeafShare& sh, const LeafGroup (&g)[K], uint32_t (&start)[K]) {
+    const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
+    uint32_t cnt = 0;
 #pragma unroll
-    for (uint32_t s = 16; s; s >>= 1) {
-        const uint32_t v = __shfl_sync(0xFFFFFFFFu, incl, o + s - 1);
-        if (v <= p) o += s;
-    }
-    const uint32_t o_incl = __shfl_sync(0xFFFFFFFFu, incl, o);
-    const uint32_t o_cnt = __shfl_sync(0xFFFFFFFFu, cnt, o);
-    const uint32_t o_bits = __shfl_sync(0xFFFFFFFFu, tbits, o);
-    const uint32_t o_base = __shfl_sync(0xFFFFFFFFu, tbase, o);
-    LeafPair lp;
-    lp.owner = o;
-    lp.bit = nth_set_bit(o_bits, p - (o_incl - o_cnt));
-    lp.rec = o_base + lp.bit;
-    return lp;
-}
-
-// Lane's pair count and its inclusive prefix over the warp; returns the total.
-__device__ __forceinline__ uint32_t leaf_scan(uint32_t tbits, uint32_t& cnt, uint32_t& incl) {
-    const uint32_t lane = threadIdx.x & 31u;
-    cnt = __popc(tbits);
-    incl = cnt;
+    for (int k = 0; k < K; ++k) cnt += __popc(g[k].bits);
+    uint32_t incl = cnt;
 #pragma unroll
     for (uint32_t o = 1; o < 32; o <<= 1) {
         const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, o);
         if (lane >= o) incl += v;
     }
+    uint32_t rank = 0, at = incl - cnt;
+#pragma unroll
+    for (int k = 0; k < K; ++k) rank += __popc(__ballot_sync(0xFFFFFFFFu, g[k].bits != 0) & lt);
+    uint4* ent = sh.ent + (threadIdx.x - lane) * K;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        start[k] = at;
+        if (g[k].bits) {
+            ent[rank++] = make_uint4(g[k].bits, g[k].valid, g[k].base, at | (lane << 16));
+            at += __popc(g[k].bits);
+        }
+    }
     return __shfl_sync(0xFFFFFFFFu, incl, 31);
 }
 
-// Node part of a closest-hit step: visits one node; its leaf triangles are
-// returned in tbits (relative to tbase) for the warp-wide test. Returns -1 on
-// an abort (as closest_step), else 0.
+// Pair base + lane of the list (base a multiple of 32, the rounds in order;
+// `seen` counts the groups that started in earlier rounds): its owner lane and
+// record, and its bit in the owner's mask. Every lane must call it.
+struct LeafPair {
+    uint32_t owner, bit, rec;
+    bool live;
+};
+template <int K>
+__device__ __forceinline__ LeafPair leaf_pair(const LeafShare& sh, const LeafGroup (&g)[K], const uint32_t (&start)[K],
+                                              uint32_t base, uint32_t total, uint32_t& seen) {
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t m = 0;
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+        if (g[k].bits && start[k] - base < 32u) m |= 1u << (start[k] - base);
+    m = __reduce_or_sync(0xFFFFFFFFu, m);
+    const uint32_t idx = seen + __popc(m & (0xFFFFFFFFu >> (31u - lane))) - 1u;
+    seen += __popc(m);
+    LeafPair lp;
+    lp.owner = 0;
+    lp.bit = 0;
+    lp.rec = 0;
+    lp.live = base + lane < total;
+    if (lp.live) {
+        const uint4 e = sh.ent[(threadIdx.x - lane) * K + idx];
+        lp.bit = nth_set_bit(e.x, base + lane - (e.w & 0xFFFFu));
+        lp.owner = e.w >> 16;
+        lp.rec = leaf_record(e.z, e.y, lp.bit);
+    }
+    return lp;
+}
+
+// Node part of a step: visits one node, culling boxes beyond tcur; its leaf
+// triangles are left in lg for the warp-wide test. Returns -1 on an abort (as
+// closest_step), else 0.
 template <bool kCount, typename Stack>
-__device__ __forceinline__ int closest_node(const DevScene& s, const TRay& r, uint32_t octp, ClosestState& c,
-                                            const Stack& stack, uint32_t& tbits, uint32_t& tbase, uint32_t& nnode,
-                                            uint32_t& ntri) {
-    const uint32_t node = wide_pop_child(c.gbase, c.gbits, octp);
+__device__ __forceinline__ int visit_node(const DevScene& s, const TRay& r, const WideDir& dir, float tcur, AnyState& c,
+                                          const Stack& stack, LeafGroup& lg, uint32_t& nnode) {
+    const uint32_t node = wide_pop_child(c.gbase, c.gbits, dir);
     if (c.gbits > 0x00FFFFFFu) {
         if (c.sp >= kWideStack) return -1;
         stack.put(c.sp++, make_uint2(c.gbase, c.gbits));
     }
     if (++c.visits > s.n_nodes || node >= s.n_nodes) return -1;
-    uint32_t imask;
-    const uint32_t hm = wide_node(s.nodes + (size_t)node * 5, r, octp, c.t, c.gbase, tbase, imask);
+    c.gbits = wide_node(s.nodes + (size_t)node * 5, r, dir, tcur, c.gbase, lg);
     if (kCount) ++nnode;
-    c.gbits = (hm & 0xFF000000u) | imask;
-    const uint32_t tb = hm & 0x00FFFFFFu;
-    if (tb && (uint64_t)tbase + (31u - __clz(tb)) >= s.n_tris) return -1;
-    if (kCount) ntri += __popc(tb);
-    tbits = tb;
+    if (lg.bits && (uint64_t)lg.base + __popc(lg.valid) > s.n_tris) {
+        lg.bits = 0;
+        return -1;
+    }
     return 0;
 }
 
@@ -597,45 +621,81 @@ __device__ __forceinline__ int group_pop(State& c, const Stack& stack) {
     return c.gbits <= 0x00FFFFFFu ? 1 : 0;
 }
 
-// Warp-wide closest-hit leaf tests; every lane of the warp calls it, lanes
-// without pending triangles with tbits = 0. `tris` is the calling lane's
-// triangle array: with kOwnScene each owner's array is fetched from its lane
-// (batched jobs trace different scenes in one warp).
+// The triangle array of the pair's owner: with kOwnScene each owner's array
+// is fetched from its lane (batched jobs trace different scenes in one warp).
 template <bool kOwnScene>
-__device__ __forceinline__ void closest_leaves(const LeafShare& sh, const float4* tris, uint32_t tbits, uint32_t tbase,
-                                               ClosestState& c) {
-    if (__ballot_sync(0xFFFFFFFFu, tbits != 0) == 0) return;
+__device__ __forceinline__ const float4* owner_tris(const float4* tris, uint32_t owner) {
+    if (!kOwnScene) return tris;
+    const uint64_t tv = reinterpret_cast<uint64_t>(tris);
+    const uint32_t lo = __shfl_sync(0xFFFFFFFFu, (uint32_t)tv, owner);
+    const uint32_t hi = __shfl_sync(0xFFFFFFFFu, (uint32_t)(tv >> 32), owner);
+    return reinterpret_cast<const float4*>(((uint64_t)hi << 32) | lo);
+}
+
+template <int K>
+__device__ __forceinline__ bool any_bits(const LeafGroup (&g)[K]) {
+    uint32_t b = 0;
+#pragma unroll
+    for (int k = 0; k < K; ++k) b |= g[k].bits;
+    return b != 0;
+}
+
+// The best hit of a lane's ray is kept in shared memory: its key, and, once
+// there is one, its record and barycentric terms. A NaN bound accepts nothing.
+__device__ __forceinline__ void best_begin(const LeafShare& sh, float tmax) {
+    sh.key[threadIdx.x] = tmax == tmax ? hit_key(tmax, KZ_INVALID_ID) : 0ull;
+    sh.rec[threadIdx.x] = 0xFFFFFFFFu;
+}
+
+// t of a key (a -0 comes back as +0)
+__device__ __forceinline__ float key_t(unsigned long long key) {
+    const uint32_t o = (uint32_t)(key >> 32);
+    return __uint_as_float((o & 0x80000000u) ? o & 0x7FFFFFFFu : ~o);
+}
+
+// Hit record of the lane's finished traversal; an aborted one (ok == false)
+// misses. The barycentric divisions are made for the kept hit only.
+__device__ __forceinline__ void best_finish(const LeafShare& sh, bool ok, float tmax, HitRec& h) {
+    const int32_t rec = (int32_t)sh.rec[threadIdx.x];
+    h.t = tmax;
+    h.u = h.v = 0.f;
+    h.prim = KZ_INVALID_ID;
+    h.rec = -1;
+    if (!ok || rec < 0) return;
+    const float4 w = sh.vwdt[threadIdx.x];
+    h.t = w.w;
+    h.u = w.x / w.z;
+    h.v = w.y / w.z;
+    h.prim = (uint32_t)sh.key[threadIdx.x];
+    h.rec = rec;
+}
+
+// Warp-wide closest-hit leaf tests; every lane of the warp calls it, lanes
+// without pending triangles with empty groups. `tris` is the calling lane's
+// triangle array; tcur becomes the lane's best t.
+template <bool kOwnScene, int K>
+__device__ __forceinline__ void closest_leaves(const LeafShare& sh, const float4* tris, const LeafGroup (&g)[K],
+                                               float& tcur) {
+    const bool mine = any_bits(g);
+    if (__ballot_sync(0xFFFFFFFFu, mine) == 0) return;
     const uint32_t lane = threadIdx.x & 31u, wbase = threadIdx.x - lane;
-    uint32_t cnt, incl;
-    const uint32_t total = leaf_scan(tbits, cnt, incl);
-    unsigned long long init = 0;
-    if (tbits) {
-        init = hit_key(c.t, c.prim);
-        sh.key[threadIdx.x] = init;
-    }
+    uint32_t start[K], seen = 0;
+    const uint32_t total = publish_groups(sh, g, start);
     __syncwarp();
     for (uint32_t base = 0; base < total; base += 32) {
-        const uint32_t p = base + lane;
-        const LeafPair lp = leaf_pair(p, incl, cnt, tbits, tbase);
-        const float4* tp = tris;
-        if (kOwnScene) {
-            const uint64_t tv = reinterpret_cast<uint64_t>(tris);
-            const uint32_t lo = __shfl_sync(0xFFFFFFFFu, (uint32_t)tv, lp.owner);
-            const uint32_t hi = __shfl_sync(0xFFFFFFFFu, (uint32_t)(tv >> 32), lp.owner);
-            tp = reinterpret_cast<const float4*>(((uint64_t)hi << 32) | lo);
-        }
+        const LeafPair lp = leaf_pair(sh, g, start, base, total, seen);
+        const float4* tp = owner_tris<kOwnScene>(tris, lp.owner);
         const uint32_t slot = wbase + lp.owner;
         bool cand = false;
         unsigned long long key = 0;
         float t = 0.f, V = 0.f, W = 0.f, det = 0.f;
-        if (p < total) {
+        if (lp.live) {
             const TriRay q = shared_ray(sh, slot);
             const float4* tr = tp + (size_t)lp.rec * 3;
             const float4 a = __ldg(tr), b = __ldg(tr + 1), cc = __ldg(tr + 2);
             if (tri_test_t(q, a, b, cc, t, V, W, det) && t > q.tmin) {
                 key = hit_key(t, __float_as_uint(a.w));
-                atomicMin(sh.key + slot, key);
-                cand = true;
+                cand = key < atomicMin(sh.key + slot, key);
             }
         }
         __syncwarp();
@@ -645,43 +705,7 @@ __device__ __forceinline__ void closest_leaves(const LeafShare& sh, const float4
         }
         __syncwarp();
     }
-    if (tbits) {
-        const unsigned long long k = sh.key[threadIdx.x];
-        if (k != init) {
-            const float4 w = sh.vwdt[threadIdx.x];
-            const uint32_t prim = (uint32_t)k;
-            if (w.w < c.t || (w.w == c.t && prim < c.prim)) {
-                c.t = w.w;
-                c.V = w.x;
-                c.W = w.y;
-                c.det = w.z;
-                c.prim = prim;
-                c.rec = (int32_t)sh.rec[threadIdx.x];
-            }
-        }
-    }
-    __syncwarp();
-}
-
-// Node part of an any-hit step (as closest_node, culling against tmax).
-template <bool kCount, typename Stack>
-__device__ __forceinline__ int any_node(const DevScene& s, const TRay& r, uint32_t octp, float tmax, AnyState& c,
-                                        const Stack& stack, uint32_t& tbits, uint32_t& tbase, uint32_t& nnode,
-                                        uint32_t& ntri) {
-    const uint32_t node = wide_pop_child(c.gbase, c.gbits, octp);
-    if (c.gbits > 0x00FFFFFFu) {
-        if (c.sp >= kWideStack) return -1;
-        stack.put(c.sp++, make_uint2(c.gbase, c.gbits));
-    }
-    if (++c.visits > s.n_nodes || node >= s.n_nodes) return -1;
-    uint32_t imask;
-    const uint32_t hm = wide_node(s.nodes + (size_t)node * 5, r, octp, tmax, c.gbase, tbase, imask);
-    if (kCount) ++nnode;
-    c.gbits = (hm & 0xFF000000u) | imask;
-    const uint32_t tb = hm & 0x00FFFFFFu;
-    if (tb && (uint64_t)tbase + (31u - __clz(tb)) >= s.n_tris) return -1;
-    tbits = tb;
-    return 0;
+    if (mine) tcur = fminf(tcur, key_t(sh.key[threadIdx.x]));
 }
 
 // Triangles a sequential any-hit loop over tbits (lowest bit first) tests
@@ -691,32 +715,25 @@ __device__ __forceinline__ uint32_t any_tested(uint32_t tbits, uint32_t hits) {
 }
 
 // Warp-wide any-hit leaf tests: the mask of the lane's pending triangles
-// (bits of tbits) with a hit in (tmin, tmax]. The lane's tmax is in key[] as
-// float bits (publish_tmax).
+// (bits of its groups) with a hit in (tmin, tmax]. The lane's tmax is in key[]
+// as float bits (publish_tmax).
 __device__ __forceinline__ void publish_tmax(const LeafShare& sh, float tmax) {
     sh.key[threadIdx.x] = __float_as_uint(tmax);
 }
-template <bool kOwnScene>
-__device__ __forceinline__ uint32_t any_leaves(const LeafShare& sh, const float4* tris, uint32_t tbits,
-                                               uint32_t tbase) {
-    if (__ballot_sync(0xFFFFFFFFu, tbits != 0) == 0) return 0u;
+template <bool kOwnScene, int K>
+__device__ __forceinline__ uint32_t any_leaves(const LeafShare& sh, const float4* tris, const LeafGroup (&g)[K]) {
+    const bool mine = any_bits(g);
+    if (__ballot_sync(0xFFFFFFFFu, mine) == 0) return 0u;
     const uint32_t lane = threadIdx.x & 31u, wbase = threadIdx.x - lane;
-    uint32_t cnt, incl;
-    const uint32_t total = leaf_scan(tbits, cnt, incl);
-    if (tbits) sh.rec[threadIdx.x] = 0u;
+    uint32_t start[K], seen = 0;
+    const uint32_t total = publish_groups(sh, g, start);
+    if (mine) sh.rec[threadIdx.x] = 0u;
     __syncwarp();
     for (uint32_t base = 0; base < total; base += 32) {
-        const uint32_t p = base + lane;
-        const LeafPair lp = leaf_pair(p, incl, cnt, tbits, tbase);
-        const float4* tp = tris;
-        if (kOwnScene) {
-            const uint64_t tv = reinterpret_cast<uint64_t>(tris);
-            const uint32_t lo = __shfl_sync(0xFFFFFFFFu, (uint32_t)tv, lp.owner);
-            const uint32_t hi = __shfl_sync(0xFFFFFFFFu, (uint32_t)(tv >> 32), lp.owner);
-            tp = reinterpret_cast<const float4*>(((uint64_t)hi << 32) | lo);
-        }
+        const LeafPair lp = leaf_pair(sh, g, start, base, total, seen);
+        const float4* tp = owner_tris<kOwnScene>(tris, lp.owner);
         const uint32_t slot = wbase + lp.owner;
-        if (p < total) {
+        if (lp.live) {
             const TriRay q = shared_ray(sh, slot);
             const float tmax = __uint_as_float((uint32_t)sh.key[slot]);
             const float4* tr = tp + (size_t)lp.rec * 3;
@@ -726,7 +743,7 @@ __device__ __forceinline__ uint32_t any_leaves(const LeafShare& sh, const float4
         }
     }
     __syncwarp();
-    const uint32_t hits = tbits ? sh.rec[threadIdx.x] : 0u;
+    const uint32_t hits = mine ? sh.rec[threadIdx.x] : 0u;
     __syncwarp();
     return hits;
 }
@@ -758,36 +775,11 @@ constexpr uint32_t kTraceRefill = KZ_TRACE_REFILL;
 #endif
 constexpr uint32_t kAnyRefill = KZ_ANY_REFILL;
 
-template <typename Ctr, typename Start, typename Step>
-__device__ __forceinline__ void persistent_rays(Ctr n, Ctr* next, uint32_t refill, Start start, Step step) {
-    const uint32_t lane = threadIdx.x & 31u;
-    bool busy = false, more = true;
-    for (;;) {
-        const uint32_t idle = __ballot_sync(0xFFFFFFFFu, !busy);
-        if (!more && idle == 0xFFFFFFFFu) break;
-        const uint32_t n_idle = __popc(idle);
-        if (more && n_idle >= refill) {
-            Ctr base = 0;
-            if (lane == 0) base = atomicAdd(next, (Ctr)n_idle);
-            base = __shfl_sync(0xFFFFFFFFu, base, 0);
-            if (base + n_idle >= n) more = false;
-            if (!busy) {
-                const Ctr k = base + __popc(idle & ((1u << lane) - 1u));
-                if (k < n) {
-                    busy = true;
-                    start(k);
-                }
-            }
-        }
-        if (busy && step()) busy = false;
-    }
-}
-
-// persistent_rays with the warp-wide leaf part: node(tbits, tbase) runs on
-// the busy lanes and returns -1 on an abort, else 0; leaves(tbits, tbase)
-// runs on all 32 lanes; finish(rc) on the busy lanes returns true once the
-// ray is finished and its result written.
-template <typename Ctr, typename Start, typename Node, typename Leaves, typename Finish>
+// node(lg) runs on the busy lanes and returns -1 on an abort, 0 while nodes
+// remain and 1 when none do; leaves(groups) runs on all 32 lanes; finish(rc)
+// on the busy lanes returns true once the ray is finished and its result
+// written.
+template <int K, typename Ctr, typename Start, typename Node, typename Leaves, typename Finish>
 __device__ __forceinline__ void persistent_rays_shared(Ctr n, Ctr* next, uint32_t refill, Start start, Node node,
                                                        Leaves leaves, Finish finish) {
     const uint32_t lane = threadIdx.x & 31u;
@@ -809,10 +801,14 @@ __device__ __forceinline__ void persistent_rays_shared(Ctr n, Ctr* next, uint32_
                 }
             }
         }
-        uint32_t tbits = 0, tbase = 0;
-        int rc = 0;
-        if (busy) rc = node(tbits, tbase);
-        leaves(tbits, tbase);
+        LeafGroup g[K];
+        int rc = busy ? 0 : 1;
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            g[k].bits = g[k].valid = g[k].base = 0;
+            if (rc == 0) rc = node(g[k]);
+        }
+        leaves(g);
         if (busy && finish(rc)) busy = false;
     }
 }
