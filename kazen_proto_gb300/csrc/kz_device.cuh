@@ -248,16 +248,17 @@ __device__ __forceinline__ f3 sample_vndf(int dist, f3 wi, float ax, float ay, f
         double Z = 1.0 + c + K * exp(-cot_t * cot_t);
         double lo = -1.0, hi = c;
         double uu = fmin(fmax((double)u1, 1e-7), 1.0 - 1e-7);
-        double b = -1.0 + uu * (c + 1.0);
-        for (int it = 0; it < 40; ++it) {
+        double b = -1.0 + uu * (c + 1.0), ei = 0.0;
+        int it = 0;
+        for (; it < 40; ++it) {
             if (!(b > lo && b < hi)) b = 0.5 * (lo + hi);
-            double ei = erfinv(b);
+            ei = erfinv(b);
             double val = (1.0 + b + K * exp(-ei * ei)) / Z - uu;
             if (fabs(val) < 1e-9) break;
             if (val > 0) hi = b; else lo = b;
             b -= val / ((1.0 - ei * tan_t) / Z);
         }
-        sx = (float)erfinv(b);
+        sx = (float)(it < 40 ? ei : erfinv(b));  // a search that ended early left ei at its own b
         sy = (float)erfinv(2.0 * fmin(fmax((double)u2, 1e-7), 1.0 - 1e-7) - 1.0);
     }
     float cp = 1.f, sp = 0.f;
