@@ -201,7 +201,7 @@ struct kz_scene {
     kz_scene_info info{};
 
     // device scene
-    DevBuf nodes, tris, geom_offset, geom_light, mats, lights, light_cdf, light_tris, mat_class;
+    DevBuf nodes, tris, geom_offset, geom_light, mats, lights, light_cdf, light_tris, mat_class, mat_plain;
     // textures and environment
     std::vector<kz::DevTexture> textures;  // offsets into tex_texels
     std::vector<float> tex_texels;
@@ -217,7 +217,7 @@ struct kz_scene {
     DevBuf s_rays, s_t, s_prim, s_geom, s_u, s_v, s_occ, s_ctr, s_next;
 
     // wavefront buffers
-    DevBuf pa[5], pb[5], sh[3], ctr, film, film64;
+    DevBuf pa[5], pb[5], sh[3], heavy, ctr, film, film64;
     kz::DevCounters* ctr_host = nullptr;  // pinned
 
     bool cuda_ready = false;
@@ -226,9 +226,9 @@ struct kz_scene {
         if (!cuda_ready) return;
         cudaSetDevice(device);
         if (stream) cudaStreamSynchronize(stream);
-        DevBuf* all[] = {&nodes, &tris, &geom_offset, &geom_light, &mats, &mat_class, &lights, &light_cdf,
+        DevBuf* all[] = {&nodes, &tris, &geom_offset, &geom_light, &mats, &mat_class, &mat_plain, &lights, &light_cdf,
                          &light_tris, &status, &s_rays, &s_t, &s_prim, &s_geom, &s_u, &s_v, &s_occ, &s_ctr, &s_next,
-                         &ctr, &film, &film64, &d_tri_uv, &d_mat_tex, &d_textures, &d_texels, &d_tri_nrm};
+                         &heavy, &ctr, &film, &film64, &d_tri_uv, &d_mat_tex, &d_textures, &d_texels, &d_tri_nrm};
         for (DevBuf* b : all) b->release();
         for (auto& b : pa) b.release();
         for (auto& b : pb) b.release();
@@ -323,8 +323,15 @@ kz_status alloc_paths(DevBuf* b, uint32_t cap, kz::PathSoA& p) {
     return KZ_OK;
 }
 
-// Wavefront path tracing of `total` paths; contributions are summed into
-// film (and film64) on the device.
+// The queue of split shading for wavefronts large enough for it (else none).
+kz_status alloc_heavy(kz_scene* s, uint32_t cap, kz::HeavyQueue& q) {
+    if (cap < kz::split_shading_capacity()) return KZ_OK;
+    KZ_TRY(s->heavy.ensure((size_t)cap * 2 * sizeof(uint32_t)));
+    q.paths = s->heavy.as<uint32_t>();
+    q.cap = cap;
+    return KZ_OK;
+}
+
 // Guiding hooks of the wavefront loop (null for plain rendering).
 struct GuideHooks {
     const kz::GuideShade* gs = nullptr;
@@ -355,6 +362,8 @@ kz_status run_wavefront(kz_scene* s, const kz::DevCamera* cam, const kz_ray* ray
     KZ_TRY(alloc_paths(s->pb, cap, B));
     for (int k = 0; k < 3; ++k) KZ_TRY(s->sh[k].ensure((size_t)cap * sizeof(float4)));
     kz::ShadowSoA sq{s->sh[0].as<float4>(), s->sh[1].as<float4>(), s->sh[2].as<float4>()};
+    kz::HeavyQueue hq;
+    if (!gh) KZ_TRY(alloc_heavy(s, cap, hq));
     KZ_TRY(s->ctr.ensure(sizeof(kz::DevCounters)));
     kz::DevCounters* ctr = s->ctr.as<kz::DevCounters>();
     cudaStream_t strm = s->stream;
@@ -400,7 +409,8 @@ kz_status run_wavefront(kz_scene* s, const kz::DevCamera* cam, const kz_ray* ray
             kz::launch_trace_paths_dev(s->dev, A, cap, ctr, count, block, strm);
             if (gh) kz::launch_guide_infer_paths_dev(s->dev, A, cap, ctr, gh->gd, gh->raw, strm);
             if (e) KZ_CUDA(cudaEventRecord(e[2], strm));
-            kz::launch_shade_dev(s->dev, pp, A, cap, B, sq, ctr, film, film64, gh ? gh->gs : nullptr, block, strm);
+            st.kernel_launches +=
+                kz::launch_shade_dev(s->dev, pp, A, cap, B, sq, hq, ctr, film, film64, gh ? gh->gs : nullptr, block, strm);
             if (e) KZ_CUDA(cudaEventRecord(e[3], strm));
             if (gh)
                 kz::launch_trace_shadow_guided(s->dev, sq, cap, ctr, film, film64, gh->gs->recs, gh->gs->nee,
@@ -409,7 +419,7 @@ kz_status run_wavefront(kz_scene* s, const kz::DevCamera* cam, const kz_ray* ray
                 kz::launch_trace_shadow_dev(s->dev, sq, cap, ctr, count, film, film64, strm);
             kz::launch_finish(ctr, strm);
             if (e) KZ_CUDA(cudaEventRecord(e[4], strm));
-            st.kernel_launches += gh ? 7 : 6;
+            st.kernel_launches += gh ? 6 : 5;
             std::swap(A, B);
         }
         KZ_CUDA(cudaGetLastError());
@@ -837,30 +847,48 @@ kz_status kz_scene_build(kz_scene* s) {
     KZ_TRY(upload(s->geom_offset, goff, st));
     KZ_TRY(upload(s->geom_light, glight, st));
     KZ_TRY(upload(s->mats, s->materials, st));
+    uint32_t has_heavy = 0;
     {
-        // shading class of each material (by its first lobe), the key the
-        // shading kernel groups a block's paths by
+        // shading class of each material and, for the plain ones, the lobe's weight
         std::vector<uint8_t> cls(s->materials.size());
+        std::vector<float4> plain(s->materials.size(), make_float4(0.f, 0.f, 0.f, 0.f));
         for (size_t m = 0; m < s->materials.size(); ++m) {
             const kz_material& mt = s->materials[m];
-            uint8_t c = 3;  // no lobe (emitter only)
-            if (mt.n_lobes > 0) {
-                switch (mt.lobes[0].closure_id) {
+            const kz_lobe& l = mt.lobes[0];
+            uint8_t c = kz::kPlainClass;
+            const bool diffuse = mt.n_lobes == 1 && l.closure_id == KZ_CLOSURE_DIFFUSE && l.params[0] == 0.f &&
+                                 l.params[1] == 1.f && l.params[2] == 0.f;
+            if (mt.n_lobes == 0 || diffuse) {
+                const bool emits = mt.Le[0] != 0.f || mt.Le[1] != 0.f || mt.Le[2] != 0.f;
+                plain[m] = make_float4(0.f, 0.f, 0.f, emits ? 1.f : 0.f);
+                if (diffuse) {
+                    plain[m].x = l.weight[0];
+                    plain[m].y = l.weight[1];
+                    plain[m].z = l.weight[2];
+                }
+            } else {
+                switch (l.closure_id) {
                 case KZ_CLOSURE_KP_MIRROR: case KZ_CLOSURE_KP_DIELECTRIC: case KZ_CLOSURE_REFLECTION:
                 case KZ_CLOSURE_REFRACTION: case KZ_CLOSURE_TRANSPARENT:
-                    c = 2;  // delta
+                    c = kz::kDeltaClass;
                     break;
                 case KZ_CLOSURE_KP_GLOSS: case KZ_CLOSURE_KP_GLASS: case KZ_CLOSURE_CONDUCTOR_GGX:
                 case KZ_CLOSURE_KP_PRINCIPLE_SPECULAR_REFL: case KZ_CLOSURE_WARD: case KZ_CLOSURE_KP_MICROFACET:
                 case KZ_CLOSURE_KP_PRINCIPLE_CLEARCOAT: case KZ_CLOSURE_PHONG:
-                    c = 1;  // glossy
+                    c = kz::kGlossyClass;
                     break;
                 default:
-                    c = 0;  // diffuse-like
+                    c = kz::kDiffuseClass;
                 }
+                for (uint32_t k = 0; k < mt.n_lobes; ++k)
+                    if ((mt.lobes[k].closure_id == KZ_CLOSURE_KP_GLOSS || mt.lobes[k].closure_id == KZ_CLOSURE_KP_GLASS) &&
+                        mt.lobes[k].params[0] == (float)KZ_DIST_BECKMANN)
+                        c = kz::kBeckmannClass;
             }
             cls[m] = c;
+            if (c != kz::kPlainClass) has_heavy = 1;
         }
+        KZ_TRY(upload(s->mat_plain, plain, st));
         KZ_TRY(upload(s->mat_class, cls, st));
     }
     KZ_TRY(upload(s->lights, lights, st));
@@ -901,6 +929,8 @@ kz_status kz_scene_build(kz_scene* s) {
     d.geom_light = s->geom_light.as<int32_t>();
     d.materials = s->mats.as<kz_material>();
     d.mat_class = s->mat_class.as<uint8_t>();
+    d.mat_plain = s->mat_plain.as<float4>();
+    d.has_heavy = has_heavy;
     d.n_materials = (uint32_t)s->materials.size();
     d.lights = s->lights.as<kz::DevLight>();
     d.light_cdf = s->light_cdf.as<float>();
@@ -1670,7 +1700,7 @@ extern "C" kz_status kz_scene_release_scratch(kz_scene* s) {
     KZ_CUDA(cudaSetDevice(s->device));
     KZ_CUDA(cudaStreamSynchronize(s->stream));
     DevBuf* all[] = {&s->s_rays, &s->s_t, &s->s_prim, &s->s_geom, &s->s_u, &s->s_v, &s->s_occ, &s->s_ctr, &s->s_next,
-                     &s->film, &s->film64};
+                     &s->heavy, &s->film, &s->film64};
     for (DevBuf* b : all) b->release();
     for (auto& b : s->pa) b.release();
     for (auto& b : s->pb) b.release();
@@ -1699,6 +1729,8 @@ kz_status batch_wavefront(const kz_batch_job* jobs, uint32_t n_jobs, const kz_ba
     KZ_TRY(alloc_paths(s->pb, cap, B));
     for (int k = 0; k < 3; ++k) KZ_TRY(s->sh[k].ensure((size_t)cap * sizeof(float4)));
     kz::ShadowSoA sq{s->sh[0].as<float4>(), s->sh[1].as<float4>(), s->sh[2].as<float4>()};
+    kz::HeavyQueue hq;
+    if (cfg.mode == KZ_BATCH_WAVEFRONT) KZ_TRY(alloc_heavy(s, cap, hq));
     KZ_TRY(s->ctr.ensure(sizeof(kz::DevCounters)));
     kz::DevCounters* ctr = s->ctr.as<kz::DevCounters>();
     for (uint32_t j = 0; j < n_jobs; ++j) KZ_CUDA(cudaMemsetAsync(fptr[j], 0, npix[j] * 12, strm));
@@ -1712,9 +1744,12 @@ kz_status batch_wavefront(const kz_batch_job* jobs, uint32_t n_jobs, const kz_ba
     // they started and a captured batch can be replayed as is
     uint32_t iters = std::max<uint32_t>(4, max_depth + 1);
     iters += iters & 1u;
-    bool textured = false;  // the texture tint is compiled out unless a job needs it
-    for (uint32_t j = 0; j < n_jobs; ++j)
+    // the texture tint is compiled out, and the second shading kernel left out, unless a job needs it
+    bool textured = false, heavy = false;
+    for (uint32_t j = 0; j < n_jobs; ++j) {
         textured |= jobs[j].scene->dev.mat_tex != nullptr || jobs[j].scene->dev.tri_nrm != nullptr;
+        heavy |= jobs[j].scene->dev.has_heavy != 0;
+    }
     // refill period P: free wavefront slots take new paths every P-th
     // iteration (P = 1: every iteration); in between the wavefront drains, so
     // the generation launches are fewer and the live paths fewer too
@@ -1728,7 +1763,7 @@ kz_status batch_wavefront(const kz_batch_job* jobs, uint32_t n_jobs, const kz_ba
             kz::launch_plan(ctr, cap, strm, gen);
             if (gen) kz::launch_generate_batch_dev(djobs, n_jobs, a, ctr, cap, block, strm);
             kz::launch_trace_paths_batch(djobs, a, cap, ctr, strm);
-            kz::launch_shade_batch(djobs, a, cap, b, sq, ctr, block, textured, strm);
+            kz::launch_shade_batch(djobs, a, cap, b, sq, hq, ctr, block, textured, heavy, strm);
             kz::launch_trace_shadow_batch(djobs, sq, cap, ctr, strm);
             kz::launch_finish(ctr, strm);
             std::swap(a, b);
@@ -2120,10 +2155,10 @@ extern "C" kz_status kz_li_batch_noalloc(kz_scene* s, const kz_ray* rays, uint64
         KZ_CUDA(cudaStreamSynchronize(strm));
         KZ_CUDA(cudaGetLastError());
         st.path_bounces += nA;
-        st.shadow_rays += hc.n_shadow;
+        st.shadow_rays += hc.queue.shadow;
         st.iterations += 1;
         if (hc.status) return fail((kz_status)hc.status, "device status %u during Li batch", hc.status);
-        nA = hc.n_next;
+        nA = hc.queue.next;
         std::swap(A, B);
     }
     if (count) {

@@ -24,37 +24,26 @@ __global__ void k_generate_batch_dev(const DevJob* __restrict__ jobs, uint32_t n
 template <bool kAttr>
 __device__ __forceinline__ void batch_shade(const DevJob* __restrict__ jobs, PathSoA in, PathSoA out, ShadowSoA sq,
                                             DevCounters* ctr, uint32_t i, uint32_t n_in) {
-#if KZ_SHADE_SORT
-    i = block_group_by_kind(
-        i, i < n_in ? shade_kind(jobs[__float_as_uint(in.d4[i].w) >> kJobShift].scene, in.hit[i]) : 5u);
-#endif
+    uint32_t kind = i < n_in ? shade_kind(jobs[__float_as_uint(in.d4[i].w) >> kJobShift].scene, in.hit[i]) : kNoPath;
+    i = block_group_by_kind(i, kind);
     ShadeOut so;
     if (i < n_in) {
         const float4 d4 = in.d4[i];
         const DevJob& J = jobs[__float_as_uint(d4.w) >> kJobShift];
-        shade_vertex<false, kAttr>(J.scene, J.pp, in.hit[i], in.o4[i], d4, in.b4[i], in.rng[i], GuideShade{}, nullptr,
-                                  so);
+        if (kind == 1u + kPlainClass)
+            shade_plain<kAttr>(J.scene, J.pp, in.hit[i], in.o4[i], d4, in.b4[i], in.rng[i], so);
+        else
+            shade_vertex<false, kAttr>(J.scene, J.pp, in.hit[i], in.o4[i], d4, in.b4[i], in.rng[i], GuideShade{},
+                                      nullptr, so);
         if (!is_zero(so.Lsum)) film_add(J.film, nullptr, so.film_idx, so.Lsum);
     }
-    const bool cont = so.cont, shadow = so.shadow;
-    const uint32_t slot = warp_append(cont, &ctr->n_next);
-    if (cont) {
-        out.o4[slot] = so.o_next;
-        out.d4[slot] = so.d_next;
-        out.b4[slot] = so.b_next;
-        out.rng[slot] = so.rng_next;
-    }
-    const uint32_t sslot = warp_append(shadow, &ctr->n_shadow);
-    if (shadow) {
-        sq.o4[sslot] = so.s_o;
-        sq.d4[sslot] = so.s_d;
-        sq.c4[sslot] = so.s_c;
-    }
+    store_next(out, sq, so, warp_append_pair(so.cont, so.shadow, ctr));
 }
 
 template <bool kAttr>
 __global__ void __launch_bounds__(256, KZ_SHADE_MIN_BLOCKS) k_shade_batch(const DevJob* __restrict__ jobs, PathSoA in, PathSoA out,
                                                      ShadowSoA sq, DevCounters* ctr) {
+    if (blockIdx.x * blockDim.x >= ctr->n_active) return;  // the grid covers the wavefront's capacity
     batch_shade<kAttr>(jobs, in, out, sq, ctr, blockIdx.x * blockDim.x + threadIdx.x, ctr->n_active);
 }
 
@@ -190,13 +179,21 @@ cudaError_t launch_batch_persistent(const DevJob* jobs, uint32_t n_jobs, PathSoA
     return cudaLaunchCooperativeKernel(f, dim3(blocks), dim3(256), args, kBatchSmem, st);
 }
 
-void launch_shade_batch(const DevJob* jobs, PathSoA in, uint32_t cap, PathSoA out, ShadowSoA sq, DevCounters* ctr,
-                        uint32_t block, bool textured, cudaStream_t st) {  // textured: textures or normals
-    if (!cap) return;
+int launch_shade_batch(const DevJob* jobs, PathSoA in, uint32_t cap, PathSoA out, ShadowSoA sq, HeavyQueue hq,
+                       DevCounters* ctr, uint32_t block, bool textured, bool heavy, cudaStream_t st) {
+    if (!cap) return 0;  // textured: textures or normals
+    if (hq.paths) {
+        if (textured)
+            return launch_split_shading<true, true>(DevScene{}, PathParams{}, jobs, in, cap, out, sq, hq, ctr, nullptr,
+                                                    nullptr, heavy, st);
+        return launch_split_shading<false, true>(DevScene{}, PathParams{}, jobs, in, cap, out, sq, hq, ctr, nullptr,
+                                                 nullptr, heavy, st);
+    }
     if (textured)
         k_shade_batch<true><<<grid_for(cap, block), block, 0, st>>>(jobs, in, out, sq, ctr);
     else
         k_shade_batch<false><<<grid_for(cap, block), block, 0, st>>>(jobs, in, out, sq, ctr);
+    return 1;
 }
 
 }  // namespace kz

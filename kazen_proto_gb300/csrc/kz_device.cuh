@@ -303,6 +303,7 @@ struct LobeSample {
     f3 weight;
     float pdf;
     bool valid, delta;
+    f3 f;  // lobe_eval's value at wo (valid, not delta)
 };
 
 __device__ __forceinline__ bool lobe_is_delta(uint32_t id) {
@@ -714,7 +715,7 @@ KZ_LOBE_FN LobeEval lobe_eval(const kz_lobe& l, f3 wi, f3 wo) {
 }
 
 KZ_LOBE_FN LobeSample lobe_sample(const kz_lobe& l, f3 wi, float u0, float u1, float u2) {
-    LobeSample s{mk(0.f, 0.f, 0.f), mk(0.f, 0.f, 0.f), 0.f, false, false};
+    LobeSample s{mk(0.f, 0.f, 0.f), mk(0.f, 0.f, 0.f), 0.f, false, false, mk(0.f, 0.f, 0.f)};
     switch (l.closure_id) {
     case KZ_CLOSURE_DIFFUSE:
     case KZ_CLOSURE_KP_PRINCIPLE_DIFFUSE:
@@ -731,6 +732,7 @@ KZ_LOBE_FN LobeSample lobe_sample(const kz_lobe& l, f3 wi, float u0, float u1, f
         if (e.pdf <= 0.f) return s;
         s.pdf = e.pdf;
         s.weight = e.f * (1.f / e.pdf);
+        s.f = e.f;
         s.valid = true;
         return s;
     }
@@ -841,6 +843,7 @@ KZ_LOBE_FN LobeSample lobe_sample(const kz_lobe& l, f3 wi, float u0, float u1, f
         if (e.pdf <= 0.f) return s;
         s.pdf = e.pdf;
         s.weight = e.f * (1.f / e.pdf);
+        s.f = e.f;
         s.valid = true;
         return s;
     }
@@ -857,6 +860,7 @@ KZ_LOBE_FN LobeSample lobe_sample(const kz_lobe& l, f3 wi, float u0, float u1, f
         if (e.pdf <= 0.f) return s;
         s.pdf = e.pdf;
         s.weight = e.f * (1.f / e.pdf);
+        s.f = e.f;
         s.valid = true;
         return s;
     }
@@ -881,6 +885,7 @@ KZ_LOBE_FN LobeSample lobe_sample(const kz_lobe& l, f3 wi, float u0, float u1, f
         if (e.pdf <= 0.f) return s;
         s.pdf = e.pdf;
         s.weight = e.f * (1.f / e.pdf);
+        s.f = e.f;
         s.valid = true;
         return s;
     }

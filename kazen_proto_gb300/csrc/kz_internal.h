@@ -32,6 +32,13 @@ struct DevTexture {
     float Ca[3] = {1.f, 1.f, 1.f}, Cb[3] = {0.f, 0.f, 0.f};
 };
 
+// Shading classes of materials, the key the shading kernels group paths by: a
+// plain one has at most one lobe, diffuse about the shading normal; the others
+// are heavy: with a lobe whose sampling is the FP64 Beckmann search, or by the
+// first lobe glossy, diffuse-like or delta.
+enum : uint32_t { kPlainClass, kBeckmannClass, kGlossyClass, kDiffuseClass, kDeltaClass, kNumClasses };
+constexpr uint32_t kHeavyClasses = kNumClasses - 1;
+
 struct DevScene {
     const uint4* nodes = nullptr;       // n_nodes * 5 (80-byte 8-wide nodes)
     const float4* tris = nullptr;       // n_tris * 3, leaf order
@@ -39,7 +46,9 @@ struct DevScene {
     const uint32_t* geom_offset = nullptr;  // first global triangle id per mesh
     const int32_t* geom_light = nullptr;    // light index per mesh or -1
     const kz_material* materials = nullptr;
-    const uint8_t* mat_class = nullptr;  // per material: 0 diffuse-like, 1 glossy, 2 delta, 3 no lobe
+    const uint8_t* mat_class = nullptr;  // shading class of each material
+    const float4* mat_plain = nullptr;   // per material of kPlainClass: its lobe's weight (0 without), w = 1: it emits
+    uint32_t has_heavy = 0;              // some material is not plain
     uint32_t n_materials = 0;
     const DevLight* lights = nullptr;
     const float* light_cdf = nullptr;
@@ -135,10 +144,22 @@ struct PathParams {
     uint32_t estimator = 0;  // 0: NEE + BSDF sampling with MIS, 1: NEE only, 2: BSDF sampling only
 };
 
+// Paths that the first shading kernel leaves to the second (split shading): two
+// arrays of `cap` path indices; paths == nullptr: one kernel shades all.
+struct HeavyQueue {
+    uint32_t* paths = nullptr;
+    uint32_t cap = 0;
+};
+
 // Counters the stage kernels update on the device.
 struct DevCounters {
-    uint32_t n_next;     // continuing paths written by shade
-    uint32_t n_shadow;   // shadow rays queued by shade
+    union {
+        unsigned long long n_append;  // both counts, for one atomic
+        struct {
+            uint32_t next;    // continuing paths written by shade
+            uint32_t shadow;  // shadow rays queued by shade
+        } queue;
+    };
     uint32_t status;     // device-side error (KZ_ERR_STACK ...)
     uint32_t n_active;   // paths in the current buffer (device-driven loop)
     unsigned long long fetch[4];  // closest nodes, closest tris, shadow nodes, shadow tris
@@ -149,6 +170,7 @@ struct DevCounters {
     uint32_t gen_count, gen_slot;  // how many, and where in the buffer
     uint32_t trace_next;           // persistent kernels: next path / shadow ray to fetch
     uint32_t shadow_next;
+    uint32_t heavy[kHeavyClasses], heavy_next;  // split shading: paths queued by class, fetch cursor
     uint32_t bar_count, bar_gen;   // grid barrier of the persistent batch kernel
     uint32_t bar_abort;            // set when a barrier wait ran out
 };
@@ -258,9 +280,12 @@ void launch_trace_paths_dev(const DevScene& s, PathSoA p, uint32_t cap, DevCount
 void launch_shade_guided_dev(const DevScene& s, const PathParams& pp, PathSoA in, uint32_t cap, PathSoA out,
                              ShadowSoA sq, DevCounters* ctr, float* film, double* film64, const GuideShade& gs,
                              uint32_t block, cudaStream_t st);
-void launch_shade_dev(const DevScene& s, const PathParams& pp, PathSoA in, uint32_t cap, PathSoA out, ShadowSoA sq,
-                      DevCounters* ctr, float* film, double* film64, const GuideShade* gs, uint32_t block,
-                      cudaStream_t st);
+// Both return the number of kernels launched.
+int launch_shade_dev(const DevScene& s, const PathParams& pp, PathSoA in, uint32_t cap, PathSoA out, ShadowSoA sq,
+                     HeavyQueue hq, DevCounters* ctr, float* film, double* film64, const GuideShade* gs, uint32_t block,
+                     cudaStream_t st);
+// Capacity from which a wavefront is given a HeavyQueue.
+uint32_t split_shading_capacity();
 // Persistent batch renderer: grid = ctas blocks of `block` threads; each lane
 // keeps one path in registers and refills from the global counter every
 // `period` vertices (warp-aggregated fetch).
@@ -268,8 +293,8 @@ void launch_shade_dev(const DevScene& s, const PathParams& pp, PathSoA in, uint3
 void launch_generate_batch_dev(const DevJob* jobs, uint32_t n_jobs, PathSoA dst, DevCounters* ctr, uint32_t cap,
                                uint32_t block, cudaStream_t st);
 void launch_trace_paths_batch(const DevJob* jobs, PathSoA p, uint32_t cap, DevCounters* ctr, cudaStream_t st);
-void launch_shade_batch(const DevJob* jobs, PathSoA in, uint32_t cap, PathSoA out, ShadowSoA sq, DevCounters* ctr,
-                        uint32_t block, bool textured, cudaStream_t st);
+int launch_shade_batch(const DevJob* jobs, PathSoA in, uint32_t cap, PathSoA out, ShadowSoA sq, HeavyQueue hq,
+                       DevCounters* ctr, uint32_t block, bool textured, bool heavy, cudaStream_t st);
 void launch_trace_shadow_batch(const DevJob* jobs, ShadowSoA sq, uint32_t cap, DevCounters* ctr, cudaStream_t st);
 int batch_persistent_blocks_per_sm(bool textured);
 cudaError_t launch_batch_persistent(const DevJob* jobs, uint32_t n_jobs, PathSoA A, PathSoA B, ShadowSoA sq,

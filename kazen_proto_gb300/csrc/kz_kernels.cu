@@ -107,21 +107,29 @@ void launch_generate_rays_dev(const kz_ray* rays, const PathParams& pp, PathSoA 
     if (!cap) return;
     k_generate_rays_dev<<<grid_for(cap, block), block, 0, st>>>(rays, pp, dst, ctr);
 }
-void launch_shade_dev(const DevScene& s, const PathParams& pp, PathSoA in, uint32_t cap, PathSoA out, ShadowSoA sq,
-                      DevCounters* ctr, float* film, double* film64, const GuideShade* gs, uint32_t block,
-                      cudaStream_t st) {
-    if (!cap) return;
+int launch_shade_dev(const DevScene& s, const PathParams& pp, PathSoA in, uint32_t cap, PathSoA out, ShadowSoA sq,
+                     HeavyQueue hq, DevCounters* ctr, float* film, double* film64, const GuideShade* gs, uint32_t block,
+                     cudaStream_t st) {
+    if (!cap) return 0;
+    const bool attr = s.mat_tex || s.tri_nrm;
     if (gs) {
         launch_shade_guided_dev(s, pp, in, cap, out, sq, ctr, film, film64, *gs, block, st);
-        return;
-    }
-    if (s.mat_tex || s.tri_nrm)
+    } else if (hq.paths) {
+        if (attr)
+            return launch_split_shading<true, false>(s, pp, nullptr, in, cap, out, sq, hq, ctr, film, film64,
+                                                     s.has_heavy != 0, st);
+        return launch_split_shading<false, false>(s, pp, nullptr, in, cap, out, sq, hq, ctr, film, film64,
+                                                  s.has_heavy != 0, st);
+    } else if (attr) {
         k_shade<false, true><<<grid_for(cap, block), block, 0, st>>>(s, pp, in, cap, out, sq, ctr, film, film64,
                                                                      GuideShade{}, &ctr->n_active);
-    else
+    } else {
         k_shade<false, false><<<grid_for(cap, block), block, 0, st>>>(s, pp, in, cap, out, sq, ctr, film, film64,
                                                                       GuideShade{}, &ctr->n_active);
+    }
+    return 1;
 }
+uint32_t split_shading_capacity() { return KZ_SPLIT_SHADING; }
 void launch_shade(const DevScene& s, const PathParams& pp, PathSoA in, uint32_t n_in, PathSoA out, ShadowSoA sq,
                   DevCounters* ctr, float* film, double* film64, uint32_t block, cudaStream_t st) {
     if (!n_in) return;

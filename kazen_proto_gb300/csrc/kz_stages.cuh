@@ -362,6 +362,174 @@ struct ShadeOut {
     uint32_t film_idx = 0;
 };
 
+// Next-event estimation's light sample seen from P: the light picked by u0, its
+// triangle by u1, the point on it by u2 and u3.
+struct LightSample {
+    f3 dir, Le;
+    float dist, dist2, pdf;  // pdf in solid angle, with the pick probability
+    bool point, lit;         // lit: P lies on the emitting side
+};
+__device__ __forceinline__ LightSample sample_light(const DevScene& s, f3 P, float u0, float u1, float u2, float u3) {
+    const uint32_t nl = s.n_lights;
+    const uint32_t li = min((uint32_t)(u0 * (float)nl), nl - 1);
+    const DevLight lt = s.lights[li];
+    LightSample r;
+    // a point light (PointLight, light.cpp:18-31) has no triangles: its
+    // position is the one light_tris record it names
+    r.point = lt.tri_count == 0;
+    f3 p, nlgt = mk(0.f, 0.f, 0.f);
+    if (r.point) {
+        p = xyz(__ldg(s.light_tris + (size_t)lt.tri_begin * 3));
+    } else {
+        const uint32_t kk = cdf_sample(s.light_cdf + lt.cdf_begin, lt.tri_count, u1);
+        const float4* lq = s.light_tris + (size_t)(lt.tri_begin + kk) * 3;
+        const f3 a0 = xyz(__ldg(lq)), a1 = xyz(__ldg(lq + 1)), a2 = xyz(__ldg(lq + 2));
+        const float su0 = sqrtf(u2);
+        const float bu0 = 1.f - su0;
+        const float bv0 = u3 * su0;
+        p = a0 * bu0 + a1 * bv0 + a2 * (1.f - bu0 - bv0);
+        nlgt = normalize(cross(a1 - a0, a2 - a0));
+    }
+    const f3 lv = p - P;
+    r.dist2 = dot(lv, lv);
+    r.dist = sqrtf(r.dist2);
+    r.dir = mk(lv.x / r.dist, lv.y / r.dist, lv.z / r.dist);
+    const float cos_l = r.point ? 1.f : -dot(r.dir, nlgt);
+    r.lit = cos_l > 0.f && r.dist2 > 0.f;
+    // a delta light is picked with probability 1/nl and weighs no MIS
+    r.pdf = r.point ? 1.0f / (float)nl : r.dist2 / (cos_l * lt.area) * (1.0f / (float)nl);
+    r.Le = ld3(lt.Le);
+    return r;
+}
+
+// Shading normal and point of a hit: the interpolated vertex normal, with the
+// point moved off the flat triangle by the shadow-terminator offset (Hanika
+// 2021), as TriangleMesh::post_hit does (shape.cpp:628-656); Ng and P as they
+// are for a mesh without normals.
+__device__ __forceinline__ void smooth_hit(const DevScene& s, int rec, const float4 hit, f3 v0, f3 v1, f3 v2, f3& Ns,
+                                           f3& P) {
+    const float4 m0 = __ldg(s.tri_nrm + (size_t)rec * 3);
+    if (m0.w == 0.f) return;
+    const f3 n0 = xyz(m0), n1 = xyz(__ldg(s.tri_nrm + (size_t)rec * 3 + 1)),
+             n2 = xyz(__ldg(s.tri_nrm + (size_t)rec * 3 + 2));
+    const float b0 = 1.f - hit.y - hit.z;
+    Ns = normalize(n0 * b0 + n1 * hit.y + n2 * hit.z);
+    const f3 Pb = v0 * b0 + v1 * hit.y + v2 * hit.z;
+    const float e0 = fminf(0.f, dot(Pb - v0, n0)), e1 = fminf(0.f, dot(Pb - v1, n1)),
+                e2 = fminf(0.f, dot(Pb - v2, n2));
+    P = Pb - (n0 * (b0 * e0) + n1 * (hit.y * e1) + n2 * (hit.z * e2));
+}
+
+// Texture tint of a hit at its uv (interpolated vertex uvs; the barycentrics
+// of vertices 1, 2 when the mesh has none).
+__device__ __forceinline__ f3 hit_tint(const DevScene& s, int rec, const float4 hit, int32_t tex) {
+    const float2 q0 = s.tri_uv[(size_t)rec * 3], q1 = s.tri_uv[(size_t)rec * 3 + 1], q2 = s.tri_uv[(size_t)rec * 3 + 2];
+    const float b0 = 1.f - hit.y - hit.z;
+    return tex_eval(s, tex, b0 * q0.x + hit.y * q1.x + hit.z * q2.x, b0 * q0.y + hit.y * q1.y + hit.z * q2.y);
+}
+
+// Weight of an emission hit against the light sample it competes with (MIS),
+// or against nothing: after a specular bounce, and when only one of the two
+// estimators runs.
+__device__ __forceinline__ float emission_weight(const DevScene& s, const PathParams& pp, uint32_t geom, bool prev_spec,
+                                                 float prev_pdf, float t, f3 d, f3 Ng) {
+    if (prev_spec || pp.estimator == 2u) return 1.f;
+    const int li = __ldg(s.geom_light + geom);
+    if (li < 0) return 1.f;
+    if (pp.estimator == 1u) return 0.f;  // this light was sampled directly
+    const float cos_l = -dot(d, Ng);
+    const float lpdf = (t * t) / (cos_l * s.lights[li].area) * (1.0f / (float)s.n_lights);
+    return power_heuristic(prev_pdf, lpdf);
+}
+
+// A path that leaves the scene: throughput times the environment, without MIS
+// (the environment is not sampled as a light), integrator.cpp:545-552.
+__device__ __forceinline__ void shade_miss(const DevScene& s, const PathParams& pp, const float4 d4, const float4 b4,
+                                           ShadeOut& out) {
+    out.Lsum = hmul(xyz(b4), env_radiance(s, xyz(d4)));
+    out.film_idx = __float_as_uint(b4.w) / pp.spp;
+}
+
+// One vertex of a plain material (kPlainClass: at most one lobe, diffuse about
+// the shading normal), as shade_vertex shades it, bit for bit: with one lobe
+// its selection probability is wsum / wsum, the lobe's value and pdf are both
+// max(cos, 0) / pi, and neither the incident direction nor the frame is needed
+// for the light sample. Most vertices of most scenes are of
+// this kind, and the general function holds arrays over eight lobes and calls
+// the 21-way lobe switch twice.
+template <bool kAttr>
+__device__ __forceinline__ void shade_plain(const DevScene& s, const PathParams& pp, const float4 hit, const float4 o4,
+                                            const float4 d4, const float4 b4, unsigned long long rng_state,
+                                            ShadeOut& out) {
+    const int rec = __float_as_int(hit.w);
+    const uint32_t pid = __float_as_uint(b4.w);
+    const uint32_t flags = __float_as_uint(d4.w);
+    const uint32_t depth = flags & 0xffu;
+    Pcg rng;
+    rng.state = rng_state;
+    rng.inc = ((uint64_t)pid << 1u) | 1u;
+    float u[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) u[k] = rng.nextf();
+
+    const float4* tp = s.tris + (size_t)rec * 3;
+    const float4 ta = __ldg(tp), tb = __ldg(tp + 1), tc = __ldg(tp + 2);
+    const uint32_t m = __float_as_uint(tc.w);
+    const f3 v0 = xyz(ta), v1 = xyz(tb), v2 = xyz(tc);
+    const f3 Ng = normalize(cross(v1 - v0, v2 - v0)), d = xyz(d4);
+    f3 N = Ng, P = xyz(o4) + d * hit.x;
+    if (kAttr && s.tri_nrm) smooth_hit(s, rec, hit, v0, v1, v2, N, P);
+    const float4 plain = __ldg(s.mat_plain + m);
+    f3 lw = xyz(plain);
+    if (kAttr && s.mat_tex) {
+        const int32_t mtex = __ldg(s.mat_tex + m);
+        if (mtex >= 0) lw = hmul(lw, hit_tint(s, rec, hit, mtex));
+    }
+    f3 beta = xyz(b4);
+    out.film_idx = pid / pp.spp;
+    if (plain.w != 0.f && dot(d, N) < 0.f)  // the material emits
+        out.Lsum = hmul(beta, ld3(s.materials[m].Le)) *
+                   emission_weight(s, pp, __float_as_uint(tb.w), (flags & kSpecularFlag) != 0, o4.w, hit.x, d, Ng);
+    const float wsum = (lw.x * beta.x + lw.y * beta.y + lw.z * beta.z) * (1.f / (beta.x + beta.y + beta.z));
+    if (!(wsum > 0.f)) return;
+    const float lp = wsum <= 3.402823466e38f ? 1.f : __int_as_float(0x7fffffff);  // inf / inf
+
+    if (pp.estimator != 2u && s.n_lights > 0) {
+        const LightSample ls = sample_light(s, P, u[0], u[1], u[2], u[3]);
+        if (ls.lit) {
+            const float e = fmaxf(dot(ls.dir, N), 0.f) * kInvPi;
+            const f3 f = lw * e;
+            if (!is_zero(f)) {
+                const float w = ls.point || pp.estimator == 1u ? 1.f : power_heuristic(ls.pdf, lp * e);
+                const f3 Le_l = ls.point ? ls.Le * (1.f / (ls.dist2 * 0.1f)) : ls.Le;
+                const f3 c = hmul(hmul(beta, f), Le_l) * (w / ls.pdf);
+                out.shadow = true;
+                out.s_o = make_float4(P.x, P.y, P.z, ls.dist - kRayEps);
+                out.s_d = make_float4(ls.dir.x, ls.dir.y, ls.dir.z, __uint_as_float(out.film_idx));
+                out.s_c = make_float4(c.x, c.y, c.z, __uint_as_float(flags >> kJobShift));
+            }
+        }
+    }
+    if (depth + 1 >= pp.max_depth) return;
+    if (depth >= pp.rr_min) {
+        const float prob = fminf(max_comp(beta) * 0.9025f, 0.99f);
+        if (prob < u[4]) return;
+        beta = beta * (1.f / prob);
+    }
+    const f3 wo = cosine_hemisphere(u[6], u[7]);
+    const float e = fmaxf(wo.y, 0.f) * kInvPi;
+    const float pdf = lp * e;
+    if (!(pdf > 0.f)) return;
+    beta = hmul(beta, (lw * e) * (1.f / pdf));
+    if (is_zero(beta)) return;
+    const f3 dn = normalize(Frame(N).to_world(wo));
+    out.cont = true;
+    out.o_next = make_float4(P.x, P.y, P.z, pdf);
+    out.d_next = make_float4(dn.x, dn.y, dn.z, __uint_as_float((depth + 1) | (flags & kJobMask)));
+    out.b_next = make_float4(beta.x, beta.y, beta.z, b4.w);
+    out.rng_next = rng.state;
+}
+
 // One shaded path vertex: emission, next-event estimation (the shadow ray is
 // returned, not traced), roulette and direction sampling. `raw` holds the
 // guiding network's outputs for this path (guided mode only). kAttr = false
@@ -395,34 +563,11 @@ __device__ __forceinline__ void shade_vertex(const DevScene& s, const PathParams
         const f3 Ng = normalize(cross(v1 - v0, v2 - v0));
         const f3 d = xyz(d4);
         f3 P = xyz(o4) + d * hit.x;
-        // shading normal: the interpolated vertex normal, with the shading
-        // point moved off the flat triangle by the shadow-terminator offset
-        // (Hanika 2021), as TriangleMesh::post_hit does (shape.cpp:628-656)
         f3 Ns = Ng;
-        if (kAttr && s.tri_nrm) {
-            const float4 m0 = __ldg(s.tri_nrm + (size_t)rec * 3);
-            if (m0.w != 0.f) {
-                const f3 n0 = xyz(m0), n1 = xyz(__ldg(s.tri_nrm + (size_t)rec * 3 + 1)),
-                         n2 = xyz(__ldg(s.tri_nrm + (size_t)rec * 3 + 2));
-                const float b0 = 1.f - hit.y - hit.z;
-                Ns = normalize(n0 * b0 + n1 * hit.y + n2 * hit.z);
-                const f3 Pb = v0 * b0 + v1 * hit.y + v2 * hit.z;
-                const float e0 = fminf(0.f, dot(Pb - v0, n0)), e1 = fminf(0.f, dot(Pb - v1, n1)),
-                            e2 = fminf(0.f, dot(Pb - v2, n2));
-                P = Pb - (n0 * (b0 * e0) + n1 * (hit.y * e1) + n2 * (hit.z * e2));
-            }
-        }
-        // texture tint of the material at the hit's uv (interpolated vertex
-        // uvs; the barycentrics of vertices 1, 2 when the mesh has none)
+        if (kAttr && s.tri_nrm) smooth_hit(s, rec, hit, v0, v1, v2, Ns, P);
         const int32_t mtex = kAttr && s.mat_tex ? __ldg(s.mat_tex + __float_as_uint(tc.w)) : -1;
         const bool textured = mtex >= 0;
-        f3 tint = mk(1.f, 1.f, 1.f);
-        if (textured) {
-            const float2 q0 = s.tri_uv[(size_t)rec * 3], q1 = s.tri_uv[(size_t)rec * 3 + 1],
-                         q2 = s.tri_uv[(size_t)rec * 3 + 2];
-            const float b0 = 1.f - hit.y - hit.z;
-            tint = tex_eval(s, mtex, b0 * q0.x + hit.y * q1.x + hit.z * q2.x, b0 * q0.y + hit.y * q1.y + hit.z * q2.y);
-        }
+        const f3 tint = textured ? hit_tint(s, rec, hit, mtex) : mk(1.f, 1.f, 1.f);
         const Frame fr(Ns);
         const f3 wi = -fr.to_local(d);
         f3 beta = xyz(b4);
@@ -434,20 +579,7 @@ __device__ __forceinline__ void shade_vertex(const DevScene& s, const PathParams
         // single_emissive_surface, integrator.cpp:454)
         const f3 Le = ld3(mat.Le);
         if (!is_zero(Le) && dot(d, Ns) < 0.f) {
-            float w = 1.f;
-            if (!prev_spec && pp.estimator != 2u) {
-                const int li = __ldg(s.geom_light + geom);
-                if (li >= 0) {
-                    if (pp.estimator == 1u) {
-                        w = 0.f;  // NEE only: after a non-specular bounce this light was sampled directly
-                    } else {
-                        const float cos_l = -dot(d, Ng);
-                        const float lpdf = (hit.x * hit.x) / (cos_l * s.lights[li].area) * (1.0f / (float)nl);
-                        w = power_heuristic(prev_pdf, lpdf);
-                    }
-                }
-            }
-            Lsum = Lsum + hmul(beta, Le) * w;
+            Lsum = Lsum + hmul(beta, Le) * emission_weight(s, pp, geom, prev_spec, prev_pdf, hit.x, d, Ng);
             // MIS-weighted, like the next-event samples it pairs with
             if (kGuided && gs.recs) propagate(gs.recs, rbase, depth, Lsum);
         }
@@ -478,32 +610,11 @@ __device__ __forceinline__ void shade_vertex(const DevScene& s, const PathParams
 
         // 2. next-event estimation (none when sampling the BSDF only)
         if (pp.estimator != 2u && nl > 0 && any_smooth && wsum > 0.f) {
-            const uint32_t li = min((uint32_t)(u[0] * (float)nl), nl - 1);
-            const DevLight lt = s.lights[li];
-            // a point light (PointLight, light.cpp:18-31) has no triangles:
-            // its position is the one light_tris record it names
-            const bool point = lt.tri_count == 0;
-            f3 p, nlgt = mk(0.f, 0.f, 0.f);
-            if (point) {
-                p = xyz(__ldg(s.light_tris + (size_t)lt.tri_begin * 3));
-            } else {
-                const uint32_t kk = cdf_sample(s.light_cdf + lt.cdf_begin, lt.tri_count, u[1]);
-                const float4* lq = s.light_tris + (size_t)(lt.tri_begin + kk) * 3;
-                const f3 a0 = xyz(__ldg(lq)), a1 = xyz(__ldg(lq + 1)), a2 = xyz(__ldg(lq + 2));
-                const float su0 = sqrtf(u[2]);
-                const float bu0 = 1.f - su0;
-                const float bv0 = u[3] * su0;
-                p = a0 * bu0 + a1 * bv0 + a2 * (1.f - bu0 - bv0);
-                nlgt = normalize(cross(a1 - a0, a2 - a0));
-            }
-            const f3 lv = p - P;
-            const float dist2 = dot(lv, lv);
-            const float dist = sqrtf(dist2);
-            const f3 ldir = mk(lv.x / dist, lv.y / dist, lv.z / dist);
-            const float cos_l = point ? 1.f : -dot(ldir, nlgt);
-            if (cos_l > 0.f && dist2 > 0.f) {
-                // a delta light is picked with probability 1/nl and weighs no MIS
-                const float lpdf = point ? 1.0f / (float)nl : dist2 / (cos_l * lt.area) * (1.0f / (float)nl);
+            const LightSample ls = sample_light(s, P, u[0], u[1], u[2], u[3]);
+            const f3 ldir = ls.dir;
+            const float dist = ls.dist, dist2 = ls.dist2, lpdf = ls.pdf;
+            const bool point = ls.point;
+            if (ls.lit) {
                 const f3 wo = fr.to_local(ldir);
                 f3 f = mk(0.f, 0.f, 0.f);
                 float bpdf = 0.f;
@@ -523,7 +634,7 @@ __device__ __forceinline__ void shade_vertex(const DevScene& s, const PathParams
                 if (!is_zero(f)) {
                     const float w = point || pp.estimator == 1u ? 1.f : power_heuristic(lpdf, bpdf);
                     // PointLight::sample's falloff: radiance / (0.1 |d|^2)
-                    const f3 Le_l = point ? ld3(lt.Le) * (1.f / (dist2 * 0.1f)) : ld3(lt.Le);
+                    const f3 Le_l = point ? ls.Le * (1.f / (dist2 * 0.1f)) : ls.Le;
                     const f3 c = hmul(hmul(beta, f), Le_l) * (w / lpdf);
                     out.shadow = true;
                     out.s_o = make_float4(P.x, P.y, P.z, dist - kRayEps);
@@ -640,7 +751,8 @@ __device__ __forceinline__ void shade_vertex(const DevScene& s, const PathParams
                     for (uint32_t k = 0; k < nlobes; ++k) {
                         const kz_lobe& lb = mat.lobes[k];
                         if (lobe_is_delta(lb.closure_id)) continue;
-                        const LobeEval e = lobe_eval(lb, wi, smp.wo);
+                        // the sampled lobe's own value came with the sample
+                        const LobeEval e = k == sel ? LobeEval{smp.f, smp.pdf} : lobe_eval(lb, wi, smp.wo);
                         f = f + hmul(lobe_weight(lb, textured, tint), e.f);
                         pdf += lp[k] * e.pdf;
                     }
@@ -667,14 +779,10 @@ __device__ __forceinline__ void shade_vertex(const DevScene& s, const PathParams
         out.Lsum = Lsum;
         out.film_idx = film_idx;
     } else if (s.has_env) {
-        // a miss: throughput times the environment, without MIS (the
-        // environment is not sampled as a light), integrator.cpp:545-552
-        const uint32_t pid = __float_as_uint(b4.w);
-        out.Lsum = hmul(xyz(b4), env_radiance(s, xyz(d4)));
-        out.film_idx = pid / pp.spp;
+        shade_miss(s, pp, d4, b4, out);
         if (kGuided && gs.recs) {
             const uint32_t depth = __float_as_uint(d4.w) & 0xffu;
-            propagate(gs.recs, ((uint64_t)pid - gs.pass_first) * pp.max_depth, depth, out.Lsum);
+            propagate(gs.recs, ((uint64_t)__float_as_uint(b4.w) - gs.pass_first) * pp.max_depth, depth, out.Lsum);
         }
     }
 }
@@ -724,7 +832,7 @@ __device__ __forceinline__ void batch_trace_shadow(AnySmem& m, const DevJob* __r
     uint32_t dn = 0, dt = 0;
     DevScene ls;
     persistent_any_in<false, true>(
-        m, ls, ctr->n_shadow, &ctr->shadow_next,
+        m, ls, ctr->queue.shadow, &ctr->shadow_next,
         [&](uint32_t k, TRay& r, float& tmax) {
             const float4 o = sq.o4[k], d = sq.d4[k];
             trace_fields(ls, jobs[__float_as_uint(sq.c4[k].w)].scene);
@@ -762,10 +870,11 @@ __device__ __forceinline__ void plan_iteration(DevCounters* c, uint32_t cap, boo
     c->gen_slot = c->n_active;
     c->next_path += n_new;
     c->n_active += n_new;
-    c->n_next = 0;
-    c->n_shadow = 0;
+    c->n_append = 0;
     c->trace_next = 0;
     c->shadow_next = 0;
+    c->heavy_next = 0;
+    for (int k = 0; k < kHeavyClasses; ++k) c->heavy[k] = 0;
     if (c->n_active) {
         c->iterations += 1;
         c->path_bounces += c->n_active;
@@ -774,11 +883,41 @@ __device__ __forceinline__ void plan_iteration(DevCounters* c, uint32_t cap, boo
 
 // End of an iteration: the continuing paths become the next wavefront.
 __device__ __forceinline__ void finish_iteration(DevCounters* c) {
-    c->shadow_rays += c->n_shadow;
-    c->n_active = c->n_next;
+    c->shadow_rays += c->queue.shadow;
+    c->n_active = c->queue.next;
 }
 
 inline unsigned grid_for(uint64_t n, unsigned block) { return (unsigned)((n + block - 1) / block); }
+
+// Slots of a vertex's continuing path and shadow ray in the two queues, one
+// 64-bit atomic per warp for both. Every lane of the warp calls it.
+struct AppendSlots {
+    uint32_t cont, shadow;
+};
+__device__ __forceinline__ AppendSlots warp_append_pair(bool cont, bool shadow, DevCounters* ctr) {
+    const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
+    const uint32_t bc = __ballot_sync(0xFFFFFFFFu, cont), bs = __ballot_sync(0xFFFFFFFFu, shadow);
+    unsigned long long base = 0;
+    if (lane == 0 && (bc | bs))
+        base = atomicAdd(&ctr->n_append, ((unsigned long long)__popc(bs) << 32) | (unsigned)__popc(bc));
+    base = __shfl_sync(0xFFFFFFFFu, base, 0);
+    return AppendSlots{(uint32_t)base + __popc(bc & lt), (uint32_t)(base >> 32) + __popc(bs & lt)};
+}
+
+__device__ __forceinline__ void store_next(const PathSoA& out, const ShadowSoA& sq, const ShadeOut& so,
+                                           const AppendSlots& at) {
+    if (so.cont) {
+        out.o4[at.cont] = so.o_next;
+        out.d4[at.cont] = so.d_next;
+        out.b4[at.cont] = so.b_next;
+        out.rng[at.cont] = so.rng_next;
+    }
+    if (so.shadow) {
+        sq.o4[at.shadow] = so.s_o;
+        sq.d4[at.shadow] = so.s_d;
+        sq.c4[at.shadow] = so.s_c;
+    }
+}
 
 // Blocks of `block` threads resident on the whole device for kernel f.
 template <typename F>
@@ -791,7 +930,8 @@ static unsigned resident_grid(F f, unsigned block) {
 }
 
 // Shading kind of a traced path: 0 a miss, 1 + the material's shading class
-// for a hit (diffuse-like, glossy, delta, no lobe).
+// (kz_internal.h) for a hit, kNoPath for a thread without one.
+constexpr uint32_t kNoPath = 1u + kNumClasses, kNumKinds = kNoPath + 1u;
 __device__ __forceinline__ uint32_t shade_kind(const DevScene& s, const float4 hit) {
     const int rec = __float_as_int(hit.w);
     if (rec < 0) return 0u;
@@ -799,28 +939,30 @@ __device__ __forceinline__ uint32_t shade_kind(const DevScene& s, const float4 h
     return 1u + __ldg(s.mat_class + m);
 }
 
-// Regroups a block's paths by kind (0..5, 5 = no path) before they are
-// shaded, so each warp runs one branch of shade_vertex: a counting sort in
-// shared memory; returns the path index this thread shades. The order within
+// Regroups a block's paths by kind before they are shaded, so each warp runs
+// one branch of the shading: a counting sort in shared memory; returns the
+// path index this thread shades and sets `kind` to its kind. The order within
 // a kind is arbitrary; each path's result is not. blockDim.x <= 256.
-__device__ __forceinline__ uint32_t block_group_by_kind(uint32_t i, uint32_t kind) {
-    __shared__ uint32_t s_cnt[6];
+__device__ __forceinline__ uint32_t block_group_by_kind(uint32_t i, uint32_t& kind) {
+    __shared__ uint32_t s_cnt[kNumKinds];
     __shared__ uint32_t s_perm[256];
-    if (threadIdx.x < 6) s_cnt[threadIdx.x] = 0u;
+    if (threadIdx.x < kNumKinds) s_cnt[threadIdx.x] = 0u;
     __syncthreads();
     const uint32_t rank = atomicAdd(&s_cnt[kind], 1u);
     __syncthreads();
     uint32_t first = 0u;
     for (uint32_t k = 0; k < kind; ++k) first += s_cnt[k];
-    s_perm[first + rank] = i;
+    s_perm[first + rank] = threadIdx.x | (kind << 16);
     __syncthreads();
-    return s_perm[threadIdx.x];
+    const uint32_t p = s_perm[threadIdx.x];
+    kind = p >> 16;
+    return i - threadIdx.x + (p & 0xFFFFu);
 }
 
-// Plain shading runs 6 blocks per SM (40 registers, ~770 bytes of spills to
-// L1): the kernel waits on dependent loads, and more warps hide more of
-// them. Terrain frame shade stage at 4 / 5 / 6 / 7 / 8 blocks per SM: 32.5 /
-// 31.6 / 31.1 / 31.9 / 31.9 ms (3 and 2 blocks, more registers: slower).
+// The one-kernel shading runs 6 blocks per SM (40 registers, ~860 bytes of
+// spills to L1): it waits on dependent loads, and more warps hide more of
+// them. Terrain frame shade stage, when this kernel shaded all of it, at 4 / 5 /
+// 6 / 7 / 8 blocks per SM: 32.5 / 31.6 / 31.1 / 31.9 / 31.9 ms.
 #ifndef KZ_SHADE_MIN_BLOCKS
 #define KZ_SHADE_MIN_BLOCKS 6
 #endif
@@ -830,15 +972,11 @@ __device__ __forceinline__ uint32_t block_group_by_kind(uint32_t i, uint32_t kin
 #ifndef KZ_SHADE_GUIDED_MIN_BLOCKS
 #define KZ_SHADE_GUIDED_MIN_BLOCKS 3
 #endif
-// KZ_SHADE_SORT: group each block's paths by kind (miss, material shading
-// class) before shading them. Measured on the terrain frame: shade stage
-// 40.4 -> 33.4 ms, trace +1.3 ms (the next wavefront's order changes), frame
-// 1,441 -> 1,480 Mpaths*bounces/s. (Also writing the continuing paths
+// Each block's paths are grouped by kind (miss, material shading class) before
+// they are shaded: without it a warp holds several kinds and runs them in turn
+// (8.2 of 32 lanes active against 19.7). (Also writing the continuing paths
 // grouped by the octant of their next direction, one atomic per block,
 // measured trace -3.0 ms but shade +4.2 ms: not kept.)
-#ifndef KZ_SHADE_SORT
-#define KZ_SHADE_SORT 1
-#endif
 template <bool kGuided, bool kAttr = true>
 __global__ void __launch_bounds__(256, kGuided ? KZ_SHADE_GUIDED_MIN_BLOCKS : KZ_SHADE_MIN_BLOCKS)
     k_shade(DevScene s, PathParams pp, PathSoA in, uint32_t n_in, PathSoA out,
@@ -846,29 +984,164 @@ __global__ void __launch_bounds__(256, kGuided ? KZ_SHADE_GUIDED_MIN_BLOCKS : KZ
                                                GuideShade gs, const uint32_t* n_dev) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (n_dev) n_in = *n_dev;
-#if KZ_SHADE_SORT
-    i = block_group_by_kind(i, i < n_in ? shade_kind(s, in.hit[i]) : 5u);
-#endif
+    if (blockIdx.x * blockDim.x >= n_in) return;  // the grid covers the wavefront's capacity
+    uint32_t kind = i < n_in ? shade_kind(s, in.hit[i]) : kNoPath;
+    i = block_group_by_kind(i, kind);
     ShadeOut so;
-    if (i < n_in) {
+    if (!kGuided && kind == 1u + kPlainClass)
+        shade_plain<kAttr>(s, pp, in.hit[i], in.o4[i], in.d4[i], in.b4[i], in.rng[i], so);
+    else if (i < n_in)
         shade_vertex<kGuided, kAttr>(s, pp, in.hit[i], in.o4[i], in.d4[i], in.b4[i], in.rng[i], gs,
                                      kGuided ? gs.raw + (size_t)i * kGuideOut : nullptr, so);
-        if (!is_zero(so.Lsum)) film_add(film, film64, so.film_idx, so.Lsum);
+    if (!is_zero(so.Lsum)) film_add(film, film64, so.film_idx, so.Lsum);
+    const AppendSlots at = warp_append_pair(so.cont, so.shadow, ctr);
+    store_next(out, sq, so, at);
+}
+
+// ------------------------------------------------------------------ split shading
+// Large wavefronts are shaded by two kernels. k_shade_plain goes over all
+// paths once: it finishes the misses and the plain vertices itself and sorts
+// the others into a queue per material class. k_shade_heavy then takes the
+// queues 32 paths of one class at a time, the longest class first. In one
+// kernel the general vertex sets the registers (40 with 860 bytes of spills),
+// and a block waits for its slowest warp, which a Beckmann sample's FP64 search
+// makes ten times slower than the rest. Both wait on dependent loads; the
+// plain pass moves about 230 bytes a path, the heavy one is left with the lobe
+// switch and FP64. Shade stage, one kernel before / two: terrain 1080p 30.8 /
+// 23.6 ms (11.7 of it plain), slit room 12.1 / 6.9 ms, 641 x 359 frame of
+// mixed materials 16.3 / 3.0 ms, box room 0.59 / 0.45 ms.
+// Blocks per SM, terrain + materials shade: plain (256 threads) 4 / 5 / 6 / 8:
+// 27.5 / 27.6 / 28.1 / 32.8 ms; heavy (128 threads) 4 / 6 / 8 / 12: 27.8 /
+// 27.6 / 27.4 / 28.3 ms.
+#ifndef KZ_PLAIN_MIN_BLOCKS
+#define KZ_PLAIN_MIN_BLOCKS 4
+#endif
+#ifndef KZ_HEAVY_MIN_BLOCKS
+#define KZ_HEAVY_MIN_BLOCKS 8
+#endif
+constexpr int kHeavyThreads = 128;
+
+// Queue place of the k-th path of a heavy class: two arrays of the wavefront's
+// capacity, each filled from both ends (a path is in one class only).
+__device__ __forceinline__ uint32_t* heavy_slot(const HeavyQueue& q, uint32_t cls, uint32_t k) {
+    uint32_t* a = q.paths + (cls >= 2u ? q.cap : 0u);
+    return (cls & 1u) ? a + (q.cap - 1u - k) : a + k;
+}
+
+template <bool kAttr, bool kJobs>
+__global__ void __launch_bounds__(256, KZ_PLAIN_MIN_BLOCKS)
+    k_shade_plain(DevScene scene, PathParams params, const DevJob* __restrict__ jobs, PathSoA in, PathSoA out,
+                  ShadowSoA sq, HeavyQueue hq, DevCounters* ctr, float* film, double* film64) {
+    // per warp: appended paths and shadow rays, then the four heavy classes; double buffered over the rounds
+    __shared__ unsigned long long s_app[2][8];
+    __shared__ uint32_t s_heavy[2][kHeavyClasses][8];
+    const uint32_t n = ctr->n_active, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, lt = (1u << lane) - 1u;
+    uint32_t buf = 0;
+    for (uint32_t base = blockIdx.x * 256u; base < n; base += gridDim.x * 256u, buf ^= 1u) {
+        const uint32_t i = base + threadIdx.x;
+        ShadeOut so;
+        uint32_t heavy = kHeavyClasses;  // none
+        if (i < n) {
+            const float4 hit = in.hit[i], d4 = in.d4[i];
+            const DevJob* J = kJobs ? jobs + (__float_as_uint(d4.w) >> kJobShift) : nullptr;
+            const DevScene& s = kJobs ? J->scene : scene;
+            const PathParams& pp = kJobs ? J->pp : params;
+            const uint32_t kind = shade_kind(s, hit);
+            if (kind == 1u + kPlainClass) shade_plain<kAttr>(s, pp, hit, in.o4[i], d4, in.b4[i], in.rng[i], so);
+            else if (kind) heavy = kind - 2u;
+            else if (s.has_env) shade_miss(s, pp, d4, in.b4[i], so);
+            if (!is_zero(so.Lsum)) film_add(kJobs ? J->film : film, kJobs ? nullptr : film64, so.film_idx, so.Lsum);
+        }
+        // one atomic per queue and block, not per warp
+        const uint32_t bc = __ballot_sync(0xFFFFFFFFu, so.cont), bs = __ballot_sync(0xFFFFFFFFu, so.shadow);
+        uint32_t bh = 0;  // this lane's class among the warp's
+#pragma unroll
+        for (uint32_t c = 0; c < kHeavyClasses; ++c) {
+            const uint32_t b = __ballot_sync(0xFFFFFFFFu, heavy == c);
+            if (heavy == c) bh = b;
+            if (lane == 0) s_heavy[buf][c][warp] = __popc(b);
+        }
+        if (lane == 0) s_app[buf][warp] = ((unsigned long long)__popc(bs) << 32) | (unsigned)__popc(bc);
+        __syncthreads();
+        if (warp == 0) {  // lanes 8 c + w: warp w of class c
+            const uint32_t c = lane >> 3, w = lane & 7u;
+            const uint32_t v = s_heavy[buf][c][w];
+            uint32_t incl = v;
+#pragma unroll
+            for (uint32_t o = 1; o < 8; o <<= 1) {
+                const uint32_t x = __shfl_up_sync(0xFFFFFFFFu, incl, o, 8);
+                if (w >= o) incl += x;
+            }
+            uint32_t first = 0;
+            if (w == 7 && incl) first = atomicAdd(&ctr->heavy[c], incl);
+            s_heavy[buf][c][w] = __shfl_sync(0xFFFFFFFFu, first, 7, 8) + incl - v;
+        } else if (warp == 1 && lane < 8) {
+            const unsigned long long v = s_app[buf][lane];
+            unsigned long long incl = v, first = 0;
+#pragma unroll
+            for (uint32_t o = 1; o < 8; o <<= 1) {
+                const unsigned long long x = __shfl_up_sync(0xFFu, incl, o);
+                if (lane >= o) incl += x;
+            }
+            if (lane == 7 && incl) first = atomicAdd(&ctr->n_append, incl);
+            s_app[buf][lane] = __shfl_sync(0xFFu, first, 7) + incl - v;
+        }
+        __syncthreads();
+        const unsigned long long at = s_app[buf][warp];
+        store_next(out, sq, so, AppendSlots{(uint32_t)at + __popc(bc & lt), (uint32_t)(at >> 32) + __popc(bs & lt)});
+        if (heavy < kHeavyClasses) *heavy_slot(hq, heavy, s_heavy[buf][heavy][warp] + __popc(bh & lt)) = i;
     }
-    const bool cont = so.cont, shadow = so.shadow;
-    const uint32_t slot = warp_append(cont, &ctr->n_next);
-    if (cont) {
-        out.o4[slot] = so.o_next;
-        out.d4[slot] = so.d_next;
-        out.b4[slot] = so.b_next;
-        out.rng[slot] = so.rng_next;
+}
+
+template <bool kAttr, bool kJobs>
+__global__ void __launch_bounds__(kHeavyThreads, KZ_HEAVY_MIN_BLOCKS)
+    k_shade_heavy(DevScene scene, PathParams params, const DevJob* __restrict__ jobs, PathSoA in, PathSoA out,
+                  ShadowSoA sq, HeavyQueue hq, DevCounters* ctr, float* film, double* film64) {
+    const uint32_t lane = threadIdx.x & 31u;
+    for (;;) {
+        uint32_t p = 0;
+        if (lane == 0) p = atomicAdd(&ctr->heavy_next, 32u);
+        p = __shfl_sync(0xFFFFFFFFu, p, 0);
+        uint32_t cls = 0, n = 0;
+        for (; cls < kHeavyClasses; ++cls) {  // each class's range is rounded up to whole warps
+            n = ctr->heavy[cls];
+            const uint32_t r = (n + 31u) & ~31u;
+            if (p < r) break;
+            p -= r;
+        }
+        if (cls == kHeavyClasses) break;
+        ShadeOut so;
+        if (p + lane < n) {
+            const uint32_t i = *heavy_slot(hq, cls, p + lane);
+            const float4 d4 = in.d4[i];
+            const DevJob* J = kJobs ? jobs + (__float_as_uint(d4.w) >> kJobShift) : nullptr;
+            shade_vertex<false, kAttr>(kJobs ? J->scene : scene, kJobs ? J->pp : params, in.hit[i], in.o4[i], d4,
+                                       in.b4[i], in.rng[i], GuideShade{}, nullptr, so);
+            if (!is_zero(so.Lsum)) film_add(kJobs ? J->film : film, kJobs ? nullptr : film64, so.film_idx, so.Lsum);
+        }
+        store_next(out, sq, so, warp_append_pair(so.cont, so.shadow, ctr));
     }
-    const uint32_t sslot = warp_append(shadow, &ctr->n_shadow);
-    if (shadow) {
-        sq.o4[sslot] = so.s_o;
-        sq.d4[sslot] = so.s_d;
-        sq.c4[sslot] = so.s_c;
-    }
+}
+
+// Wavefronts from this capacity on are shaded by the two kernels; smaller ones
+// by the one: there the second launch and its dependent queue cost what the
+// split saves (65,537 Li rays of depth 5: 0.94 ms with one kernel, 1.01 with
+// two; a 25,220-path preview of mixed materials 1.16 and 1.11).
+#ifndef KZ_SPLIT_SHADING
+#define KZ_SPLIT_SHADING (1u << 18)
+#endif
+template <bool kAttr, bool kJobs>
+static int launch_split_shading(const DevScene& s, const PathParams& pp, const DevJob* jobs, PathSoA in, uint32_t cap,
+                                PathSoA out, ShadowSoA sq, HeavyQueue hq, DevCounters* ctr, float* film,
+                                double* film64, bool heavy, cudaStream_t st) {
+    static const unsigned gp = resident_grid(k_shade_plain<kAttr, kJobs>, 256);
+    static const unsigned gh = resident_grid(k_shade_heavy<kAttr, kJobs>, kHeavyThreads);
+    k_shade_plain<kAttr, kJobs><<<std::min(gp, grid_for(cap, 256)), 256, 0, st>>>(s, pp, jobs, in, out, sq, hq, ctr,
+                                                                                film, film64);
+    if (!heavy) return 1;
+    k_shade_heavy<kAttr, kJobs><<<std::min(gh, grid_for(cap, kHeavyThreads)), kHeavyThreads, 0, st>>>(
+        s, pp, jobs, in, out, sq, hq, ctr, film, film64);
+    return 2;
 }
 
 }  // namespace

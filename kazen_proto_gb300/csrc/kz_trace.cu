@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(256) k_trace_shadow(DevScene s, ShadowSoA sq, 
                                                       double* film64, VRec* recs, NRec* nee, uint32_t max_depth) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t dn = 0, dt = 0;
-    if (i < ctr->n_shadow) {
+    if (i < ctr->queue.shadow) {
         const float4 o = sq.o4[i], d = sq.d4[i];
         TRay r = make_tray(xyz(o), xyz(d), kRayEps);
         bool overflow;
@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(256, KZ_TRACE_MINB) k_trace_shadow_persistent(
         }
     };
     persistent_any<kCount>(
-        s, ctr->n_shadow, &ctr->shadow_next,
+        s, ctr->queue.shadow, &ctr->shadow_next,
         [&](uint32_t k, TRay& r, float& tmax) {
             const float4 o = sq.o4[k], d = sq.d4[k];
             r = make_tray(xyz(o), xyz(d), kRayEps);
