@@ -415,7 +415,8 @@ kz_status kz_render_guided(kz_scene* scene, kz_guide* guide, const kz_camera* ca
  *    by device counters; the stage kernels find each path's scene, camera and
  *    film through its job index, so small jobs share the GPU instead of
  *    underfilling it. With use_graph, each batch of iterations is one CUDA
- *    graph launch (one host synchronisation per batch).
+ *    graph launch (one host synchronisation per batch); paths that fit into
+ *    the wavefront at once take one batch, which is launched directly.
  *  KZ_BATCH_MEGAKERNEL: one persistent kernel; lanes keep a path each and
  *    refill from a global path counter every refill_period vertices.
  *  KZ_BATCH_PERSISTENT: the wavefront's whole loop (every stage of every

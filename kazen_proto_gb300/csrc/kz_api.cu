@@ -218,7 +218,8 @@ struct kz_scene {
 
     // wavefront buffers
     DevBuf pa[5], pb[5], sh[3], heavy, ctr, film, film64;
-    kz::DevCounters* ctr_host = nullptr;  // pinned
+    kz::DevCounters* ctr_host = nullptr;  // pinned, ctr_host_n of them
+    size_t ctr_host_n = 0;
 
     bool cuda_ready = false;
 
@@ -323,6 +324,25 @@ kz_status alloc_paths(DevBuf* b, uint32_t cap, kz::PathSoA& p) {
     return KZ_OK;
 }
 
+// Counters of n iterations, on the device and (pinned) on the host.
+kz_status alloc_counters(kz_scene* s, size_t n) {
+    KZ_TRY(s->ctr.ensure(n * sizeof(kz::DevCounters)));
+    if (s->ctr_host_n >= n) return KZ_OK;
+    if (s->ctr_host) cudaFreeHost(s->ctr_host);
+    s->ctr_host = nullptr;
+    s->ctr_host_n = 0;
+    KZ_CUDA(cudaMallocHost((void**)&s->ctr_host, n * sizeof(kz::DevCounters)));
+    s->ctr_host_n = n;
+    return KZ_OK;
+}
+
+// Largest wavefront whose shadow rays are traced beside the next iteration's
+// paths. The joint kernel holds the closest-hit loop's shared memory, and so
+// less L1, for both; in return one tail of long rays is waited for, not two.
+// Joint / apart: 65,537 Li rays 0.54 / 0.63 ms, 262,144-path guided iterations
+// 8.1 / 8.7 ms a frame, 1 M-path box frame 0.82 / 0.86, 24 jobs in one batch
+// 6.2 / 6.4, 16 M-path slit room 23.3 / 23.0 and terrain 129.0 / 126.5.
+constexpr uint32_t kBothCap = 1u << 23;
 // The queue of split shading for wavefronts large enough for it (else none).
 kz_status alloc_heavy(kz_scene* s, uint32_t cap, kz::HeavyQueue& q) {
     if (cap < kz::split_shading_capacity()) return KZ_OK;
@@ -339,10 +359,17 @@ struct GuideHooks {
     float* raw = nullptr;
 };
 
-// Wavefront path tracing of `total` paths, driven by device-side counters:
-// the host enqueues batches of iterations (plan, generate, trace, [infer],
-// shade, shadow, finish) and synchronises once per batch. Contributions are
-// summed into film (and film64) on the device.
+// Wavefront path tracing of `total` paths, driven by device-side counters: the
+// host enqueues batches of iterations (generate, trace, [infer], shade) and
+// synchronises once per batch. An iteration's shadow rays are traced beside
+// the next one's paths, in one launch, in wavefronts up to kBothCap; in larger
+// ones, and with stage timing or fetch counts, they have their own. Contributions are summed into film (and film64) on the device.
+//
+// When all paths fit into the wavefront at once, only the first iteration
+// generates, a path has at most max_depth vertices, and so max_depth iterations
+// are enough: one batch, one synchronisation. The 256 x 256, 16 spp box frame
+// of depth 5 takes 18 launches and 0.82 ms; with two waves' worth of iterations
+// and planning kernels between them it took 84 and 1.20 ms.
 kz_status run_wavefront(kz_scene* s, const kz::DevCamera* cam, const kz_ray* rays_dev, uint64_t total,
                         const kz_render_config* cfg, float* film, double* film64, kz_render_stats* stats,
                         const kz::PathParams* pp_override = nullptr, const GuideHooks* gh = nullptr) {
@@ -364,20 +391,17 @@ kz_status run_wavefront(kz_scene* s, const kz::DevCamera* cam, const kz_ray* ray
     kz::ShadowSoA sq{s->sh[0].as<float4>(), s->sh[1].as<float4>(), s->sh[2].as<float4>()};
     kz::HeavyQueue hq;
     if (!gh) KZ_TRY(alloc_heavy(s, cap, hq));
-    KZ_TRY(s->ctr.ensure(sizeof(kz::DevCounters)));
-    kz::DevCounters* ctr = s->ctr.as<kz::DevCounters>();
-    cudaStream_t strm = s->stream;
-    {
-        kz::DevCounters init{};
-        init.total = total;
-        *s->ctr_host = init;
-        KZ_CUDA(cudaMemcpyAsync(ctr, s->ctr_host, sizeof(kz::DevCounters), cudaMemcpyHostToDevice, strm));
-    }
     const bool timing = (cfg->flags & KZ_RENDER_FLAG_TIMING) != 0;
     const bool count = (cfg->flags & KZ_RENDER_FLAG_COUNT) != 0;
-    // one batch covers the life of two waves of paths: the host waits for the
-    // device once per batch, and fewer waits leave fewer idle gaps
-    const uint32_t batch = 2 * std::max<uint32_t>(4, cfg->max_depth + 1);
+    const bool both = !timing && !count && cap <= kBothCap;
+    const bool one_wave = total <= cap;
+    // otherwise one batch covers the life of two waves of paths: the host waits
+    // for the device once per batch, and fewer waits leave fewer idle gaps
+    const uint32_t batch = one_wave ? cfg->max_depth : 2 * std::max<uint32_t>(4, cfg->max_depth + 1);
+    KZ_TRY(alloc_counters(s, batch + 1));  // the first: the state before the batch
+    kz::DevCounters* ctr = s->ctr.as<kz::DevCounters>();
+    cudaStream_t strm = s->stream;
+    KZ_CUDA(cudaMemsetAsync(ctr, 0, (batch + 1) * sizeof(kz::DevCounters), strm));
     std::vector<cudaEvent_t> ev;
     if (timing) {
         ev.assign(5 * (size_t)batch, nullptr);
@@ -397,33 +421,46 @@ kz_status run_wavefront(kz_scene* s, const kz::DevCamera* cam, const kz_ray* ray
     } guard{ev};
     kz_render_stats st{};
     st.paths = total;
-    for (;;) {
+    const kz::GuideShade* gs = gh ? gh->gs : nullptr;
+    std::vector<uint8_t> generated(batch);
+    for (bool first_batch = true;; first_batch = false) {
         const NvtxRange batch_range("wavefront batch");
+        if (!first_batch) kz::launch_carry(ctr, batch + 1, ctr + batch, ctr + batch, strm);
+        const kz::DevCounters* last_gen = ctr;
         for (uint32_t it = 0; it < batch; ++it) {
             cudaEvent_t* e = timing ? &ev[5 * (size_t)it] : nullptr;
+            kz::DevCounters *cur = ctr + it + 1, *prev = ctr + it;
+            const uint32_t* n_active = &prev->queue.next;
             if (e) KZ_CUDA(cudaEventRecord(e[0], strm));
-            kz::launch_plan(ctr, cap, strm);
-            if (cam) kz::launch_generate_camera_dev(*cam, pp, A, ctr, cap, block, strm);
-            else kz::launch_generate_rays_dev(rays_dev, pp, A, ctr, cap, block, strm);
+            generated[it] = !one_wave || it == 0;
+            if (generated[it]) {
+                const kz::IterSlots slots{cur, prev, last_gen, total, cap};
+                if (cam) kz::launch_generate_camera_dev(*cam, pp, A, slots, block, strm);
+                else kz::launch_generate_rays_dev(rays_dev, pp, A, slots, block, strm);
+                last_gen = cur;
+                n_active = &cur->n_active;
+                st.kernel_launches += 1;
+            }
             if (e) KZ_CUDA(cudaEventRecord(e[1], strm));
-            kz::launch_trace_paths_dev(s->dev, A, cap, ctr, count, block, strm);
-            if (gh) kz::launch_guide_infer_paths_dev(s->dev, A, cap, ctr, gh->gd, gh->raw, strm);
-            if (e) KZ_CUDA(cudaEventRecord(e[2], strm));
-            st.kernel_launches +=
-                kz::launch_shade_dev(s->dev, pp, A, cap, B, sq, hq, ctr, film, film64, gh ? gh->gs : nullptr, block, strm);
-            if (e) KZ_CUDA(cudaEventRecord(e[3], strm));
-            if (gh)
-                kz::launch_trace_shadow_guided(s->dev, sq, cap, ctr, film, film64, gh->gs->recs, gh->gs->nee,
-                                               pp.max_depth, block, strm);
+            if (both && it > 0)
+                kz::launch_trace_both(s->dev, A, cap, n_active, cur, sq, prev, film, film64, gs, pp.max_depth, strm);
             else
-                kz::launch_trace_shadow_dev(s->dev, sq, cap, ctr, count, film, film64, strm);
-            kz::launch_finish(ctr, strm);
+                kz::launch_trace_paths_dev(s->dev, A, cap, n_active, cur, count, strm);
+            if (gh) kz::launch_guide_infer_paths_dev(s->dev, A, cap, n_active, gh->gd, gh->raw, strm);
+            if (e) KZ_CUDA(cudaEventRecord(e[2], strm));
+            st.kernel_launches += 1 + (gh ? 1 : 0) +
+                                  kz::launch_shade_dev(s->dev, pp, A, cap, B, sq, hq, cur, n_active, film, film64, gs,
+                                                       block, strm);
+            if (e) KZ_CUDA(cudaEventRecord(e[3], strm));
+            if (!both || it + 1 == batch) {
+                kz::launch_trace_shadow_dev(s->dev, sq, cap, cur, count, film, film64, gs, pp.max_depth, strm);
+                st.kernel_launches += 1;
+            }
             if (e) KZ_CUDA(cudaEventRecord(e[4], strm));
-            st.kernel_launches += gh ? 6 : 5;
             std::swap(A, B);
         }
         KZ_CUDA(cudaGetLastError());
-        KZ_CUDA(cudaMemcpyAsync(s->ctr_host, ctr, sizeof(kz::DevCounters), cudaMemcpyDeviceToHost, strm));
+        KZ_CUDA(cudaMemcpyAsync(s->ctr_host, ctr, (batch + 1) * sizeof(kz::DevCounters), cudaMemcpyDeviceToHost, strm));
         KZ_CUDA(cudaStreamSynchronize(strm));
         if (timing)
             for (uint32_t it = 0; it < batch; ++it) {
@@ -434,19 +471,19 @@ kz_status run_wavefront(kz_scene* s, const kz::DevCamera* cam, const kz_ray* ray
                 st.shade_ms += ms[2];
                 st.shadow_ms += ms[3];
             }
-        const kz::DevCounters& hc = *s->ctr_host;
-        if (hc.status) return fail((kz_status)hc.status, "device status %u during rendering", hc.status);
-        if (hc.n_active == 0 && hc.next_path >= hc.total) break;
-    }
-    const kz::DevCounters& hc = *s->ctr_host;
-    st.path_bounces = hc.path_bounces;
-    st.shadow_rays = hc.shadow_rays;
-    st.iterations = hc.iterations;
-    if (count) {
-        st.closest_node_fetches = hc.fetch[0];
-        st.closest_tri_fetches = hc.fetch[1];
-        st.shadow_node_fetches = hc.fetch[2];
-        st.shadow_tri_fetches = hc.fetch[3];
+        for (uint32_t it = 0; it < batch; ++it) {
+            const kz::DevCounters& hc = s->ctr_host[it + 1];
+            if (hc.status) return fail((kz_status)hc.status, "device status %u during rendering", hc.status);
+            const uint32_t n = generated[it] ? hc.n_active : s->ctr_host[it].queue.next;
+            st.path_bounces += n;
+            st.shadow_rays += hc.queue.shadow;
+            st.iterations += n ? 1 : 0;
+            st.closest_node_fetches += hc.fetch[0];
+            st.closest_tri_fetches += hc.fetch[1];
+            st.shadow_node_fetches += hc.fetch[2];
+            st.shadow_tri_fetches += hc.fetch[3];
+        }
+        if (one_wave || (s->ctr_host[batch].queue.next == 0 && s->ctr_host[batch].next_path >= total)) break;
     }
     if (stats) *stats = st;
     return KZ_OK;
@@ -463,7 +500,6 @@ kz_status init_cuda(kz_scene* s) {
     s->cuda_ready = true;  // from here on the destructor releases what exists
     KZ_CUDA(cudaStreamCreateWithFlags(&s->own_stream, cudaStreamNonBlocking));
     KZ_CUDA(cudaMallocHost((void**)&s->status_host, sizeof(uint32_t)));
-    KZ_CUDA(cudaMallocHost((void**)&s->ctr_host, sizeof(kz::DevCounters)));
     if (!s->stream) s->stream = s->own_stream;
     KZ_TRY(s->status.ensure(sizeof(uint32_t)));
     KZ_CUDA(cudaMemset(s->status.ptr, 0, sizeof(uint32_t)));
@@ -1570,7 +1606,6 @@ kz_status kz_render_guided(kz_scene* s, kz_guide* g, const kz_camera* camera, co
     if (film64) KZ_CUDA(cudaMemsetAsync(film64, 0, npix * 24, strm));
     const uint64_t want = cfg->wavefront_size ? cfg->wavefront_size : KZ_RENDER_DEFAULT_WAVEFRONT;
     const uint32_t cap = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(want, per_pass));
-    const uint32_t block = cfg->block_size ? cfg->block_size : 256u;
     const uint64_t n_recs = per_pass * cfg->max_depth;
     KZ_TRY(g->recs.ensure(n_recs * sizeof(kz::VRec)));
     KZ_TRY(g->nee.ensure(n_recs * sizeof(kz::NRec)));
@@ -1731,45 +1766,61 @@ kz_status batch_wavefront(const kz_batch_job* jobs, uint32_t n_jobs, const kz_ba
     kz::ShadowSoA sq{s->sh[0].as<float4>(), s->sh[1].as<float4>(), s->sh[2].as<float4>()};
     kz::HeavyQueue hq;
     if (cfg.mode == KZ_BATCH_WAVEFRONT) KZ_TRY(alloc_heavy(s, cap, hq));
-    KZ_TRY(s->ctr.ensure(sizeof(kz::DevCounters)));
+    const bool persistent = cfg.mode == KZ_BATCH_PERSISTENT;
+    // refill period P: free wavefront slots take new paths every P-th
+    // iteration (P = 1: every iteration); in between the wavefront drains, so
+    // the generation launches are fewer and the live paths fewer too
+    const uint32_t period = std::max<uint32_t>(1, cfg.refill_period);
+    // all paths at once: as many iterations as vertices, and only the first
+    // generates (run_wavefront); else an even number of iterations per batch,
+    // so the path buffers end where they started and a captured batch can be
+    // replayed as is
+    const bool one_wave = !persistent && total <= cap;
+    uint32_t iters = max_depth;
+    if (!one_wave) {
+        iters = std::max<uint32_t>(4, max_depth + 1);
+        iters += iters & 1u;
+        if (iters % period) iters += period - iters % period;
+        iters += iters & 1u;
+    }
+    KZ_TRY(alloc_counters(s, iters + 1));
     kz::DevCounters* ctr = s->ctr.as<kz::DevCounters>();
     for (uint32_t j = 0; j < n_jobs; ++j) KZ_CUDA(cudaMemsetAsync(fptr[j], 0, npix[j] * 12, strm));
-    {
+    KZ_CUDA(cudaMemsetAsync(ctr, 0, (iters + 1) * sizeof(kz::DevCounters), strm));
+    if (persistent) {
         kz::DevCounters init{};
         init.total = total;
         *s->ctr_host = init;
         KZ_CUDA(cudaMemcpyAsync(ctr, s->ctr_host, sizeof(kz::DevCounters), cudaMemcpyHostToDevice, strm));
     }
-    // an even number of iterations per batch, so the path buffers end where
-    // they started and a captured batch can be replayed as is
-    uint32_t iters = std::max<uint32_t>(4, max_depth + 1);
-    iters += iters & 1u;
     // the texture tint is compiled out, and the second shading kernel left out, unless a job needs it
     bool textured = false, heavy = false;
     for (uint32_t j = 0; j < n_jobs; ++j) {
         textured |= jobs[j].scene->dev.mat_tex != nullptr || jobs[j].scene->dev.tri_nrm != nullptr;
         heavy |= jobs[j].scene->dev.has_heavy != 0;
     }
-    // refill period P: free wavefront slots take new paths every P-th
-    // iteration (P = 1: every iteration); in between the wavefront drains, so
-    // the generation launches are fewer and the live paths fewer too
-    const uint32_t period = std::max<uint32_t>(1, cfg.refill_period);
-    if (iters % period) iters += period - iters % period;
-    iters += iters & 1u;
+    // iterations 0 and on; the slots' first holds what the replay before left
+    const uint32_t last_gen = one_wave ? 0 : (iters - 1) / period * period;
+    const bool both = cap <= kBothCap;
     auto enqueue = [&]() {
         kz::PathSoA a = A, b = B;
+        kz::launch_carry(ctr, iters + 1, ctr + iters, ctr + last_gen + 1, strm);
+        const kz::DevCounters* gen_slot = ctr;
         for (uint32_t it = 0; it < iters; ++it) {
-            const bool gen = it % period == 0;
-            kz::launch_plan(ctr, cap, strm, gen);
-            if (gen) kz::launch_generate_batch_dev(djobs, n_jobs, a, ctr, cap, block, strm);
-            kz::launch_trace_paths_batch(djobs, a, cap, ctr, strm);
-            kz::launch_shade_batch(djobs, a, cap, b, sq, hq, ctr, block, textured, heavy, strm);
-            kz::launch_trace_shadow_batch(djobs, sq, cap, ctr, strm);
-            kz::launch_finish(ctr, strm);
+            kz::DevCounters *cur = ctr + it + 1, *prev = ctr + it;
+            const uint32_t* n_active = &prev->queue.next;
+            if (one_wave ? it == 0 : it % period == 0) {
+                kz::launch_generate_batch_dev(djobs, n_jobs, a, kz::IterSlots{cur, prev, gen_slot, total, cap}, block,
+                                              strm);
+                gen_slot = cur;
+                n_active = &cur->n_active;
+            }
+            kz::launch_trace_both_batch(djobs, a, cap, n_active, cur, sq, it && both ? prev : nullptr, strm);
+            kz::launch_shade_batch(djobs, a, cap, b, sq, hq, cur, n_active, block, textured, heavy, strm);
+            if (!both || it + 1 == iters) kz::launch_trace_shadow_batch(djobs, sq, cap, cur, strm);
             std::swap(a, b);
         }
     };
-    const bool persistent = cfg.mode == KZ_BATCH_PERSISTENT;
     uint32_t coop_blocks = 0;
     if (persistent) {
         int sms = 0;
@@ -1783,6 +1834,7 @@ kz_status batch_wavefront(const kz_batch_job* jobs, uint32_t n_jobs, const kz_ba
         return kz::launch_batch_persistent(djobs, n_jobs, A, B, sq, ctr, cap, period, coop_blocks, textured, strm);
     };
     kz::prepare_batch_wavefront();
+    kz::prepare_batch_shading();
     cudaGraphExec_t exec = nullptr;
     struct ExecGuard {
         cudaGraphExec_t& e;
@@ -1790,7 +1842,9 @@ kz_status batch_wavefront(const kz_batch_job* jobs, uint32_t n_jobs, const kz_ba
             if (e) cudaGraphExecDestroy(e);
         }
     } xg{exec};
-    if (cfg.use_graph) {
+    // a batch that runs once is enqueued as it is: capturing and instantiating
+    // a graph costs more than its launches
+    if (cfg.use_graph && !one_wave) {
         cudaGraph_t graph = nullptr;
         KZ_CUDA(cudaStreamBeginCapture(strm, cudaStreamCaptureModeThreadLocal));
         cudaError_t le = cudaSuccess;
@@ -1819,18 +1873,31 @@ kz_status batch_wavefront(const kz_batch_job* jobs, uint32_t n_jobs, const kz_ba
             cudaEventDestroy(b);
         }
     } evg{e0, e1};
+    uint64_t bounces = 0, shadows = 0;
     KZ_CUDA(cudaEventRecord(e0, strm));
     for (;;) {
         if (exec) KZ_CUDA(cudaGraphLaunch(exec, strm));
         else if (persistent) KZ_CUDA(enqueue_persistent());
         else enqueue();
         KZ_CUDA(cudaGetLastError());
-        KZ_CUDA(cudaMemcpyAsync(s->ctr_host, ctr, sizeof(kz::DevCounters), cudaMemcpyDeviceToHost, strm));
+        KZ_CUDA(cudaMemcpyAsync(s->ctr_host, ctr, (iters + 1) * sizeof(kz::DevCounters), cudaMemcpyDeviceToHost, strm));
         KZ_CUDA(cudaStreamSynchronize(strm));
-        const kz::DevCounters& hc = *s->ctr_host;
-        if (hc.status) return fail((kz_status)hc.status, "device status %u during batched rendering", hc.status);
-        if (hc.n_active == 0 && hc.next_path >= hc.total) break;
-        if (persistent) return fail(KZ_ERR_CUDA, "persistent batch kernel ended with paths left");
+        const kz::DevCounters* hc = s->ctr_host;
+        for (uint32_t it = 0; it <= iters; ++it)
+            if (hc[it].status)
+                return fail((kz_status)hc[it].status, "device status %u during batched rendering", hc[it].status);
+        if (persistent) {
+            bounces = hc->path_bounces;
+            shadows = hc->shadow_rays;
+            if (hc->n_active == 0 && hc->next_path >= hc->total) break;
+            return fail(KZ_ERR_CUDA, "persistent batch kernel ended with paths left");
+        }
+        for (uint32_t it = 0; it < iters; ++it) {
+            const bool gen = one_wave ? it == 0 : it % period == 0;
+            bounces += gen ? hc[it + 1].n_active : hc[it].queue.next;
+            shadows += hc[it + 1].queue.shadow;
+        }
+        if (one_wave || (hc[iters].queue.next == 0 && hc[last_gen + 1].next_path >= total)) break;
     }
     for (uint32_t j = 0; j < n_jobs; ++j)
         kz::launch_scale(fptr[j], nullptr, npix[j] * 3, 1.0f / (float)jobs[j].spp, 0.0, strm);
@@ -1842,10 +1909,9 @@ kz_status batch_wavefront(const kz_batch_job* jobs, uint32_t n_jobs, const kz_ba
     float ms = 0.f;
     KZ_CUDA(cudaEventElapsedTime(&ms, e0, e1));
     if (out_stats) {
-        const kz::DevCounters& hc = *s->ctr_host;
         out_stats->paths = total;
-        out_stats->path_bounces = hc.path_bounces;
-        out_stats->shadow_rays = hc.shadow_rays;
+        out_stats->path_bounces = bounces;
+        out_stats->shadow_rays = shadows;
         out_stats->threads = cap;
         out_stats->device_ms = ms;
     }

@@ -13,10 +13,10 @@ namespace {
 // ids [0, total) are generated in job order; a path's own id is local to its
 // job, so every job renders exactly what kz_render renders for it.
 
-__global__ void k_generate_batch_dev(const DevJob* __restrict__ jobs, uint32_t n_jobs, PathSoA dst,
-                                     const DevCounters* c) {
+__global__ void k_generate_batch_dev(const DevJob* __restrict__ jobs, uint32_t n_jobs, PathSoA dst, IterSlots it) {
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j < c->gen_count) batch_generate(jobs, n_jobs, dst, c, j);
+    const NewPaths n = new_paths(it, j);
+    if (j < n.count) batch_generate(jobs, n_jobs, dst, n.first + j, n.slot + j);
 }
 
 // Shades path i of the wavefront (i >= n_in: no path); every thread of the
@@ -42,9 +42,10 @@ __device__ __forceinline__ void batch_shade(const DevJob* __restrict__ jobs, Pat
 
 template <bool kAttr>
 __global__ void __launch_bounds__(256, KZ_SHADE_MIN_BLOCKS) k_shade_batch(const DevJob* __restrict__ jobs, PathSoA in, PathSoA out,
-                                                     ShadowSoA sq, DevCounters* ctr) {
-    if (blockIdx.x * blockDim.x >= ctr->n_active) return;  // the grid covers the wavefront's capacity
-    batch_shade<kAttr>(jobs, in, out, sq, ctr, blockIdx.x * blockDim.x + threadIdx.x, ctr->n_active);
+                                                     ShadowSoA sq, DevCounters* ctr, const uint32_t* n_active) {
+    const uint32_t n = *n_active;
+    if (blockIdx.x * blockDim.x >= n) return;  // the grid covers the wavefront's capacity
+    batch_shade<kAttr>(jobs, in, out, sq, ctr, blockIdx.x * blockDim.x + threadIdx.x, n);
 }
 
 // ------------------------------------------------------------------ one persistent launch
@@ -113,7 +114,7 @@ extern __shared__ __align__(16) unsigned char kz_batch_smem[];
 constexpr size_t kBatchSmem = sizeof(ClosestSmem) > sizeof(AnySmem) ? sizeof(ClosestSmem) : sizeof(AnySmem);
 
 __device__ __noinline__ void stage_trace_paths(const DevJob* __restrict__ jobs, PathSoA p, DevCounters* ctr) {
-    batch_trace_paths(*reinterpret_cast<ClosestSmem*>(kz_batch_smem), jobs, p, ctr);
+    batch_trace_paths(*reinterpret_cast<ClosestSmem*>(kz_batch_smem), jobs, p, ctr->n_active, ctr);
 }
 __device__ __noinline__ void stage_trace_shadow(const DevJob* __restrict__ jobs, ShadowSoA sq, DevCounters* ctr) {
     batch_trace_shadow(*reinterpret_cast<AnySmem*>(kz_batch_smem), jobs, sq, ctr);
@@ -141,7 +142,7 @@ __global__ void __launch_bounds__(256, 4) k_batch_persistent(const DevJob* __res
         const uint32_t n_active = vc->n_active, gen_count = vc->gen_count;
         if (n_active == 0 && vc->next_path >= vc->total) return;
         for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < gen_count; j += stride)
-            batch_generate(jobs, n_jobs, A, ctr, j);
+            batch_generate(jobs, n_jobs, A, ctr->gen_first + j, ctr->gen_slot + j);
         if (!grid_barrier(ctr)) return;
         stage_trace_paths(jobs, A, ctr);
         if (!grid_barrier(ctr)) return;
@@ -157,10 +158,14 @@ __global__ void __launch_bounds__(256, 4) k_batch_persistent(const DevJob* __res
 
 }  // namespace
 
-void launch_generate_batch_dev(const DevJob* jobs, uint32_t n_jobs, PathSoA dst, DevCounters* ctr, uint32_t cap,
-                               uint32_t block, cudaStream_t st) {
-    if (!cap) return;
-    k_generate_batch_dev<<<grid_for(cap, block), block, 0, st>>>(jobs, n_jobs, dst, ctr);
+void launch_generate_batch_dev(const DevJob* jobs, uint32_t n_jobs, PathSoA dst, const IterSlots& it, uint32_t block,
+                               cudaStream_t st) {
+    if (!it.cap) return;
+    k_generate_batch_dev<<<grid_for(it.cap, block), block, 0, st>>>(jobs, n_jobs, dst, it);
+}
+void prepare_batch_shading() {
+    (void)split_grids<false, true>();
+    (void)split_grids<true, true>();
 }
 // Blocks per SM of the persistent batch kernel (0: it does not fit).
 int batch_persistent_blocks_per_sm(bool textured) {
@@ -180,19 +185,20 @@ cudaError_t launch_batch_persistent(const DevJob* jobs, uint32_t n_jobs, PathSoA
 }
 
 int launch_shade_batch(const DevJob* jobs, PathSoA in, uint32_t cap, PathSoA out, ShadowSoA sq, HeavyQueue hq,
-                       DevCounters* ctr, uint32_t block, bool textured, bool heavy, cudaStream_t st) {
+                       DevCounters* ctr, const uint32_t* n_active, uint32_t block, bool textured, bool heavy,
+                       cudaStream_t st) {
     if (!cap) return 0;  // textured: textures or normals
     if (hq.paths) {
         if (textured)
-            return launch_split_shading<true, true>(DevScene{}, PathParams{}, jobs, in, cap, out, sq, hq, ctr, nullptr,
-                                                    nullptr, heavy, st);
-        return launch_split_shading<false, true>(DevScene{}, PathParams{}, jobs, in, cap, out, sq, hq, ctr, nullptr,
-                                                 nullptr, heavy, st);
+            return launch_split_shading<true, true>(DevScene{}, PathParams{}, jobs, in, cap, out, sq, hq, ctr,
+                                                    n_active, nullptr, nullptr, heavy, st);
+        return launch_split_shading<false, true>(DevScene{}, PathParams{}, jobs, in, cap, out, sq, hq, ctr,
+                                                 n_active, nullptr, nullptr, heavy, st);
     }
     if (textured)
-        k_shade_batch<true><<<grid_for(cap, block), block, 0, st>>>(jobs, in, out, sq, ctr);
+        k_shade_batch<true><<<grid_for(cap, block), block, 0, st>>>(jobs, in, out, sq, ctr, n_active);
     else
-        k_shade_batch<false><<<grid_for(cap, block), block, 0, st>>>(jobs, in, out, sq, ctr);
+        k_shade_batch<false><<<grid_for(cap, block), block, 0, st>>>(jobs, in, out, sq, ctr, n_active);
     return 1;
 }
 

@@ -151,7 +151,9 @@ struct HeavyQueue {
     uint32_t cap = 0;
 };
 
-// Counters the stage kernels update on the device.
+// Counters the stage kernels update on the device. The device-driven loop has
+// one of these per iteration, all cleared beforehand, so that no kernel is
+// needed between iterations to move or reset them.
 struct DevCounters {
     union {
         unsigned long long n_append;  // both counts, for one atomic
@@ -161,10 +163,11 @@ struct DevCounters {
         } queue;
     };
     uint32_t status;     // device-side error (KZ_ERR_STACK ...)
-    uint32_t n_active;   // paths in the current buffer (device-driven loop)
+    uint32_t n_active;   // paths in the current buffer, where the iteration generated paths
     unsigned long long fetch[4];  // closest nodes, closest tris, shadow nodes, shadow tris
-    // device-driven loop: path ids [0, total) are generated in order
-    unsigned long long next_path, total;
+    unsigned long long next_path;  // first path id not yet generated (path ids are generated in order)
+    // single-launch batch kernel: one set of counters for the whole loop
+    unsigned long long total;
     unsigned long long path_bounces, shadow_rays, iterations;
     unsigned long long gen_first;  // first path id generated this iteration
     uint32_t gen_count, gen_slot;  // how many, and where in the buffer
@@ -173,6 +176,15 @@ struct DevCounters {
     uint32_t heavy[kHeavyClasses], heavy_next;  // split shading: paths queued by class, fetch cursor
     uint32_t bar_count, bar_gen;   // grid barrier of the persistent batch kernel
     uint32_t bar_abort;            // set when a barrier wait ran out
+};
+
+// An iteration's place in the device-driven loop: its counters, those of the
+// iteration before and of the last one that generated paths.
+struct IterSlots {
+    DevCounters* cur;
+    const DevCounters *prev, *last_gen;
+    unsigned long long total;  // paths of the whole call
+    uint32_t cap;              // capacity of the wavefront
 };
 
 // One job of a batched render: its scene, camera and film.
@@ -214,12 +226,6 @@ void launch_trace_paths(const DevScene& s, PathSoA p, uint32_t n, DevCounters* c
 void launch_shade(const DevScene& s, const PathParams& pp, PathSoA in, uint32_t n_in, PathSoA out,
                   ShadowSoA sq, DevCounters* ctr, float* film, double* film64, uint32_t block,
                   cudaStream_t st);
-void launch_shade_guided(const DevScene& s, const PathParams& pp, PathSoA in, uint32_t n_in, PathSoA out,
-                         ShadowSoA sq, DevCounters* ctr, float* film, double* film64, const GuideShade& gs,
-                         uint32_t block, cudaStream_t st);
-void launch_trace_shadow_guided(const DevScene& s, ShadowSoA sq, uint32_t n_max, DevCounters* ctr, float* film,
-                                double* film64, VRec* recs, NRec* nee, uint32_t max_depth, uint32_t block,
-                                cudaStream_t st);
 // Training samples from a pass's vertex and next-event records: 3 float4 per
 // sample ((p01, weight), (n, -), (dir, -)); *count and the weight sum *wsum.
 void launch_guide_collect(const VRec* recs, const NRec* nee, uint64_t n_recs, float4* samples, uint32_t cap,
@@ -227,8 +233,6 @@ void launch_guide_collect(const VRec* recs, const NRec* nee, uint64_t n_recs, fl
 
 // ---- guiding network (kz_mlp.cu) -------------------------------------------
 cudaError_t guide_kernel_setup();
-void launch_guide_infer_paths(const DevScene& s, PathSoA p, uint32_t n, const GuideDev& gd, float* raw,
-                              cudaStream_t st);
 void launch_guide_infer_points(const float4* pts, uint32_t n, const GuideDev& gd, float* raw, cudaStream_t st);
 // One training batch of `rows` samples; row r reads sample ((r + offset) * stride) % count.
 // Adds the weighted loss to *loss and the gradient to grad; a sample's weight
@@ -256,56 +260,63 @@ cudaError_t launch_guide_wgrad_tc(const __nv_bfloat16* rec, uint32_t n, float* g
 void launch_guide_adam(float* w, float* m, float* v, const float* grad, __nv_bfloat16* wbf, float lr, int step,
                        cudaStream_t st);
 void launch_guide_to_bf16(const float* w, __nv_bfloat16* wbf, cudaStream_t st);
-// Persistent shadow pass of the device-driven loop.
-void launch_trace_shadow_dev(const DevScene& s, ShadowSoA sq, uint32_t n_max, DevCounters* ctr, bool count,
-                             float* film, double* film64, cudaStream_t st);
 void launch_trace_shadow(const DevScene& s, ShadowSoA sq, uint32_t n_max, DevCounters* ctr, bool count,
                          float* film, double* film64, uint32_t block, cudaStream_t st);
 void launch_scale(float* film, double* film64, uint64_t n, float sf, double sd, cudaStream_t st);
 
-// Device-driven wavefront: one iteration = plan, generate, trace, [infer],
-// shade, shadow, finish; every count lives in DevCounters, so the host can
-// enqueue many iterations between synchronisations. Grids are sized for the
-// capacity `cap`; threads beyond the device-side count exit.
-// plan: reserve slots for new paths (unless !generate) and reset the
-// iteration's queue counters
-void launch_plan(DevCounters* ctr, uint32_t cap, cudaStream_t st, bool generate = true);
-void launch_finish(DevCounters* ctr, cudaStream_t st);
-void launch_generate_camera_dev(const DevCamera& cam, const PathParams& pp, PathSoA dst, DevCounters* ctr,
-                                uint32_t cap, uint32_t block, cudaStream_t st);
-void launch_generate_rays_dev(const kz_ray* rays, const PathParams& pp, PathSoA dst, DevCounters* ctr, uint32_t cap,
+// Device-driven wavefront: one iteration = [generate], trace, [infer], shade;
+// every count lives in the iterations' DevCounters, so the host can enqueue
+// many iterations between synchronisations. The trace launch also traces the
+// shadow rays of the iteration before (launch_trace_both), or they have a
+// launch of their own. `n_active` points to the iteration's path count: its
+// own n_active if it generated paths, else queue.next of the one before. Grids
+// are sized for the capacity `cap`; threads beyond the count exit.
+void launch_generate_camera_dev(const DevCamera& cam, const PathParams& pp, PathSoA dst, const IterSlots& it,
+                                uint32_t block, cudaStream_t st);
+void launch_generate_rays_dev(const kz_ray* rays, const PathParams& pp, PathSoA dst, const IterSlots& it,
                               uint32_t block, cudaStream_t st);
-void launch_trace_paths_dev(const DevScene& s, PathSoA p, uint32_t cap, DevCounters* ctr, bool count, uint32_t block,
-                            cudaStream_t st);
+void launch_trace_paths_dev(const DevScene& s, PathSoA p, uint32_t cap, const uint32_t* n_active, DevCounters* ctr,
+                            bool count, cudaStream_t st);
+void launch_trace_both(const DevScene& s, PathSoA p, uint32_t cap, const uint32_t* n_active, DevCounters* ctr,
+                       ShadowSoA sq, DevCounters* prev, float* film, double* film64, const GuideShade* gs,
+                       uint32_t max_depth, cudaStream_t st);
+void launch_trace_shadow_dev(const DevScene& s, ShadowSoA sq, uint32_t n_max, DevCounters* ctr, bool count,
+                             float* film, double* film64, const GuideShade* gs, uint32_t max_depth, cudaStream_t st);
 void launch_shade_guided_dev(const DevScene& s, const PathParams& pp, PathSoA in, uint32_t cap, PathSoA out,
-                             ShadowSoA sq, DevCounters* ctr, float* film, double* film64, const GuideShade& gs,
-                             uint32_t block, cudaStream_t st);
+                             ShadowSoA sq, DevCounters* ctr, const uint32_t* n_active, float* film, double* film64,
+                             const GuideShade& gs, uint32_t block, cudaStream_t st);
 // Both return the number of kernels launched.
 int launch_shade_dev(const DevScene& s, const PathParams& pp, PathSoA in, uint32_t cap, PathSoA out, ShadowSoA sq,
-                     HeavyQueue hq, DevCounters* ctr, float* film, double* film64, const GuideShade* gs, uint32_t block,
-                     cudaStream_t st);
+                     HeavyQueue hq, DevCounters* ctr, const uint32_t* n_active, float* film, double* film64,
+                     const GuideShade* gs, uint32_t block, cudaStream_t st);
+int launch_shade_batch(const DevJob* jobs, PathSoA in, uint32_t cap, PathSoA out, ShadowSoA sq, HeavyQueue hq,
+                       DevCounters* ctr, const uint32_t* n_active, uint32_t block, bool textured, bool heavy,
+                       cudaStream_t st);
 // Capacity from which a wavefront is given a HeavyQueue.
 uint32_t split_shading_capacity();
+// Clears `n` iterations' counters; the first carries on from `last` and `last_gen`.
+void launch_carry(DevCounters* slots, uint32_t n, const DevCounters* last, const DevCounters* last_gen,
+                  cudaStream_t st);
+// Batched wavefront stages over the job table.
+void launch_generate_batch_dev(const DevJob* jobs, uint32_t n_jobs, PathSoA dst, const IterSlots& it, uint32_t block,
+                               cudaStream_t st);
+void launch_trace_both_batch(const DevJob* jobs, PathSoA p, uint32_t cap, const uint32_t* n_active, DevCounters* ctr,
+                             ShadowSoA sq, DevCounters* prev, cudaStream_t st);
 // Persistent batch renderer: grid = ctas blocks of `block` threads; each lane
 // keeps one path in registers and refills from the global counter every
 // `period` vertices (warp-aggregated fetch).
-// Batched wavefront stages over the job table (device-driven counters).
-void launch_generate_batch_dev(const DevJob* jobs, uint32_t n_jobs, PathSoA dst, DevCounters* ctr, uint32_t cap,
-                               uint32_t block, cudaStream_t st);
-void launch_trace_paths_batch(const DevJob* jobs, PathSoA p, uint32_t cap, DevCounters* ctr, cudaStream_t st);
-int launch_shade_batch(const DevJob* jobs, PathSoA in, uint32_t cap, PathSoA out, ShadowSoA sq, HeavyQueue hq,
-                       DevCounters* ctr, uint32_t block, bool textured, bool heavy, cudaStream_t st);
 void launch_trace_shadow_batch(const DevJob* jobs, ShadowSoA sq, uint32_t cap, DevCounters* ctr, cudaStream_t st);
 int batch_persistent_blocks_per_sm(bool textured);
 cudaError_t launch_batch_persistent(const DevJob* jobs, uint32_t n_jobs, PathSoA A, PathSoA B, ShadowSoA sq,
                                    DevCounters* ctr, uint32_t cap, uint32_t period, uint32_t blocks, bool textured,
                                    cudaStream_t st);
-// Queries the persistent stages' grid sizes (call before a stream capture).
+// Query the persistent stages' grid sizes (call before a stream capture).
 void prepare_batch_wavefront();
+void prepare_batch_shading();
 constexpr uint32_t kMaxBatchJobs = 1u << 20;  // job index in 20 bits of a path's flags
 void launch_render_batch(const DevJob* jobs, uint32_t n_jobs, unsigned long long total, BatchCounters* bc,
                          uint32_t period, uint32_t ctas, uint32_t block, cudaStream_t st);
-void launch_guide_infer_paths_dev(const DevScene& s, PathSoA p, uint32_t cap, const DevCounters* ctr,
+void launch_guide_infer_paths_dev(const DevScene& s, PathSoA p, uint32_t cap, const uint32_t* n_active,
                                   const GuideDev& gd, float* raw, cudaStream_t st);
 
 }  // namespace kz

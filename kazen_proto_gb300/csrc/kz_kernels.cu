@@ -57,21 +57,31 @@ __global__ void k_guide_collect(const VRec* __restrict__ recs, const NRec* __res
 }
 
 // ------------------------------------------------------------------ device-driven loop
-__global__ void k_plan(DevCounters* c, uint32_t cap, bool generate) { plan_iteration(c, cap, generate); }
-
-__global__ void k_finish(DevCounters* c) { finish_iteration(c); }
-
-__global__ void k_generate_camera_dev(DevCamera cam, PathParams pp, PathSoA dst, const DevCounters* c) {
+__global__ void k_generate_camera_dev(DevCamera cam, PathParams pp, PathSoA dst, IterSlots it) {
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= c->gen_count) return;
-    generate_camera_path(cam, pp, dst, c->gen_slot + j, c->gen_first + j);
+    const NewPaths n = new_paths(it, j);
+    if (j < n.count) generate_camera_path(cam, pp, dst, n.slot + j, n.first + j);
 }
 
-__global__ void k_generate_rays_dev(const kz_ray* __restrict__ rays, PathParams pp, PathSoA dst,
-                                    const DevCounters* c) {
+__global__ void k_generate_rays_dev(const kz_ray* __restrict__ rays, PathParams pp, PathSoA dst, IterSlots it) {
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= c->gen_count) return;
-    generate_ray_path(rays, pp, dst, c->gen_slot + j, c->gen_first + j);
+    const NewPaths n = new_paths(it, j);
+    if (j < n.count) generate_ray_path(rays, pp, dst, n.slot + j, n.first + j);
+}
+
+// Clears the iterations' counters for the next batch; the first carries over
+// the paths left alive and the path cursor.
+__global__ void k_carry(DevCounters* slots, uint32_t n, const DevCounters* last, const DevCounters* last_gen) {
+    const uint32_t alive = last->queue.next;
+    const unsigned long long next = last_gen->next_path;
+    __syncthreads();
+    uint32_t* w = reinterpret_cast<uint32_t*>(slots);
+    for (uint32_t k = threadIdx.x; k < n * (uint32_t)(sizeof(DevCounters) / 4); k += blockDim.x) w[k] = 0u;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        slots->queue.next = alive;
+        slots->next_path = next;
+    }
 }
 
 __global__ void k_scale(float* film, double* film64, uint64_t n, float sf, double sd) {
@@ -93,39 +103,39 @@ void launch_generate_rays(const kz_ray* rays, const PathParams& pp, PathSoA dst,
     if (!n_new) return;
     k_generate_rays<<<grid_for(n_new, block), block, 0, st>>>(rays, pp, dst, dst_offset, first_path, n_new);
 }
-void launch_plan(DevCounters* ctr, uint32_t cap, cudaStream_t st, bool generate) {
-    k_plan<<<1, 1, 0, st>>>(ctr, cap, generate);
+void launch_generate_camera_dev(const DevCamera& cam, const PathParams& pp, PathSoA dst, const IterSlots& it,
+                                uint32_t block, cudaStream_t st) {
+    if (!it.cap) return;
+    k_generate_camera_dev<<<grid_for(it.cap, block), block, 0, st>>>(cam, pp, dst, it);
 }
-void launch_finish(DevCounters* ctr, cudaStream_t st) { k_finish<<<1, 1, 0, st>>>(ctr); }
-void launch_generate_camera_dev(const DevCamera& cam, const PathParams& pp, PathSoA dst, DevCounters* ctr,
-                                uint32_t cap, uint32_t block, cudaStream_t st) {
-    if (!cap) return;
-    k_generate_camera_dev<<<grid_for(cap, block), block, 0, st>>>(cam, pp, dst, ctr);
-}
-void launch_generate_rays_dev(const kz_ray* rays, const PathParams& pp, PathSoA dst, DevCounters* ctr, uint32_t cap,
+void launch_generate_rays_dev(const kz_ray* rays, const PathParams& pp, PathSoA dst, const IterSlots& it,
                               uint32_t block, cudaStream_t st) {
-    if (!cap) return;
-    k_generate_rays_dev<<<grid_for(cap, block), block, 0, st>>>(rays, pp, dst, ctr);
+    if (!it.cap) return;
+    k_generate_rays_dev<<<grid_for(it.cap, block), block, 0, st>>>(rays, pp, dst, it);
+}
+void launch_carry(DevCounters* slots, uint32_t n, const DevCounters* last, const DevCounters* last_gen,
+                  cudaStream_t st) {
+    k_carry<<<1, 256, 0, st>>>(slots, n, last, last_gen);
 }
 int launch_shade_dev(const DevScene& s, const PathParams& pp, PathSoA in, uint32_t cap, PathSoA out, ShadowSoA sq,
-                     HeavyQueue hq, DevCounters* ctr, float* film, double* film64, const GuideShade* gs, uint32_t block,
-                     cudaStream_t st) {
+                     HeavyQueue hq, DevCounters* ctr, const uint32_t* n_active, float* film, double* film64,
+                     const GuideShade* gs, uint32_t block, cudaStream_t st) {
     if (!cap) return 0;
     const bool attr = s.mat_tex || s.tri_nrm;
     if (gs) {
-        launch_shade_guided_dev(s, pp, in, cap, out, sq, ctr, film, film64, *gs, block, st);
+        launch_shade_guided_dev(s, pp, in, cap, out, sq, ctr, n_active, film, film64, *gs, block, st);
     } else if (hq.paths) {
         if (attr)
-            return launch_split_shading<true, false>(s, pp, nullptr, in, cap, out, sq, hq, ctr, film, film64,
-                                                     s.has_heavy != 0, st);
-        return launch_split_shading<false, false>(s, pp, nullptr, in, cap, out, sq, hq, ctr, film, film64,
-                                                  s.has_heavy != 0, st);
+            return launch_split_shading<true, false>(s, pp, nullptr, in, cap, out, sq, hq, ctr, n_active, film,
+                                                     film64, s.has_heavy != 0, st);
+        return launch_split_shading<false, false>(s, pp, nullptr, in, cap, out, sq, hq, ctr, n_active, film,
+                                                  film64, s.has_heavy != 0, st);
     } else if (attr) {
         k_shade<false, true><<<grid_for(cap, block), block, 0, st>>>(s, pp, in, cap, out, sq, ctr, film, film64,
-                                                                     GuideShade{}, &ctr->n_active);
+                                                                     GuideShade{}, n_active);
     } else {
         k_shade<false, false><<<grid_for(cap, block), block, 0, st>>>(s, pp, in, cap, out, sq, ctr, film, film64,
-                                                                      GuideShade{}, &ctr->n_active);
+                                                                      GuideShade{}, n_active);
     }
     return 1;
 }

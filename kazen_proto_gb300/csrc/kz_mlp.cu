@@ -502,20 +502,12 @@ cudaError_t guide_kernel_setup() {
     return e;
 }
 
-void launch_guide_infer_paths(const DevScene& s, PathSoA p, uint32_t n, const GuideDev& gd, float* raw,
-                              cudaStream_t st) {
-    if (!n) return;
-    const uint32_t tiles = (n + 15) / 16;
-    const uint32_t grid = min((tiles + 3) / 4, (uint32_t)sm_count() * kInferCtasPerSm);
-    k_guide_infer<true><<<grid, 128, kSmemInfer, st>>>(s, p, nullptr, n, gd, raw, nullptr);
-}
-
-void launch_guide_infer_paths_dev(const DevScene& s, PathSoA p, uint32_t cap, const DevCounters* ctr,
+void launch_guide_infer_paths_dev(const DevScene& s, PathSoA p, uint32_t cap, const uint32_t* n_active,
                                   const GuideDev& gd, float* raw, cudaStream_t st) {
     if (!cap) return;
     const uint32_t tiles = (cap + 15) / 16;
     const uint32_t grid = min((tiles + 3) / 4, (uint32_t)sm_count() * kInferCtasPerSm);
-    k_guide_infer<true><<<grid, 128, kSmemInfer, st>>>(s, p, nullptr, cap, gd, raw, &ctr->n_active);
+    k_guide_infer<true><<<grid, 128, kSmemInfer, st>>>(s, p, nullptr, cap, gd, raw, n_active);
 }
 
 void launch_guide_infer_points(const float4* pts, uint32_t n, const GuideDev& gd, float* raw, cudaStream_t st) {

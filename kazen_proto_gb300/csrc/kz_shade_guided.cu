@@ -11,27 +11,16 @@
 
 namespace kz {
 
-void launch_shade_guided(const DevScene& s, const PathParams& pp, PathSoA in, uint32_t n_in, PathSoA out,
-                         ShadowSoA sq, DevCounters* ctr, float* film, double* film64, const GuideShade& gs,
-                         uint32_t block, cudaStream_t st) {
-    if (!n_in) return;
-    if (s.mat_tex || s.tri_nrm)
-        k_shade<true, true><<<grid_for(n_in, block), block, 0, st>>>(s, pp, in, n_in, out, sq, ctr, film, film64, gs,
-                                                                     nullptr);
-    else
-        k_shade<true, false><<<grid_for(n_in, block), block, 0, st>>>(s, pp, in, n_in, out, sq, ctr, film, film64,
-                                                                      gs, nullptr);
-}
 void launch_shade_guided_dev(const DevScene& s, const PathParams& pp, PathSoA in, uint32_t cap, PathSoA out,
-                             ShadowSoA sq, DevCounters* ctr, float* film, double* film64, const GuideShade& gs,
-                             uint32_t block, cudaStream_t st) {
+                             ShadowSoA sq, DevCounters* ctr, const uint32_t* n_active, float* film, double* film64,
+                             const GuideShade& gs, uint32_t block, cudaStream_t st) {
     if (!cap) return;
     if (s.mat_tex || s.tri_nrm)
         k_shade<true, true><<<grid_for(cap, block), block, 0, st>>>(s, pp, in, cap, out, sq, ctr, film, film64, gs,
-                                                                    &ctr->n_active);
+                                                                    n_active);
     else
         k_shade<true, false><<<grid_for(cap, block), block, 0, st>>>(s, pp, in, cap, out, sq, ctr, film, film64, gs,
-                                                                     &ctr->n_active);
+                                                                     n_active);
 }
 
 }  // namespace kz

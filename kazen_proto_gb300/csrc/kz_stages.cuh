@@ -122,21 +122,22 @@ struct ClosestSmem {
     float4 vwdt[256];
     uint4 ent[kClosestSteps * 256];
 };
-// KZ_ANY_SMEM_STACK: the any-hit loop's first stack entries in shared memory
-// (off: the terrain frame's shadow stage measured 29.1 ms with 4 or 8 entries
-// against 28.9 ms with the whole stack in local memory).
-#ifndef KZ_ANY_SMEM_STACK
-#define KZ_ANY_SMEM_STACK 0
-#endif
 struct AnySmem {
     float4 ray[2 * 256];
     unsigned long long key[256];
     uint32_t rec[256];
     uint4 ent[kAnySteps * 256];
-#if KZ_ANY_SMEM_STACK > 0 && KZ_ANY_SMEM_STACK < KZ_WIDE_STACK
-    uint2 stack[KZ_ANY_SMEM_STACK * 256];
-#endif
 };
+// The any-hit loop's arrays; a kernel that runs both loops, its warps in
+// either at the same time, takes them from the closest-hit loop's (each warp
+// keeps its own part of every array).
+__device__ __forceinline__ LeafShare any_share(AnySmem& m) {
+    return LeafShare{m.ray, m.key, m.rec, nullptr, m.ent + (threadIdx.x & ~31u) * kAnySteps};
+}
+__device__ __forceinline__ LeafShare any_share(ClosestSmem& m) {
+    return LeafShare{m.ray, m.key, m.rec, nullptr, m.ent + (threadIdx.x & ~31u) * kClosestSteps};
+}
+static_assert(kAnySteps <= kClosestSteps, "the any-hit loop's lists must fit the closest-hit loop's");
 
 // Closest hit of ray k through persistent_rays_shared: load(k, r, tmax) sets
 // the ray up, store(k, hit) writes the result; m is the block's shared memory.
@@ -155,7 +156,7 @@ __device__ __forceinline__ void persistent_closest_in(ClosestSmem& m, DevScene& 
     const LocalStack stack{stack_lm};
 #endif
     constexpr int K = kCount ? 1 : kClosestSteps;
-    const LeafShare sh{m.ray, m.key, m.rec, m.vwdt, m.ent};
+    const LeafShare sh{m.ray, m.key, m.rec, m.vwdt, m.ent + (threadIdx.x & ~31u) * kClosestSteps};
     AnyState c;
     TRay r;
     WideDir dir;
@@ -198,18 +199,13 @@ __device__ __forceinline__ void persistent_closest(DevScene& s, Ctr n, Ctr* next
 
 // Any hit of ray k through persistent_rays_shared: load(k, r, tmax) sets the
 // ray up, done(k, rc) gets 1 (no hit), 2 (hit) or -1 (aborted: miss).
-template <bool kCount, bool kOwnScene, typename Ctr, typename Load, typename Done>
-__device__ __forceinline__ void persistent_any_in(AnySmem& m, DevScene& s, Ctr n, Ctr* next, Load load, Done done,
+template <bool kCount, bool kOwnScene, typename Smem, typename Ctr, typename Load, typename Done>
+__device__ __forceinline__ void persistent_any_in(Smem& m, DevScene& s, Ctr n, Ctr* next, Load load, Done done,
                                                   uint32_t& dn, uint32_t& dt) {
-#if KZ_ANY_SMEM_STACK > 0 && KZ_ANY_SMEM_STACK < KZ_WIDE_STACK
-    uint2 stack_lm[kWideStack - KZ_ANY_SMEM_STACK];
-    const SplitStack<KZ_ANY_SMEM_STACK> stack{m.stack, stack_lm};
-#else
-    uint2 stack_lm[kWideStack];
+    uint2 stack_lm[kWideStack];  // all local: with 4 or 8 entries in shared memory the shadow stage gained nothing
     const LocalStack stack{stack_lm};
-#endif
     constexpr int K = kCount ? 1 : kAnySteps;
-    const LeafShare sh{m.ray, m.key, m.rec, nullptr, m.ent};
+    const LeafShare sh = any_share(m);
     AnyState c;
     TRay r;
     WideDir dir;
@@ -249,8 +245,6 @@ __device__ __forceinline__ void persistent_any(DevScene& s, Ctr n, Ctr* next, Lo
     __shared__ AnySmem m;
     persistent_any_in<kCount, kOwnScene>(m, s, n, next, load, done, dn, dt);
 }
-
-// Closest-hit pass of the device-driven loop (k_plan zeroes trace_next).
 
 __device__ __forceinline__ void film_add(float* film, double* film64, uint32_t idx, f3 c) {
     atomicAdd(film + 3 * (size_t)idx, c.x);
@@ -811,11 +805,11 @@ __device__ __forceinline__ void trace_fields(DevScene& dst, const DevScene& src)
 
 // Closest hits of the wavefront's paths; each path's scene through its job.
 __device__ __forceinline__ void batch_trace_paths(ClosestSmem& m, const DevJob* __restrict__ jobs, PathSoA p,
-                                                  DevCounters* ctr) {
+                                                  uint32_t n, DevCounters* ctr) {
     uint32_t dn = 0, dt = 0;
     DevScene ls;
     persistent_closest_in<false, true>(
-        m, ls, ctr->n_active, &ctr->trace_next, &ctr->status,
+        m, ls, n, &ctr->trace_next, &ctr->status,
         [&](uint32_t k, TRay& r, float& tmax) {
             const float4 o = p.o4[k], d = p.d4[k];
             trace_fields(ls, jobs[__float_as_uint(d.w) >> kJobShift].scene);
@@ -827,7 +821,8 @@ __device__ __forceinline__ void batch_trace_paths(ClosestSmem& m, const DevJob* 
 
 // Shadow rays of the wavefront; an unoccluded one adds its contribution to
 // its job's film.
-__device__ __forceinline__ void batch_trace_shadow(AnySmem& m, const DevJob* __restrict__ jobs, ShadowSoA sq,
+template <typename Smem>
+__device__ __forceinline__ void batch_trace_shadow(Smem& m, const DevJob* __restrict__ jobs, ShadowSoA sq,
                                                    DevCounters* ctr) {
     uint32_t dn = 0, dt = 0;
     DevScene ls;
@@ -848,19 +843,35 @@ __device__ __forceinline__ void batch_trace_shadow(AnySmem& m, const DevJob* __r
         dn, dt);
 }
 
-// Camera path j of this iteration's generation (j < gen_count).
+// Camera path g (over all jobs) into slot k.
 __device__ __forceinline__ void batch_generate(const DevJob* __restrict__ jobs, uint32_t n_jobs, PathSoA dst,
-                                               const DevCounters* c, uint32_t j) {
-    const unsigned long long g = c->gen_first + j;
+                                               unsigned long long g, uint32_t k) {
     const uint32_t job = find_job(jobs, n_jobs, g);
     const DevJob& J = jobs[job];
-    const uint32_t k = c->gen_slot + j;
     generate_camera_path(J.cam, J.pp, dst, k, g - J.path_begin);
     dst.d4[k].w = __uint_as_float(__float_as_uint(dst.d4[k].w) | (job << kJobShift));
 }
 
-// Counters of one iteration of the device-driven loop: how many new paths
-// fill the free slots (when `generate`), and the per-iteration cursors reset.
+// New paths of an iteration of the device-driven loop, as every thread of its
+// generating kernel works it out from the iteration before and the last one
+// that generated; one of them (j == 0) leaves it for the kernels that follow.
+struct NewPaths {
+    unsigned long long first;  // path id
+    uint32_t count, slot;
+};
+__device__ __forceinline__ NewPaths new_paths(const IterSlots& it, uint32_t j) {
+    const uint32_t alive = it.prev->queue.next, room = it.cap - alive;
+    const unsigned long long first = it.last_gen->next_path, left = it.total - first;
+    const NewPaths n{first, (uint32_t)(left < room ? left : room), alive};
+    if (j == 0) {
+        it.cur->next_path = first + n.count;
+        it.cur->n_active = alive + n.count;
+    }
+    return n;
+}
+
+// Counters of one iteration of the single-launch batch kernel: how many new
+// paths fill the free slots (when `generate`), and the cursors reset.
 __device__ __forceinline__ void plan_iteration(DevCounters* c, uint32_t cap, bool generate) {
     const uint64_t remaining = c->total - c->next_path;
     const uint32_t room = cap - c->n_active;
@@ -1031,11 +1042,12 @@ __device__ __forceinline__ uint32_t* heavy_slot(const HeavyQueue& q, uint32_t cl
 template <bool kAttr, bool kJobs>
 __global__ void __launch_bounds__(256, KZ_PLAIN_MIN_BLOCKS)
     k_shade_plain(DevScene scene, PathParams params, const DevJob* __restrict__ jobs, PathSoA in, PathSoA out,
-                  ShadowSoA sq, HeavyQueue hq, DevCounters* ctr, float* film, double* film64) {
+                  ShadowSoA sq, HeavyQueue hq, DevCounters* ctr, const uint32_t* n_active, float* film,
+                  double* film64) {
     // per warp: appended paths and shadow rays, then the four heavy classes; double buffered over the rounds
     __shared__ unsigned long long s_app[2][8];
     __shared__ uint32_t s_heavy[2][kHeavyClasses][8];
-    const uint32_t n = ctr->n_active, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, lt = (1u << lane) - 1u;
+    const uint32_t n = *n_active, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, lt = (1u << lane) - 1u;
     uint32_t buf = 0;
     for (uint32_t base = blockIdx.x * 256u; base < n; base += gridDim.x * 256u, buf ^= 1u) {
         const uint32_t i = base + threadIdx.x;
@@ -1130,16 +1142,24 @@ __global__ void __launch_bounds__(kHeavyThreads, KZ_HEAVY_MIN_BLOCKS)
 #ifndef KZ_SPLIT_SHADING
 #define KZ_SPLIT_SHADING (1u << 18)
 #endif
+struct SplitGrids {
+    unsigned plain, heavy;
+};
+template <bool kAttr, bool kJobs>
+static SplitGrids split_grids() {
+    static const SplitGrids g{resident_grid(k_shade_plain<kAttr, kJobs>, 256),
+                              resident_grid(k_shade_heavy<kAttr, kJobs>, kHeavyThreads)};
+    return g;
+}
 template <bool kAttr, bool kJobs>
 static int launch_split_shading(const DevScene& s, const PathParams& pp, const DevJob* jobs, PathSoA in, uint32_t cap,
-                                PathSoA out, ShadowSoA sq, HeavyQueue hq, DevCounters* ctr, float* film,
-                                double* film64, bool heavy, cudaStream_t st) {
-    static const unsigned gp = resident_grid(k_shade_plain<kAttr, kJobs>, 256);
-    static const unsigned gh = resident_grid(k_shade_heavy<kAttr, kJobs>, kHeavyThreads);
-    k_shade_plain<kAttr, kJobs><<<std::min(gp, grid_for(cap, 256)), 256, 0, st>>>(s, pp, jobs, in, out, sq, hq, ctr,
-                                                                                film, film64);
+                                PathSoA out, ShadowSoA sq, HeavyQueue hq, DevCounters* ctr,
+                                const uint32_t* n_active, float* film, double* film64, bool heavy, cudaStream_t st) {
+    const SplitGrids g = split_grids<kAttr, kJobs>();
+    k_shade_plain<kAttr, kJobs><<<std::min(g.plain, grid_for(cap, 256)), 256, 0, st>>>(s, pp, jobs, in, out, sq, hq, ctr,
+                                                                                n_active, film, film64);
     if (!heavy) return 1;
-    k_shade_heavy<kAttr, kJobs><<<std::min(gh, grid_for(cap, kHeavyThreads)), kHeavyThreads, 0, st>>>(
+    k_shade_heavy<kAttr, kJobs><<<std::min(g.heavy, grid_for(cap, kHeavyThreads)), kHeavyThreads, 0, st>>>(
         s, pp, jobs, in, out, sq, hq, ctr, film, film64);
     return 2;
 }

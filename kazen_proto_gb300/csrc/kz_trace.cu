@@ -13,6 +13,17 @@
 namespace kz {
 namespace {
 
+// Blocks for n rays (persistent kernels of `resident` blocks): 256 rays a
+// block, but for fewer rays than that gives every SM a block, 8 a block, one a
+// warp (persistent_rays_shared spreads them). 64 rays through 20,000 triangles:
+// 131 us in one block, 114 in eight; but 65,537 Li rays 600 us over all
+// resident blocks against 540 over 257: there the warps' steps, not the longest
+// ray, are waited for.
+unsigned trace_grid(uint64_t n, unsigned resident) {
+    const uint64_t full = (n + 255) / 256, spread = std::min<uint64_t>((n + 7) / 8, 152);
+    return (unsigned)std::min<uint64_t>(resident, std::max(full, spread));
+}
+
 // A node of the builder's layout (kz_bvh.h) to the traversal's (WideAxis,
 // kz_traverse.cuh), in place; the same boxes, children and records.
 __global__ void k_pack_nodes(uint4* nodes, uint32_t n) {
@@ -102,18 +113,73 @@ __global__ void __launch_bounds__(256) k_trace_paths(DevScene s, PathSoA p, uint
     if (kCount) warp_count(dn, dt, &ctr->fetch[0]);
 }
 
+// Closest hits of the wavefront's paths.
 template <bool kCount>
-__global__ void __launch_bounds__(256, KZ_TRACE_MINB) k_trace_paths_persistent(DevScene s, PathSoA p, DevCounters* ctr) {
-    uint32_t dn = 0, dt = 0;
-    persistent_closest<kCount>(
-        s, ctr->n_active, &ctr->trace_next, &ctr->status,
+__device__ __forceinline__ void trace_paths(ClosestSmem& m, DevScene& s, PathSoA p, uint32_t n, DevCounters* ctr,
+                                            uint32_t& dn, uint32_t& dt) {
+    persistent_closest_in<kCount, false>(
+        m, s, n, &ctr->trace_next, &ctr->status,
         [&](uint32_t k, TRay& r, float& tmax) {
             const float4 o = p.o4[k], d = p.d4[k];
             r = make_tray(xyz(o), xyz(d), kRayEps);
             tmax = __int_as_float(0x7f800000);
         },
         [&](uint32_t k, const HitRec& h) { p.hit[k] = make_float4(h.t, h.u, h.v, __int_as_float(h.rec)); }, dn, dt);
+}
+
+// The shadow rays queued in iteration `ctr`; an unoccluded one adds its
+// contribution to the film (and to the guiding records).
+template <bool kCount, bool kGuided, typename Smem>
+__device__ __forceinline__ void trace_shadow(Smem& m, DevScene& s, ShadowSoA sq, DevCounters* ctr, float* film,
+                                             double* film64, VRec* recs, NRec* nee, uint32_t max_depth, uint32_t& dn,
+                                             uint32_t& dt) {
+    const auto unoccluded = [&](uint32_t ray) {
+        const float4 cc = sq.c4[ray];
+        film_add(film, film64, __float_as_uint(sq.d4[ray].w), xyz(cc));
+        if (kGuided && recs) {
+            const uint32_t tag = __float_as_uint(cc.w);
+            const uint64_t rb = (uint64_t)(tag >> 4) * max_depth;
+            propagate(recs, rb, tag & 15u, xyz(cc));
+            if (nee) nee[rb + (tag & 15u)].n.w = 1.f;
+        }
+    };
+    persistent_any_in<kCount, false>(
+        m, s, ctr->queue.shadow, &ctr->shadow_next,
+        [&](uint32_t k, TRay& r, float& tmax) {
+            const float4 o = sq.o4[k], d = sq.d4[k];
+            r = make_tray(xyz(o), xyz(d), kRayEps);
+            tmax = o.w;
+        },
+        [&](uint32_t ray, int rc) {
+            if (rc < 0) set_status(&ctr->status, KZ_ERR_STACK);
+            if (rc == 1) unoccluded(ray);
+        },
+        dn, dt);
+}
+
+template <bool kCount>
+__global__ void __launch_bounds__(256, KZ_TRACE_MINB) k_trace_paths_persistent(DevScene s, PathSoA p,
+                                                                               const uint32_t* n_active,
+                                                                               DevCounters* ctr) {
+    __shared__ ClosestSmem m;
+    uint32_t dn = 0, dt = 0;
+    trace_paths<kCount>(m, s, p, *n_active, ctr, dn, dt);
     if (kCount) warp_count(dn, dt, &ctr->fetch[0]);
+}
+
+// An iteration's closest hits and the shadow rays of the iteration before,
+// which depend on nothing of this one, in one launch: a warp that finds no
+// path left goes on to the shadow rays, so that one tail of long rays is
+// waited for instead of two, and the launch is one instead of two.
+template <bool kGuided>
+__global__ void __launch_bounds__(256, KZ_TRACE_MINB) k_trace_both(DevScene s, PathSoA p, const uint32_t* n_active,
+                                                                   DevCounters* ctr, ShadowSoA sq, DevCounters* prev,
+                                                                   float* film, double* film64, VRec* recs, NRec* nee,
+                                                                   uint32_t max_depth) {
+    __shared__ ClosestSmem m;
+    uint32_t dn = 0, dt = 0;
+    trace_paths<false>(m, s, p, *n_active, ctr, dn, dt);
+    trace_shadow<false, kGuided>(m, s, sq, prev, film, film64, recs, nee, max_depth, dn, dt);
 }
 
 // kz_intersect_closest: rays (o, tmin, d, tmax) in, hit fields out.
@@ -157,42 +223,24 @@ __global__ void __launch_bounds__(256) k_trace_shadow(DevScene s, ShadowSoA sq, 
     if (kCount) warp_count(dn, dt, &ctr->fetch[2]);
 }
 
-// Persistent form of k_trace_shadow for the device-driven loop (k_plan zeroes
-// shadow_next each iteration).
+// Persistent form of k_trace_shadow for the device-driven loop.
 template <bool kCount, bool kGuided>
 __global__ void __launch_bounds__(256, KZ_TRACE_MINB) k_trace_shadow_persistent(DevScene s, ShadowSoA sq, DevCounters* ctr,
                                                                  float* film, double* film64, VRec* recs, NRec* nee,
                                                                  uint32_t max_depth) {
+    __shared__ AnySmem m;
     uint32_t dn = 0, dt = 0;
-    const auto unoccluded = [&](uint32_t ray) {
-        const float4 cc = sq.c4[ray];
-        film_add(film, film64, __float_as_uint(sq.d4[ray].w), xyz(cc));
-        if (kGuided && recs) {
-            const uint32_t tag = __float_as_uint(cc.w);
-            const uint64_t rb = (uint64_t)(tag >> 4) * max_depth;
-            propagate(recs, rb, tag & 15u, xyz(cc));
-            if (nee) nee[rb + (tag & 15u)].n.w = 1.f;
-        }
-    };
-    persistent_any<kCount>(
-        s, ctr->queue.shadow, &ctr->shadow_next,
-        [&](uint32_t k, TRay& r, float& tmax) {
-            const float4 o = sq.o4[k], d = sq.d4[k];
-            r = make_tray(xyz(o), xyz(d), kRayEps);
-            tmax = o.w;
-        },
-        [&](uint32_t ray, int rc) {
-            if (rc < 0) set_status(&ctr->status, KZ_ERR_STACK);
-            if (rc == 1) unoccluded(ray);
-        },
-        dn, dt);
+    trace_shadow<kCount, kGuided>(m, s, sq, ctr, film, film64, recs, nee, max_depth, dn, dt);
     if (kCount) warp_count(dn, dt, &ctr->fetch[2]);
 }
 
-__global__ void __launch_bounds__(256, KZ_TRACE_MINB) k_trace_paths_batch(const DevJob* __restrict__ jobs, PathSoA p,
-                                                                          DevCounters* ctr) {
+// Batched jobs: as k_trace_both (prev == nullptr: closest hits only).
+__global__ void __launch_bounds__(256, KZ_TRACE_MINB) k_trace_both_batch(const DevJob* __restrict__ jobs, PathSoA p,
+                                                                         const uint32_t* n_active, DevCounters* ctr,
+                                                                         ShadowSoA sq, DevCounters* prev) {
     __shared__ ClosestSmem m;
-    batch_trace_paths(m, jobs, p, ctr);
+    batch_trace_paths(m, jobs, p, *n_active, ctr);
+    if (prev) batch_trace_shadow(m, jobs, sq, prev);
 }
 
 __global__ void __launch_bounds__(256, KZ_TRACE_MINB) k_trace_shadow_batch(const DevJob* __restrict__ jobs,
@@ -211,7 +259,7 @@ void launch_intersect_closest(const DevScene& s, const kz_ray* rays, uint64_t n,
                               unsigned long long* next, uint32_t* status, cudaStream_t st) {
     if (!n) return;
     static const unsigned g = resident_grid(k_intersect_closest_persistent, 256);
-    k_intersect_closest_persistent<<<(unsigned)std::min<uint64_t>(g, grid_for(n, 256)), 256, 0, st>>>(s, rays, n, hits,
+    k_intersect_closest_persistent<<<trace_grid(n, g), 256, 0, st>>>(s, rays, n, hits,
                                                                                                      next, status);
 }
 
@@ -219,7 +267,7 @@ void launch_intersect_any(const DevScene& s, const kz_ray* rays, uint64_t n, uin
                           unsigned long long* next, uint32_t* status, cudaStream_t st) {
     if (!n) return;
     static const unsigned g = resident_grid(k_intersect_any_persistent, 256);
-    k_intersect_any_persistent<<<(unsigned)std::min<uint64_t>(g, grid_for(n, 256)), 256, 0, st>>>(s, rays, n, occ,
+    k_intersect_any_persistent<<<trace_grid(n, g), 256, 0, st>>>(s, rays, n, occ,
                                                                                                  next, status);
 }
 
@@ -236,39 +284,47 @@ void launch_trace_paths(const DevScene& s, PathSoA p, uint32_t n, DevCounters* c
     else k_trace_paths<false><<<grid_for(n, block), block, 0, st>>>(s, p, n, ctr, nullptr);
 }
 
-// The device-driven loop's closest-hit pass: persistent, 256-thread blocks,
-// as many as are resident.
-void launch_trace_paths_dev(const DevScene& s, PathSoA p, uint32_t cap, DevCounters* ctr, bool count, uint32_t,
-                            cudaStream_t st) {
+void launch_trace_paths_dev(const DevScene& s, PathSoA p, uint32_t cap, const uint32_t* n_active, DevCounters* ctr,
+                            bool count, cudaStream_t st) {
     if (!cap) return;
     if (count) {
         static const unsigned g = resident_grid(k_trace_paths_persistent<true>, 256);
-        k_trace_paths_persistent<true><<<std::min(g, grid_for(cap, 256)), 256, 0, st>>>(s, p, ctr);
+        k_trace_paths_persistent<true><<<trace_grid(cap, g), 256, 0, st>>>(s, p, n_active, ctr);
     } else {
         static const unsigned g = resident_grid(k_trace_paths_persistent<false>, 256);
-        k_trace_paths_persistent<false><<<std::min(g, grid_for(cap, 256)), 256, 0, st>>>(s, p, ctr);
+        k_trace_paths_persistent<false><<<trace_grid(cap, g), 256, 0, st>>>(s, p, n_active, ctr);
     }
 }
 
-void launch_trace_shadow_guided(const DevScene& s, ShadowSoA sq, uint32_t n_max, DevCounters* ctr, float* film,
-                                double* film64, VRec* recs, NRec* nee, uint32_t max_depth, uint32_t block,
-                                cudaStream_t st) {
-    if (!n_max) return;
-    static const unsigned g = resident_grid(k_trace_shadow_persistent<false, true>, 256);
-    k_trace_shadow_persistent<false, true><<<std::min(g, grid_for(n_max, 256)), 256, 0, st>>>(
-        s, sq, ctr, film, film64, recs, nee, max_depth);
+void launch_trace_both(const DevScene& s, PathSoA p, uint32_t cap, const uint32_t* n_active, DevCounters* ctr,
+                       ShadowSoA sq, DevCounters* prev, float* film, double* film64, const GuideShade* gs,
+                       uint32_t max_depth, cudaStream_t st) {
+    if (!cap) return;
+    if (gs) {
+        static const unsigned g = resident_grid(k_trace_both<true>, 256);
+        k_trace_both<true><<<trace_grid(cap, g), 256, 0, st>>>(
+            s, p, n_active, ctr, sq, prev, film, film64, gs->recs, gs->nee, max_depth);
+    } else {
+        static const unsigned g = resident_grid(k_trace_both<false>, 256);
+        k_trace_both<false><<<trace_grid(cap, g), 256, 0, st>>>(s, p, n_active, ctr, sq, prev,
+                                                                                    film, film64, nullptr, nullptr, 0);
+    }
 }
 
 void launch_trace_shadow_dev(const DevScene& s, ShadowSoA sq, uint32_t n_max, DevCounters* ctr, bool count,
-                             float* film, double* film64, cudaStream_t st) {
+                             float* film, double* film64, const GuideShade* gs, uint32_t max_depth, cudaStream_t st) {
     if (!n_max) return;
-    if (count) {
+    if (gs) {
+        static const unsigned g = resident_grid(k_trace_shadow_persistent<false, true>, 256);
+        k_trace_shadow_persistent<false, true><<<trace_grid(n_max, g), 256, 0, st>>>(
+            s, sq, ctr, film, film64, gs->recs, gs->nee, max_depth);
+    } else if (count) {
         static const unsigned g = resident_grid(k_trace_shadow_persistent<true, false>, 256);
-        k_trace_shadow_persistent<true, false><<<std::min(g, grid_for(n_max, 256)), 256, 0, st>>>(
+        k_trace_shadow_persistent<true, false><<<trace_grid(n_max, g), 256, 0, st>>>(
             s, sq, ctr, film, film64, nullptr, nullptr, 0);
     } else {
         static const unsigned g = resident_grid(k_trace_shadow_persistent<false, false>, 256);
-        k_trace_shadow_persistent<false, false><<<std::min(g, grid_for(n_max, 256)), 256, 0, st>>>(
+        k_trace_shadow_persistent<false, false><<<trace_grid(n_max, g), 256, 0, st>>>(
             s, sq, ctr, film, film64, nullptr, nullptr, 0);
     }
 }
@@ -285,7 +341,7 @@ void launch_trace_shadow(const DevScene& s, ShadowSoA sq, uint32_t n_max, DevCou
 }
 
 static unsigned grid_trace_batch() {
-    static const unsigned g = resident_grid(k_trace_paths_batch, 256);
+    static const unsigned g = resident_grid(k_trace_both_batch, 256);
     return g;
 }
 
@@ -299,14 +355,16 @@ void prepare_batch_wavefront() {
     (void)grid_shadow_batch();
 }
 
-void launch_trace_paths_batch(const DevJob* jobs, PathSoA p, uint32_t cap, DevCounters* ctr, cudaStream_t st) {
+void launch_trace_both_batch(const DevJob* jobs, PathSoA p, uint32_t cap, const uint32_t* n_active, DevCounters* ctr,
+                             ShadowSoA sq, DevCounters* prev, cudaStream_t st) {
     if (!cap) return;
-    k_trace_paths_batch<<<std::min(grid_trace_batch(), grid_for(cap, 256)), 256, 0, st>>>(jobs, p, ctr);
+    k_trace_both_batch<<<trace_grid(cap, grid_trace_batch()), 256, 0, st>>>(jobs, p, n_active,
+                                                                                               ctr, sq, prev);
 }
 
 void launch_trace_shadow_batch(const DevJob* jobs, ShadowSoA sq, uint32_t cap, DevCounters* ctr, cudaStream_t st) {
     if (!cap) return;
-    k_trace_shadow_batch<<<std::min(grid_shadow_batch(), grid_for(cap, 256)), 256, 0, st>>>(jobs, sq, ctr);
+    k_trace_shadow_batch<<<trace_grid(cap, grid_shadow_batch()), 256, 0, st>>>(jobs, sq, ctr);
 }
 
 }  // namespace kz

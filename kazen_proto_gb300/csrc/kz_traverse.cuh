@@ -484,7 +484,7 @@ struct LeafShare {
     unsigned long long* key;  // [256] closest: best (t, id); any hit: tmax bits
     uint32_t* rec;            // [256] closest: record of the best; any hit: mask of the triangles hit
     float4* vwdt;             // [256] closest: V, W, det, t of the best
-    uint4* ent;               // [steps * 256] pending groups of a warp: bits, valid, base, start | lane << 16
+    uint4* ent;               // [steps * 32] this warp's pending groups: bits, valid, base, start | lane << 16
 };
 
 __device__ __forceinline__ void publish_ray(const LeafShare& sh, const TRay& r) {
@@ -545,12 +545,11 @@ __device__ __forceinline__ uint32_t publish_groups(const LeafShare& sh, const Le
     uint32_t rank = 0, at = incl - cnt;
 #pragma unroll
     for (int k = 0; k < K; ++k) rank += __popc(__ballot_sync(0xFFFFFFFFu, g[k].bits != 0) & lt);
-    uint4* ent = sh.ent + (threadIdx.x - lane) * K;
 #pragma unroll
     for (int k = 0; k < K; ++k) {
         start[k] = at;
         if (g[k].bits) {
-            ent[rank++] = make_uint4(g[k].bits, g[k].valid, g[k].base, at | (lane << 16));
+            sh.ent[rank++] = make_uint4(g[k].bits, g[k].valid, g[k].base, at | (lane << 16));
             at += __popc(g[k].bits);
         }
     }
@@ -581,7 +580,7 @@ __device__ __forceinline__ LeafPair leaf_pair(const LeafShare& sh, const LeafGro
     lp.rec = 0;
     lp.live = base + lane < total;
     if (lp.live) {
-        const uint4 e = sh.ent[(threadIdx.x - lane) * K + idx];
+        const uint4 e = sh.ent[idx];
         lp.bit = nth_set_bit(e.x, base + lane - (e.w & 0xFFFFu));
         lp.owner = e.w >> 16;
         lp.rec = leaf_record(e.z, e.y, lp.bit);
@@ -779,21 +778,29 @@ constexpr uint32_t kAnyRefill = KZ_ANY_REFILL;
 // remain and 1 when none do; leaves(groups) runs on all 32 lanes; finish(rc)
 // on the busy lanes returns true once the ray is finished and its result
 // written.
+//
+// Few rays are spread over the grid's warps: only the first ceil(n / warps)
+// lanes of each take rays then, the others help with the leaf tests. A launch
+// that does not fill the device takes as long as its longest ray, and a warp's
+// step is the shorter the fewer rays it steps.
 template <int K, typename Ctr, typename Start, typename Node, typename Leaves, typename Finish>
 __device__ __forceinline__ void persistent_rays_shared(Ctr n, Ctr* next, uint32_t refill, Start start, Node node,
                                                        Leaves leaves, Finish finish) {
-    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t lane = threadIdx.x & 31u, warps = gridDim.x * (blockDim.x >> 5);
+    const uint32_t take = n >= (Ctr)warps * 32u ? 32u : (uint32_t)((n + (warps - 1u)) / warps);
+    const uint32_t takers = 0xFFFFFFFFu >> (32u - (take ? take : 1u));
+    refill = min(refill, take);
     bool busy = false, more = true;
     for (;;) {
-        const uint32_t idle = __ballot_sync(0xFFFFFFFFu, !busy);
-        if (!more && idle == 0xFFFFFFFFu) break;
+        const uint32_t idle = __ballot_sync(0xFFFFFFFFu, !busy) & takers;
+        if (!more && idle == takers) break;
         const uint32_t n_idle = __popc(idle);
         if (more && n_idle >= refill) {
             Ctr base = 0;
             if (lane == 0) base = atomicAdd(next, (Ctr)n_idle);
             base = __shfl_sync(0xFFFFFFFFu, base, 0);
             if (base + n_idle >= n) more = false;
-            if (!busy) {
+            if (!busy && ((takers >> lane) & 1u)) {
                 const Ctr k = base + __popc(idle & ((1u << lane) - 1u));
                 if (k < n) {
                     busy = true;
