@@ -5,65 +5,79 @@
 // Queries come in any order of closure kinds, and the kinds are branches of
 // one switch: a warp of 32 arbitrary queries runs most of the 21 branches with
 // one or two lanes each, the FP64 Beckmann sampler among them. So a block
-// stages a tile of queries in shared memory (coalesced), groups them by kind
-// with a counting sort, and each thread then works on queries of the sorted
-// order; results replace their query's own inputs in the tile and leave
-// coalesced. Values are those of the ungrouped kernel, bit for bit.
+// groups a tile of queries by kind with a counting sort in shared memory, and
+// its warps work through the sorted order, the FP64 searches first. Directions
+// and results move coalesced through the tile, results in place of their
+// query's own inputs. Values are those of the ungrouped kernel, bit for bit.
 //
 // 1,000,003 queries over 21 kinds (221 bytes each over both calls, 33 us at
-// the measured copy rate): evaluation 567 -> 140 us, sampling 4,856 -> 700 us.
-// The sampling that is left is bound by FP64: the Beckmann slope search of
-// one query in ten, on an FP64 rate of two lanes a clock and SM.
+// the measured copy rate), evaluation and sampling: 5,450 -> 480 us, 110 of it
+// evaluation. Bound by FP64: the Beckmann slope search of one query in ten, on
+// an FP64 rate of two lanes a clock and SM (queries of Beckmann lobes alone
+// take 1.8 us a thousand, of the others 0.07). The lobes themselves stay out of
+// the tile: with them in it two blocks fit an SM instead of four, and fewer
+// searches were in flight (717 us; 860 with the searches last).
 #include "kz_stages.cuh"
 
 namespace kz {
 namespace {
 
 constexpr int kClosureThreads = 256;
-constexpr int kLobeWords = sizeof(kz_lobe) / 4;
-constexpr int kLobeStride = kLobeWords + 1;  // words; odd, so that a word of 32 records lies in 32 banks
+constexpr int kClosureBlocks = 4;  // per SM: 64 registers a thread
 constexpr int kKinds = 32;
 
-// Bin of a lobe in the grouping: its closure id (all below 27 but the
-// conductor's), the Beckmann form of the two microfacet kinds apart.
+// Bin of a lobe in the grouping: by closure id, largest first (all are below 27
+// but the conductor's), the Beckmann form of the two microfacet kinds in bins
+// of its own before them: a tile starts with the FP64 searches, which take as
+// long as the rest of it, and its other warps work through the rest meanwhile.
 __device__ __forceinline__ uint32_t closure_kind(uint32_t id, float dist) {
     if (id == KZ_CLOSURE_KP_GLOSS || id == KZ_CLOSURE_KP_GLASS)
-        return dist == (float)KZ_DIST_BECKMANN ? id + 10u : id;
-    return id < 27u ? id : id == KZ_CLOSURE_CONDUCTOR_GGX ? 27u : 31u;
+        return dist == (float)KZ_DIST_BECKMANN ? 21u - id : 31u - id;
+    return id < 27u ? 31u - id : id == KZ_CLOSURE_CONDUCTOR_GGX ? 4u : 0u;
 }
 
-// A tile of kItems * 256 queries: lobes, two directions each (for sampling
-// the second holds the uniforms), and the sorted order.
+// A tile of kItems * 256 queries: two directions each (for sampling the second
+// holds the uniforms), the sorted order, and what a result does not fit into
+// its inputs. Lobes stay in global memory: a thread reads its query's whole
+// record, two sectors, and the kinds read before have brought one of them near.
 template <int kItems>
 struct ClosureTile {
     static constexpr int kN = kItems * kClosureThreads;
-    uint32_t lobe[kN * kLobeStride];
-    float a[kN * 3], b[kN * 3];
+    float a[kN * 3], b[kN * 3], pdf[kN];
     uint16_t order[kN];
-    uint32_t count[kKinds];
+    uint8_t flags[kN];
+    uint32_t count[kKinds], next;
 };
+
+// The warps of a block take the sorted queries 32 at a time; returns the
+// lane's place in the order (m or more: none), done once the warp's first is.
+template <typename Tile>
+__device__ __forceinline__ bool next_queries(Tile& t, uint32_t m, uint32_t& k) {
+    uint32_t first = 0;
+    if ((threadIdx.x & 31u) == 0) first = atomicAdd(&t.next, 32u);
+    first = __shfl_sync(0xFFFFFFFFu, first, 0);
+    k = first + (threadIdx.x & 31u);
+    return first < m;
+}
 
 // Loads the tile's m queries and groups them by kind.
 template <int kItems>
 __device__ __forceinline__ void load_tile(ClosureTile<kItems>& t, const kz_lobe* lobes, const float* a, const float* b,
                                           uint64_t first, uint32_t m) {
     const uint32_t tid = threadIdx.x;
-    const uint32_t* lw = reinterpret_cast<const uint32_t*>(lobes + first);
-    for (uint32_t k = tid; k < m * kLobeWords; k += kClosureThreads)
-        t.lobe[(k / kLobeWords) * kLobeStride + k % kLobeWords] = __ldg(lw + k);
     for (uint32_t k = tid; k < 3 * m; k += kClosureThreads) {
         t.a[k] = __ldg(a + 3 * first + k);
         t.b[k] = __ldg(b + 3 * first + k);
     }
     if (tid < kKinds) t.count[tid] = 0u;
+    if (tid == 0) t.next = 0u;
     __syncthreads();
     uint32_t kind[kItems], rank[kItems];
 #pragma unroll
     for (int j = 0; j < kItems; ++j) {
         const uint32_t q = tid + j * kClosureThreads;
         if (q < m) {
-            const kz_lobe& l = *reinterpret_cast<const kz_lobe*>(t.lobe + q * kLobeStride);
-            kind[j] = closure_kind(l.closure_id, l.params[0]);
+            kind[j] = closure_kind(lobes[first + q].closure_id, lobes[first + q].params[0]);
             rank[j] = atomicAdd(&t.count[kind[j]], 1u);
         }
     }
@@ -94,7 +108,7 @@ __device__ __forceinline__ void put3(float* p, f3 v) {
 }
 
 template <int kItems>
-__global__ void __launch_bounds__(kClosureThreads) k_closure_eval(const kz_lobe* __restrict__ lobes,
+__global__ void __launch_bounds__(kClosureThreads, kClosureBlocks) k_closure_eval(const kz_lobe* __restrict__ lobes,
                                                                   const float* __restrict__ wi,
                                                                   const float* __restrict__ wo, uint64_t n, int conv,
                                                                   float* f, float* pdf) {
@@ -103,22 +117,22 @@ __global__ void __launch_bounds__(kClosureThreads) k_closure_eval(const kz_lobe*
     const uint64_t first = (uint64_t)blockIdx.x * t.kN;
     const uint32_t m = (uint32_t)min((uint64_t)t.kN, n - first);
     load_tile(t, lobes, wi, wo, first, m);
-#pragma unroll 1
-    for (uint32_t k = threadIdx.x; k < m; k += kClosureThreads) {
+    for (uint32_t k; next_queries(t, m, k);) {
+        if (k >= m) continue;
         const uint32_t q = t.order[k];
-        const kz_lobe& l = *reinterpret_cast<const kz_lobe*>(t.lobe + q * kLobeStride);
+        const kz_lobe& l = lobes[first + q];
         const f3 a = ld3(t.a + 3 * q), b = ld3(t.b + 3 * q);
         const LobeEval e = conv == KZ_CONVENTION_REFERENCE ? lobe_eval_reference<true>(l, a, b) : lobe_eval(l, a, b);
         put3(t.a + 3 * q, e.f);
-        t.b[q * 3] = e.pdf;
+        t.pdf[q] = e.pdf;
     }
     __syncthreads();
     for (uint32_t k = threadIdx.x; k < 3 * m; k += kClosureThreads) f[3 * first + k] = t.a[k];
-    for (uint32_t k = threadIdx.x; k < m; k += kClosureThreads) pdf[first + k] = t.b[3 * k];
+    for (uint32_t k = threadIdx.x; k < m; k += kClosureThreads) pdf[first + k] = t.pdf[k];
 }
 
 template <int kItems>
-__global__ void __launch_bounds__(kClosureThreads) k_closure_sample(const kz_lobe* __restrict__ lobes,
+__global__ void __launch_bounds__(kClosureThreads, kClosureBlocks) k_closure_sample(const kz_lobe* __restrict__ lobes,
                                                                     const float* __restrict__ wi,
                                                                     const float* __restrict__ u, uint64_t n, float* wo,
                                                                     float* weight, float* pdf, uint8_t* flags) {
@@ -127,16 +141,15 @@ __global__ void __launch_bounds__(kClosureThreads) k_closure_sample(const kz_lob
     const uint64_t first = (uint64_t)blockIdx.x * t.kN;
     const uint32_t m = (uint32_t)min((uint64_t)t.kN, n - first);
     load_tile(t, lobes, wi, u, first, m);
-#pragma unroll 1
-    for (uint32_t k = threadIdx.x; k < m; k += kClosureThreads) {
+    for (uint32_t k; next_queries(t, m, k);) {
+        if (k >= m) continue;
         const uint32_t q = t.order[k];
-        uint32_t* rec = t.lobe + q * kLobeStride;
-        const LobeSample s = lobe_sample(*reinterpret_cast<const kz_lobe*>(rec), ld3(t.a + 3 * q), t.b[3 * q],
-                                         t.b[3 * q + 1], t.b[3 * q + 2]);
+        const kz_lobe& l = lobes[first + q];
+        const LobeSample s = lobe_sample(l, ld3(t.a + 3 * q), t.b[3 * q], t.b[3 * q + 1], t.b[3 * q + 2]);
         put3(t.a + 3 * q, s.wo);
         put3(t.b + 3 * q, s.weight);
-        rec[0] = __float_as_uint(s.pdf);
-        rec[1] = (s.valid ? 1u : 0u) | (s.delta ? 2u : 0u);
+        t.pdf[q] = s.pdf;
+        t.flags[q] = (uint8_t)((s.valid ? 1 : 0) | (s.delta ? 2 : 0));
     }
     __syncthreads();
     for (uint32_t k = threadIdx.x; k < 3 * m; k += kClosureThreads) {
@@ -144,55 +157,48 @@ __global__ void __launch_bounds__(kClosureThreads) k_closure_sample(const kz_lob
         weight[3 * first + k] = t.b[k];
     }
     for (uint32_t k = threadIdx.x; k < m; k += kClosureThreads) {
-        pdf[first + k] = __uint_as_float(t.lobe[k * kLobeStride]);
-        flags[first + k] = (uint8_t)t.lobe[k * kLobeStride + 1];
+        pdf[first + k] = t.pdf[k];
+        flags[first + k] = t.flags[k];
     }
 }
 
-// Queries per thread: four (a tile of 1,024 holds about 45 of each of 23
-// kinds, more than a warp) once that still gives every SM two tiles, else
-// one, so that small batches spread over more SMs.
-#ifndef KZ_CLOSURE_ITEMS
-#define KZ_CLOSURE_ITEMS 4
-#endif
-bool wide_tiles(uint64_t n) { return n >= (uint64_t)2 * 152 * KZ_CLOSURE_ITEMS * kClosureThreads; }
+// Queries per thread, 1, 2 or 4: a tile of 1,024 holds about 45 of each of 23
+// kinds, more than a warp, but a batch should also spread over the SMs.
+// Evaluation and sampling of 21 kinds / of five principled ones at 1 / 2 / 4
+// (and ungrouped): 16,000 queries 119 / 118 / 119 (168) and 40 / 41 / 50 us
+// (41), 80,000: 158 / 151 / 143 (463) and 43 / 43 / 50 (48), 320,000: 432 / 262
+// / 203 (1,591) and 70 / 61 / 56 (84), 1,000,000: 1,528 / 954 / 483 (5,453) and
+// 152 / 123 / 113 (185).
+int items_per_thread(uint64_t n) { return n < (1u << 16) ? 1 : n < (1u << 18) ? 2 : 4; }
 
-// Tiles above 48 KB need the limit raised (on the current device and context,
-// so with each launch).
-template <typename F>
-void allow_smem(F f, size_t bytes) {
-    cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+template <int kItems>
+void run_eval(const kz_lobe* lobes, const float* wi, const float* wo, uint64_t n, int conv, float* f, float* pdf,
+              cudaStream_t st) {
+    using T = ClosureTile<kItems>;
+    k_closure_eval<kItems><<<grid_for(n, T::kN), kClosureThreads, sizeof(T), st>>>(lobes, wi, wo, n, conv, f, pdf);
 }
+template <int kItems>
+void run_sample(const kz_lobe* lobes, const float* wi, const float* u, uint64_t n, float* wo, float* weight,
+                float* pdf, uint8_t* flags, cudaStream_t st) {
+    using T = ClosureTile<kItems>;
+    k_closure_sample<kItems><<<grid_for(n, T::kN), kClosureThreads, sizeof(T), st>>>(lobes, wi, u, n, wo, weight, pdf,
+                                                                                   flags);
+}
+static_assert(sizeof(ClosureTile<4>) <= 48 * 1024, "a tile fits the default shared memory limit");
 
 }  // namespace
 
 void launch_closure_eval(const kz_lobe* lobes, const float* wi, const float* wo, uint64_t n, int convention,
                          float* f, float* pdf, cudaStream_t st) {
     if (!n) return;
-    if (wide_tiles(n)) {
-        using T = ClosureTile<KZ_CLOSURE_ITEMS>;
-        allow_smem(k_closure_eval<KZ_CLOSURE_ITEMS>, sizeof(T));
-        k_closure_eval<KZ_CLOSURE_ITEMS><<<grid_for(n, T::kN), kClosureThreads, sizeof(T), st>>>(lobes, wi, wo, n,
-                                                                                              convention, f, pdf);
-    } else {
-        using T = ClosureTile<1>;
-        k_closure_eval<1><<<grid_for(n, T::kN), kClosureThreads, sizeof(T), st>>>(lobes, wi, wo, n, convention, f,
-                                                                                 pdf);
-    }
+    const int k = items_per_thread(n);
+    (k == 1 ? run_eval<1> : k == 2 ? run_eval<2> : run_eval<4>)(lobes, wi, wo, n, convention, f, pdf, st);
 }
 void launch_closure_sample(const kz_lobe* lobes, const float* wi, const float* u, uint64_t n, float* wo,
                            float* weight, float* pdf, uint8_t* flags, cudaStream_t st) {
     if (!n) return;
-    if (wide_tiles(n)) {
-        using T = ClosureTile<KZ_CLOSURE_ITEMS>;
-        allow_smem(k_closure_sample<KZ_CLOSURE_ITEMS>, sizeof(T));
-        k_closure_sample<KZ_CLOSURE_ITEMS><<<grid_for(n, T::kN), kClosureThreads, sizeof(T), st>>>(
-            lobes, wi, u, n, wo, weight, pdf, flags);
-    } else {
-        using T = ClosureTile<1>;
-        k_closure_sample<1><<<grid_for(n, T::kN), kClosureThreads, sizeof(T), st>>>(lobes, wi, u, n, wo, weight, pdf,
-                                                                                   flags);
-    }
+    const int k = items_per_thread(n);
+    (k == 1 ? run_sample<1> : k == 2 ? run_sample<2> : run_sample<4>)(lobes, wi, u, n, wo, weight, pdf, flags, st);
 }
 
 }  // namespace kz

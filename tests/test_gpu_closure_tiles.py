@@ -1,6 +1,7 @@
-"""Closure batches at the edges of the grouped kernels' tiles (256 queries, and
-1,024 for large batches): every query's result is the one it has in a batch of
-its own kind in small pieces, bit for bit, whatever surrounds it."""
+"""Closure batches at the edges of the grouped kernels' tiles (256 queries, 512
+from 2^16 and 1,024 from 2^18 queries on): every query's result is the one it
+has in a batch of its own kind in small pieces, bit for bit, whatever surrounds
+it."""
 import numpy as np
 import pytest
 
@@ -10,10 +11,9 @@ from test_gpu_closures import N_KINDS, dirs, lobe_grid
 
 pytestmark = pytest.mark.gpu
 
-WIDE = 2 * 152 * 1024  # first batch size with tiles of 1,024
 
-
-@pytest.mark.parametrize("n", [1, 2, 31, 255, 256, 257, 513, WIDE - 1, WIDE, WIDE + 1, WIDE + 1025])
+@pytest.mark.parametrize("n", [1, 2, 31, 255, 256, 257, 513, 2 ** 16 - 1, 2 ** 16, 2 ** 16 + 513, 2 ** 18 - 1, 2 ** 18,
+                               2 ** 18 + 1, 2 ** 18 + 1025])
 def test_batches_match_their_pieces(gpu, n):
     rng = np.random.default_rng(n)
     base = lobe_grid(rng, 40 * N_KINDS)
