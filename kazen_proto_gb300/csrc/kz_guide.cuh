@@ -115,12 +115,25 @@ __device__ __forceinline__ float mixture_pdf(const VmfMixture& m, f3 w) {
 // exponential per lobe; uses the fast hardware exp/log (relative error near
 // 2^-21, far below the network's own BF16 error). Sampling and the pdf both
 // use this form, so the estimator's weights match the sampled density.
+// The 40 outputs are read as ten 16-byte words (r is 16-byte aligned).
 __device__ __forceinline__ void mixture_for_shading(const float* r, f3 p01, f3 ext, VmfMixture& m) {
+    static_assert(kGuideOut == 5 * kGuideLobes && kGuideOut % 4 == 0, "outputs read as float4");
+    float o[kGuideOut];
+#pragma unroll
+    for (int k = 0; k < kGuideOut / 4; ++k) {
+        const float4 v = __ldcs(reinterpret_cast<const float4*>(r) + k);
+        o[4 * k] = v.x;
+        o[4 * k + 1] = v.y;
+        o[4 * k + 2] = v.z;
+        o[4 * k + 3] = v.w;
+    }
     float mx = -1e30f;
-    for (int k = 0; k < kGuideLobes; ++k) mx = fmaxf(mx, r[5 * k + 4]);
+#pragma unroll
+    for (int k = 0; k < kGuideLobes; ++k) mx = fmaxf(mx, o[5 * k + 4]);
     float s = 0.f;
+#pragma unroll
     for (int k = 0; k < kGuideLobes; ++k) {
-        const float* q = r + 5 * k;
+        const float* q = o + 5 * k;
         const f3 a = lobe_axis(q, p01, ext);
         const float l2 = dot(a, a);
         const float il = l2 > 1e-24f ? rsqrtf(l2) : 0.f;
