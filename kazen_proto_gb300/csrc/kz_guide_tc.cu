@@ -17,13 +17,19 @@
 // its FP32 result in tensor memory is read back by all eight warps
 // (tcgen05.ld, 32 lanes x 32 columns each), which apply bias, ReLU or the
 // ReLU mask and store the BF16 operand of the next product into shared
-// memory. The mixture loss of a row is computed by its half-0 thread (the
-// other half's output columns pass through shared memory). Every
+// memory. The mixture loss of a row is shared by its two threads, four lobes
+// each. Every
 // activation tile is a [128 rows][64] BF16 matrix in the 128-byte-swizzled
 // layout (kz_tc.cuh): K-major for the forward and backward products, and,
 // unchanged, the MN-major transpose for the weight-gradient products (rows
 // are then K). The last layer has 48 columns (40 outputs and 8 zeros); the
 // backward through it contracts 48 of dO's columns.
+//
+// The kernel is bound by latency: a tile is a chain of seven small products, each
+// with a barrier, on eight warps per SM. Measured, 2^18 rows: 268 us with one
+// thread a row, 224 with two that share the products' epilogues only, 193 with
+// the loss shared too and the biases read as 16-byte words (per call, with the
+// host's read of the loss).
 //
 // BF16 rounding points are those of the warp-level kernels (and of the numpy
 // restatement): features, weights, activations after ReLU, dO and the dZ;
@@ -103,6 +109,73 @@ __device__ __forceinline__ uint32_t positive_mask_half(const unsigned char* tile
     return m;
 }
 
+// -log q(w) of a row's mixture and its gradient with respect to the row's raw
+// outputs, shared by the row's two threads: half h holds lobes 4 h .. 4 h + 3
+// (r, g: 5 values each). Per-lobe terms (some ten exponentials, logarithms
+// and divisions each) are computed once, by the lobe's own thread; the sums
+// over the eight lobes are taken by both, in the order of mixture_nll_grad
+// (kz_guide.cuh), so that every value is that function's, bit for bit. `row`:
+// 16 floats of shared memory; `pair`: a barrier of the two threads' warps.
+constexpr int kHalfLobes = kGuideLobes / 2;
+template <typename Sync>
+__device__ __forceinline__ float nll_grad_half(const float (&r)[5 * kHalfLobes], uint32_t half, f3 w, float scale,
+                                               float (&g)[5 * kHalfLobes], f3 p01, f3 ext, float* row, Sync pair) {
+#pragma unroll
+    for (int j = 0; j < kHalfLobes; ++j) row[kHalfLobes * half + j] = r[5 * j + 4];
+    pair();
+    float e[kGuideLobes], mx = -1e30f, s = 0.f, q = 0.f;
+#pragma unroll
+    for (int k = 0; k < kGuideLobes; ++k) {
+        e[k] = row[k];
+        mx = fmaxf(mx, e[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < kGuideLobes; ++k) {
+        e[k] = expf(e[k] - mx);
+        s += e[k];
+    }
+    f3 mu[kHalfLobes];
+    float wt[kHalfLobes], wv[kHalfLobes], kappa[kHalfLobes], kap_raw[kHalfLobes], len[kHalfLobes];
+#pragma unroll
+    for (int j = 0; j < kHalfLobes; ++j) {
+        const f3 a = lobe_axis(r + 5 * j, p01, ext);
+        const float l = sqrtf(dot(a, a));
+        len[j] = l;
+        mu[j] = l > 1e-12f ? mk(a.x / l, a.y / l, a.z / l) : mk(0.f, 0.f, 1.f);
+        kap_raw[j] = kKappaMin + softplus(r[5 * j + 3]);
+        kappa[j] = fminf(kap_raw[j], kKappaMax);
+        wt[j] = (half ? e[kHalfLobes + j] : e[j]) / s;
+        const float v = expf(vmf_log_norm(kappa[j]) + kappa[j] * (dot(mu[j], w) - 1.f));
+        wv[j] = wt[j] * v;
+        row[kGuideLobes + kHalfLobes * half + j] = wv[j];
+    }
+    pair();
+#pragma unroll
+    for (int k = 0; k < kGuideLobes; ++k) q += row[kGuideLobes + k];
+    q = fmaxf(q, 1e-30f);
+#pragma unroll
+    for (int j = 0; j < kHalfLobes; ++j) {
+        float* gk = g + 5 * j;
+        const float resp = wv[j] / q;  // responsibility
+        gk[4] = scale * (wt[j] - resp);
+        const float ek = expf(-2.f * kappa[j]);
+        const float dlogv = 1.f / kappa[j] - 2.f * ek / (1.f - ek) + (dot(mu[j], w) - 1.f);
+        const float dk_dz = kap_raw[j] < kKappaMax ? 1.f / (1.f + expf(-r[5 * j + 3])) : 0.f;
+        gk[3] = scale * (-resp * dlogv * dk_dz);
+        if (len[j] > 1e-12f) {
+            const float c = dot(mu[j], w);
+            const f3 proj = hmul((w - mu[j] * c) * (1.f / len[j]), ext);
+            const float t = -resp * kappa[j] * scale;
+            gk[0] = t * proj.x;
+            gk[1] = t * proj.y;
+            gk[2] = t * proj.z;
+        } else {
+            gk[0] = gk[1] = gk[2] = 0.f;
+        }
+    }
+    return -logf(q);
+}
+
 // D = A (tile at `a`, K-major, K = 16 * ksteps) x B^T (tile at `b`, K-major)
 __device__ __forceinline__ void mma_chain(uint32_t d, uint32_t a, uint32_t b, int ksteps, uint32_t idesc) {
     for (int ks = 0; ks < ksteps; ++ks)
@@ -167,7 +240,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_guide_train_tc(const float4* __
     const uint32_t tmem = *tmem_slot;
     const uint32_t lanes = (uint32_t)(32 * (warp & 3)) << 16;  // this warp's TMEM lane quadrant
     const uint32_t S = tmem + lanes + kScratch + 32u * half;  // this thread's 32 scratch columns
-    float* raw_hi = reinterpret_cast<float*>(sm + oD1);       // [128][8] outputs 32..39 (dZ1's tile is free then)
+    float* pair_terms = reinterpret_cast<float*>(sm + oD1);   // [128][16] of nll_grad_half (dZ1's tile is free then)
 
     const f3 ext = mk(1.f / gd.box_inv.x, 1.f / gd.box_inv.y, 1.f / gd.box_inv.z);
     const float* Wf = gd.wf;
@@ -190,21 +263,17 @@ __global__ void __launch_bounds__(kThreads, 1) k_guide_train_tc(const float4* __
         return *failed == 0u;
     };
     // one product into the scratch accumulator, then this thread's 32 columns
-    // (16 for half 1 of the 48-column product; the rest zero)
+    // (columns 16 .. 47 for half 1 of the 48-column product)
     auto product = [&](uint32_t a, uint32_t b, int ksteps, uint32_t idesc, float (&v)[32], bool narrow) {
         if (t == 0) {
             mma_chain(tmem + kScratch, base + a, base + b, ksteps, idesc);
             umma_commit(bar_mma);
         }
         wait_phase(bar_mma, ph_mma);
-        if (narrow && half) {
-            tmem_ld16(S, v);
-#pragma unroll
-            for (int k = 16; k < 32; ++k) v[k] = 0.f;
-        } else {
-            tmem_ld32(S, v);
-        }
+        tmem_ld32(narrow && half ? S - 16u : S, v);
     };
+    // a barrier of this warp and the one with the other halves of its rows
+    auto pair_sync = [&]() { asm volatile("bar.sync %0, 64;" ::"r"(1 + (warp & 3)) : "memory"); };
 
     for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         const uint32_t r = tile * kT + row;
@@ -216,11 +285,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_guide_train_tc(const float4* __
             const float4 a = samples[3 * si], b = samples[3 * si + 1];
             p = mk(a.x, a.y, a.z);
             nn = mk(b.x, b.y, b.z);
-            if (half == 0) {
-                const float4 c = samples[3 * si + 2];
-                dir = mk(c.x, c.y, c.z);
-                w = fminf(a.w * inv_n, wcap);
-            }
+            const float4 c = samples[3 * si + 2];
+            dir = mk(c.x, c.y, c.z);
+            w = fminf(a.w * inv_n, wcap);
         }
         // the previous tile's weight-gradient products read the tiles rewritten below
         if (any_wg) wait_phase(bar_wg, ph_wg);
@@ -252,39 +319,52 @@ __global__ void __launch_bounds__(kThreads, 1) k_guide_train_tc(const float4* __
             product(ain[l], wl[l], 4, kIdF64, v, false);
             const float* bias = Wf + boff[l] + 32 * half;
 #pragma unroll
-            for (int k = 0; k < 32; ++k) v[k] = fmaxf(v[k] + __ldg(bias + k), 0.f);
+            for (int k = 0; k < 32; k += 4) {
+                const float4 b = __ldg(reinterpret_cast<const float4*>(bias + k));
+                v[k] = fmaxf(v[k] + b.x, 0.f);
+                v[k + 1] = fmaxf(v[k + 1] + b.y, 0.f);
+                v[k + 2] = fmaxf(v[k + 2] + b.z, 0.f);
+                v[k + 3] = fmaxf(v[k + 3] + b.w, 0.f);
+            }
             store_half(sm + aout[l], row, half, v);
             ok = stage_sync();
         }
         if (!ok) break;
-        // ---- outputs, loss and its gradient (the half-0 thread of the row)
+        // ---- outputs, loss and its gradient: lobes 4 half .. 4 half + 3
         product(oH3, oW4, 4, kIdF48, v, true);
-        if (half) {
+        {
+            float raw[20], g[20];  // outputs 20 half .. 20 half + 19
 #pragma unroll
-            for (int k = 0; k < 8; ++k) raw_hi[row * 8 + k] = v[k];  // outputs 32..39
-        }
-        __syncthreads();
-        if (half == 0) {
-            float raw[kGuideOut], g[kGuideOut];
-#pragma unroll
-            for (int k = 0; k < 32; ++k) raw[k] = v[k] + __ldg(Wf + kOffB4 + k);
-#pragma unroll
-            for (int k = 0; k < 8; ++k) raw[32 + k] = raw_hi[row * 8 + k] + __ldg(Wf + kOffB4 + 32 + k);
+            for (int k = 0; k < 20; k += 4) {
+                const float4 b = __ldg(reinterpret_cast<const float4*>(Wf + kOffB4 + 20 * half + k));
+                raw[k] = (half ? v[k + 4] : v[k]) + b.x;
+                raw[k + 1] = (half ? v[k + 5] : v[k + 1]) + b.y;
+                raw[k + 2] = (half ? v[k + 6] : v[k + 2]) + b.z;
+                raw[k + 3] = (half ? v[k + 7] : v[k + 3]) + b.w;
+            }
+            const float nll = nll_grad_half(raw, half, dir, w, g, p, ext, pair_terms + row * 16, pair_sync);
             if (valid) {
-                loss_acc += w * mixture_nll_grad(raw, dir, w, g, p, ext);
+                if (half == 0) loss_acc += w * nll;
             } else {
 #pragma unroll
-                for (int k = 0; k < kGuideOut; ++k) g[k] = 0.f;
+                for (int k = 0; k < 20; ++k) g[k] = 0.f;
             }
-            float lo[32], hi[32];
+            // BF16 columns 20 half .. + 19 of dO's line; half 1 also the zeros up to 63
+            uint32_t h[10];
 #pragma unroll
-            for (int k = 0; k < 32; ++k) lo[k] = g[k];
+            for (int k = 0; k < 10; ++k) h[k] = pack2(g[2 * k], g[2 * k + 1]);
+            unsigned char* line = sm + oDO;
+            if (half == 0) {
+                *reinterpret_cast<uint4*>(line + sw128(row, 0)) = make_uint4(h[0], h[1], h[2], h[3]);
+                *reinterpret_cast<uint4*>(line + sw128(row, 1)) = make_uint4(h[4], h[5], h[6], h[7]);
+                *reinterpret_cast<uint2*>(line + sw128(row, 2)) = make_uint2(h[8], h[9]);
+            } else {
+                *reinterpret_cast<uint2*>(line + sw128(row, 2) + 8) = make_uint2(h[0], h[1]);
+                *reinterpret_cast<uint4*>(line + sw128(row, 3)) = make_uint4(h[2], h[3], h[4], h[5]);
+                *reinterpret_cast<uint4*>(line + sw128(row, 4)) = make_uint4(h[6], h[7], h[8], h[9]);
 #pragma unroll
-            for (int k = 0; k < 8; ++k) hi[k] = g[32 + k];
-#pragma unroll
-            for (int k = 8; k < 32; ++k) hi[k] = 0.f;
-            store_half(sm + oDO, row, 0, lo);
-            store_half(sm + oDO, row, 1, hi);
+                for (int c = 5; c < 8; ++c) *reinterpret_cast<uint4*>(line + sw128(row, c)) = make_uint4(0u, 0u, 0u, 0u);
+            }
         }
         if (!stage_sync()) break;
         // ---- backward: dZ3, dZ2, dZ1
