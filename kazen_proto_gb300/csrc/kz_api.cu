@@ -211,7 +211,9 @@ struct kz_scene {
     DevBuf d_tri_uv, d_mat_tex, d_textures, d_texels, d_tri_nrm;
     kz::DevScene dev;
     DevBuf status;        // uint32 device status word for batch calls
-    uint32_t* status_host = nullptr;  // pinned
+    uint32_t* status_host = nullptr;  // pinned; the few-ray buffer lies behind it
+    unsigned char* few_host = nullptr;  // kFewHost rays and their results (host pointer, and the device's)
+    unsigned char* few_dev = nullptr;
 
     // batch scratch (host-memory calls)
     DevBuf s_rays, s_t, s_prim, s_geom, s_u, s_v, s_occ, s_ctr, s_next;
@@ -241,6 +243,13 @@ struct kz_scene {
 };
 
 namespace {
+
+// A host call of so few rays goes through mapped pinned memory: the kernel reads
+// the rays and writes the hits there itself, in place of a copy from pageable
+// memory and up to five back to it, each of which the host waits for.
+constexpr uint64_t kFewHost = 1024;
+constexpr size_t kFewBytes = sizeof(kz_ray) + 5 * 4;  // ray, t, prim, geom, u, v
+static_assert(kFewHost <= kz::kFewRays, "few host rays take the kernel that needs no fetch counter");
 
 template <typename T>
 kz_status upload(DevBuf& b, const std::vector<T>& v, cudaStream_t st) {
@@ -442,7 +451,7 @@ kz_status run_wavefront(kz_scene* s, const kz::DevCamera* cam, const kz_ray* ray
                 st.kernel_launches += 1;
             }
             if (e) KZ_CUDA(cudaEventRecord(e[1], strm));
-            if (both && it > 0)
+            if (both)  // the first slot has no shadow rays
                 kz::launch_trace_both(s->dev, A, cap, n_active, cur, sq, prev, film, film64, gs, pp.max_depth, strm);
             else
                 kz::launch_trace_paths_dev(s->dev, A, cap, n_active, cur, count, strm);
@@ -499,7 +508,10 @@ kz_status init_cuda(kz_scene* s) {
     KZ_CUDA(cudaGetDevice(&s->device));
     s->cuda_ready = true;  // from here on the destructor releases what exists
     KZ_CUDA(cudaStreamCreateWithFlags(&s->own_stream, cudaStreamNonBlocking));
-    KZ_CUDA(cudaMallocHost((void**)&s->status_host, sizeof(uint32_t)));
+    KZ_CUDA(cudaHostAlloc((void**)&s->status_host, 64 + kFewHost * kFewBytes, cudaHostAllocMapped));
+    s->few_host = reinterpret_cast<unsigned char*>(s->status_host) + 64;
+    KZ_CUDA(cudaHostGetDevicePointer((void**)&s->few_dev, s->status_host, 0));
+    s->few_dev += 64;
     if (!s->stream) s->stream = s->own_stream;
     KZ_TRY(s->status.ensure(sizeof(uint32_t)));
     KZ_CUDA(cudaMemset(s->status.ptr, 0, sizeof(uint32_t)));
@@ -1055,8 +1067,26 @@ kz_status kz_intersect_closest(kz_scene* s, const kz_ray* rays, uint64_t n, kz_h
         KZ_CUDA(cudaStreamSynchronize(st));
         return KZ_OK;
     }
-    KZ_TRY(s->s_next.ensure(sizeof(unsigned long long)));
-    KZ_CUDA(cudaMemsetAsync(s->s_next.ptr, 0, sizeof(unsigned long long), st));
+    if (mem == KZ_MEM_HOST && n <= kFewHost) {
+        std::memcpy(s->few_host, rays, n * sizeof(kz_ray));
+        const size_t at = n * sizeof(kz_ray), step = n * 4;
+        unsigned char* d = s->few_dev + at;
+        const kz_hits dh{reinterpret_cast<float*>(d), reinterpret_cast<uint32_t*>(d + step),
+                         reinterpret_cast<uint32_t*>(d + 2 * step), reinterpret_cast<float*>(d + 3 * step),
+                         reinterpret_cast<float*>(d + 4 * step)};
+        kz::launch_intersect_closest(s->dev, reinterpret_cast<const kz_ray*>(s->few_dev), n, dh, nullptr,
+                                     s->status.as<uint32_t>(), st);
+        KZ_CUDA(cudaGetLastError());
+        const kz_status rc = sync_and_status(s);
+        void* to[5] = {hits.t, hits.prim_id, hits.geom_id, hits.u, hits.v};
+        for (int k = 0; k < 5; ++k)
+            if (to[k]) std::memcpy(to[k], s->few_host + at + k * step, step);
+        return rc;
+    }
+    if (n > kz::kFewRays) {
+        KZ_TRY(s->s_next.ensure(sizeof(unsigned long long)));
+        KZ_CUDA(cudaMemsetAsync(s->s_next.ptr, 0, sizeof(unsigned long long), st));
+    }
     if (mem == KZ_MEM_DEVICE) {
         kz::launch_intersect_closest(s->dev, rays, n, hits, s->s_next.as<unsigned long long>(),
                                      s->status.as<uint32_t>(), st);
@@ -1097,8 +1127,20 @@ kz_status kz_intersect_any(kz_scene* s, const kz_ray* rays, uint64_t n, uint8_t*
         else std::memset(occluded, 0, n);
         return KZ_OK;
     }
-    KZ_TRY(s->s_next.ensure(sizeof(unsigned long long)));
-    KZ_CUDA(cudaMemsetAsync(s->s_next.ptr, 0, sizeof(unsigned long long), st));
+    if (mem == KZ_MEM_HOST && n <= kFewHost) {
+        std::memcpy(s->few_host, rays, n * sizeof(kz_ray));
+        const size_t at = n * sizeof(kz_ray);
+        kz::launch_intersect_any(s->dev, reinterpret_cast<const kz_ray*>(s->few_dev), n, s->few_dev + at, nullptr,
+                                 s->status.as<uint32_t>(), st);
+        KZ_CUDA(cudaGetLastError());
+        const kz_status rc = sync_and_status(s);
+        std::memcpy(occluded, s->few_host + at, n);
+        return rc;
+    }
+    if (n > kz::kFewRays) {
+        KZ_TRY(s->s_next.ensure(sizeof(unsigned long long)));
+        KZ_CUDA(cudaMemsetAsync(s->s_next.ptr, 0, sizeof(unsigned long long), st));
+    }
     if (mem == KZ_MEM_DEVICE) {
         kz::launch_intersect_any(s->dev, rays, n, occluded, s->s_next.as<unsigned long long>(),
                                  s->status.as<uint32_t>(), st);

@@ -203,6 +203,12 @@ struct BatchCounters {
 };
 
 // ---- launchers (kz_kernels.cu) -------------------------------------------
+// At most so many rays take a warp each (warp_traverse), in the calls on rays
+// and in the stages of wavefronts up to the joint trace's size. Closest hits
+// through 250,000 triangles, a warp a ray / a lane a ray: 2,000 rays 52 / 119 us,
+// 4,000 51 / 127, 16,000 88 / 127, 32,000 138 / 152; through 2,000 triangles 27 /
+// 41, 27 / 40, 43 / 42, 63 / 44.
+constexpr uint64_t kFewRays = 16384;
 // Nodes as the builder writes them to the layout the traversal reads, in place.
 void launch_pack_nodes(uint4* nodes, uint32_t n, cudaStream_t st);
 // `next` is a zeroed 64-bit fetch counter for the persistent kernel.

@@ -189,6 +189,14 @@ __device__ __forceinline__ void persistent_closest_in(ClosestSmem& m, DevScene& 
         });
 }
 
+// A warp's stack where its pending groups lie otherwise (other warps of the
+// block may be in the persistent loops).
+template <typename Smem>
+__device__ __forceinline__ uint2* warp_stack(Smem& m) {
+    static_assert(kAnySteps * 32 * sizeof(uint4) >= kWarpStack * sizeof(uint2), "a warp's lists hold its stack");
+    return reinterpret_cast<uint2*>(any_share(m).ent);
+}
+
 // The same with the block's own static shared memory.
 template <bool kCount, bool kOwnScene = false, typename Ctr, typename Load, typename Store>
 __device__ __forceinline__ void persistent_closest(DevScene& s, Ctr n, Ctr* next, uint32_t* status, Load load,
@@ -244,6 +252,30 @@ __device__ __forceinline__ void persistent_any(DevScene& s, Ctr n, Ctr* next, Lo
                                                uint32_t& dt) {
     __shared__ AnySmem m;
     persistent_any_in<kCount, kOwnScene>(m, s, n, next, load, done, dn, dt);
+}
+
+// At most kFewRays rays, a warp per ray: load, store and done as in the
+// persistent loops (load on every lane, store and done on one).
+template <typename Load, typename Store>
+__device__ __forceinline__ void few_closest(ClosestSmem& m, DevScene& s, uint32_t n, uint32_t* next, uint32_t* status,
+                                            Load load, Store store) {
+    warp_rays(n, next, [&](uint32_t k) {
+        TRay r;
+        float tmax;
+        load(k, r, tmax);
+        if (!warp_closest(s, r, tmax, warp_stack(m), [&](const HitRec& h) { store(k, h); }))
+            set_status(status, KZ_ERR_STACK);
+    });
+}
+template <typename Smem, typename Load, typename Done>
+__device__ __forceinline__ void few_any(Smem& m, DevScene& s, uint32_t n, uint32_t* next, Load load, Done done) {
+    warp_rays(n, next, [&](uint32_t k) {
+        TRay r;
+        float tmax;
+        load(k, r, tmax);
+        const int rc = warp_any(s, r, tmax, warp_stack(m));
+        if ((threadIdx.x & 31u) == 0) done(k, rc);
+    });
 }
 
 __device__ __forceinline__ void film_add(float* film, double* film64, uint32_t idx, f3 c) {
@@ -808,15 +840,19 @@ __device__ __forceinline__ void batch_trace_paths(ClosestSmem& m, const DevJob* 
                                                   uint32_t n, DevCounters* ctr) {
     uint32_t dn = 0, dt = 0;
     DevScene ls;
-    persistent_closest_in<false, true>(
-        m, ls, n, &ctr->trace_next, &ctr->status,
-        [&](uint32_t k, TRay& r, float& tmax) {
-            const float4 o = p.o4[k], d = p.d4[k];
-            trace_fields(ls, jobs[__float_as_uint(d.w) >> kJobShift].scene);
-            r = make_tray(xyz(o), xyz(d), kRayEps);
-            tmax = __int_as_float(0x7f800000);
-        },
-        [&](uint32_t k, const HitRec& h) { p.hit[k] = make_float4(h.t, h.u, h.v, __int_as_float(h.rec)); }, dn, dt);
+    const auto load = [&](uint32_t k, TRay& r, float& tmax) {
+        const float4 o = p.o4[k], d = p.d4[k];
+        trace_fields(ls, jobs[__float_as_uint(d.w) >> kJobShift].scene);
+        r = make_tray(xyz(o), xyz(d), kRayEps);
+        tmax = __int_as_float(0x7f800000);
+    };
+    const auto store = [&](uint32_t k, const HitRec& h) {
+        p.hit[k] = make_float4(h.t, h.u, h.v, __int_as_float(h.rec));
+    };
+    if (n <= kFewRays)
+        few_closest(m, ls, n, &ctr->trace_next, &ctr->status, load, store);
+    else
+        persistent_closest_in<false, true>(m, ls, n, &ctr->trace_next, &ctr->status, load, store, dn, dt);
 }
 
 // Shadow rays of the wavefront; an unoccluded one adds its contribution to
@@ -826,21 +862,22 @@ __device__ __forceinline__ void batch_trace_shadow(Smem& m, const DevJob* __rest
                                                    DevCounters* ctr) {
     uint32_t dn = 0, dt = 0;
     DevScene ls;
-    persistent_any_in<false, true>(
-        m, ls, ctr->queue.shadow, &ctr->shadow_next,
-        [&](uint32_t k, TRay& r, float& tmax) {
-            const float4 o = sq.o4[k], d = sq.d4[k];
-            trace_fields(ls, jobs[__float_as_uint(sq.c4[k].w)].scene);
-            r = make_tray(xyz(o), xyz(d), kRayEps);
-            tmax = o.w;
-        },
-        [&](uint32_t ray, int rc) {
-            if (rc < 0) set_status(&ctr->status, KZ_ERR_STACK);
-            if (rc == 1)
-                film_add(jobs[__float_as_uint(sq.c4[ray].w)].film, nullptr, __float_as_uint(sq.d4[ray].w),
-                         xyz(sq.c4[ray]));
-        },
-        dn, dt);
+    const auto load = [&](uint32_t k, TRay& r, float& tmax) {
+        const float4 o = sq.o4[k], d = sq.d4[k];
+        trace_fields(ls, jobs[__float_as_uint(sq.c4[k].w)].scene);
+        r = make_tray(xyz(o), xyz(d), kRayEps);
+        tmax = o.w;
+    };
+    const auto done = [&](uint32_t ray, int rc) {
+        if (rc < 0) set_status(&ctr->status, KZ_ERR_STACK);
+        if (rc == 1)
+            film_add(jobs[__float_as_uint(sq.c4[ray].w)].film, nullptr, __float_as_uint(sq.d4[ray].w),
+                     xyz(sq.c4[ray]));
+    };
+    if (ctr->queue.shadow <= kFewRays)
+        few_any(m, ls, ctr->queue.shadow, &ctr->shadow_next, load, done);
+    else
+        persistent_any_in<false, true>(m, ls, ctr->queue.shadow, &ctr->shadow_next, load, done, dn, dt);
 }
 
 // Camera path g (over all jobs) into slot k.

@@ -13,15 +13,10 @@
 namespace kz {
 namespace {
 
-// Blocks for n rays (persistent kernels of `resident` blocks): 256 rays a
-// block, but for fewer rays than that gives every SM a block, 8 a block, one a
-// warp (persistent_rays_shared spreads them). 64 rays through 20,000 triangles:
-// 131 us in one block, 114 in eight; but 65,537 Li rays 600 us over all
-// resident blocks against 540 over 257: there the warps' steps, not the longest
-// ray, are waited for.
-unsigned trace_grid(uint64_t n, unsigned resident) {
-    const uint64_t full = (n + 255) / 256, spread = std::min<uint64_t>((n + 7) / 8, 152);
-    return (unsigned)std::min<uint64_t>(resident, std::max(full, spread));
+// Blocks of a stage of at most `cap` rays: all that are resident, since few rays
+// take a warp each; larger queues leave the rest idle (trace_blocks).
+unsigned stage_grid(uint64_t cap, unsigned resident) {
+    return (unsigned)std::min<uint64_t>(resident, (cap + 7) / 8);
 }
 
 // A node of the builder's layout (kz_bvh.h) to the traversal's (WideAxis,
@@ -113,18 +108,24 @@ __global__ void __launch_bounds__(256) k_trace_paths(DevScene s, PathSoA p, uint
     if (kCount) warp_count(dn, dt, &ctr->fetch[0]);
 }
 
-// Closest hits of the wavefront's paths.
-template <bool kCount>
+// Closest hits of the wavefront's paths. kFew: with the way of few rays beside
+// the persistent loop; the kernel of wavefronts above the joint trace's size
+// leaves it out, its registers cost the loop 2 % there.
+template <bool kCount, bool kFew>
 __device__ __forceinline__ void trace_paths(ClosestSmem& m, DevScene& s, PathSoA p, uint32_t n, DevCounters* ctr,
                                             uint32_t& dn, uint32_t& dt) {
-    persistent_closest_in<kCount, false>(
-        m, s, n, &ctr->trace_next, &ctr->status,
-        [&](uint32_t k, TRay& r, float& tmax) {
-            const float4 o = p.o4[k], d = p.d4[k];
-            r = make_tray(xyz(o), xyz(d), kRayEps);
-            tmax = __int_as_float(0x7f800000);
-        },
-        [&](uint32_t k, const HitRec& h) { p.hit[k] = make_float4(h.t, h.u, h.v, __int_as_float(h.rec)); }, dn, dt);
+    const auto load = [&](uint32_t k, TRay& r, float& tmax) {
+        const float4 o = p.o4[k], d = p.d4[k];
+        r = make_tray(xyz(o), xyz(d), kRayEps);
+        tmax = __int_as_float(0x7f800000);
+    };
+    const auto store = [&](uint32_t k, const HitRec& h) {
+        p.hit[k] = make_float4(h.t, h.u, h.v, __int_as_float(h.rec));
+    };
+    if (kFew && n <= kFewRays)
+        few_closest(m, s, n, &ctr->trace_next, &ctr->status, load, store);
+    else
+        persistent_closest_in<kCount, false>(m, s, n, &ctr->trace_next, &ctr->status, load, store, dn, dt);
 }
 
 // The shadow rays queued in iteration `ctr`; an unoccluded one adds its
@@ -143,18 +144,20 @@ __device__ __forceinline__ void trace_shadow(Smem& m, DevScene& s, ShadowSoA sq,
             if (nee) nee[rb + (tag & 15u)].n.w = 1.f;
         }
     };
-    persistent_any_in<kCount, false>(
-        m, s, ctr->queue.shadow, &ctr->shadow_next,
-        [&](uint32_t k, TRay& r, float& tmax) {
-            const float4 o = sq.o4[k], d = sq.d4[k];
-            r = make_tray(xyz(o), xyz(d), kRayEps);
-            tmax = o.w;
-        },
-        [&](uint32_t ray, int rc) {
-            if (rc < 0) set_status(&ctr->status, KZ_ERR_STACK);
-            if (rc == 1) unoccluded(ray);
-        },
-        dn, dt);
+    const auto load = [&](uint32_t k, TRay& r, float& tmax) {
+        const float4 o = sq.o4[k], d = sq.d4[k];
+        r = make_tray(xyz(o), xyz(d), kRayEps);
+        tmax = o.w;
+    };
+    const auto done = [&](uint32_t ray, int rc) {
+        if (rc < 0) set_status(&ctr->status, KZ_ERR_STACK);
+        if (rc == 1) unoccluded(ray);
+    };
+    const uint32_t n = ctr->queue.shadow;
+    if (!kCount && n <= kFewRays)
+        few_any(m, s, n, &ctr->shadow_next, load, done);
+    else
+        persistent_any_in<kCount, false>(m, s, n, &ctr->shadow_next, load, done, dn, dt);
 }
 
 template <bool kCount>
@@ -163,7 +166,7 @@ __global__ void __launch_bounds__(256, KZ_TRACE_MINB) k_trace_paths_persistent(D
                                                                                DevCounters* ctr) {
     __shared__ ClosestSmem m;
     uint32_t dn = 0, dt = 0;
-    trace_paths<kCount>(m, s, p, *n_active, ctr, dn, dt);
+    trace_paths<kCount, false>(m, s, p, *n_active, ctr, dn, dt);
     if (kCount) warp_count(dn, dt, &ctr->fetch[0]);
 }
 
@@ -178,7 +181,7 @@ __global__ void __launch_bounds__(256, KZ_TRACE_MINB) k_trace_both(DevScene s, P
                                                                    uint32_t max_depth) {
     __shared__ ClosestSmem m;
     uint32_t dn = 0, dt = 0;
-    trace_paths<false>(m, s, p, *n_active, ctr, dn, dt);
+    trace_paths<false, true>(m, s, p, *n_active, ctr, dn, dt);
     trace_shadow<false, kGuided>(m, s, sq, prev, film, film64, recs, nee, max_depth, dn, dt);
 }
 
@@ -196,6 +199,28 @@ __global__ void __launch_bounds__(256, KZ_TRACE_MINB) k_intersect_closest_persis
             tmax = b.w;
         },
         [&](unsigned long long k, const HitRec& h) { store_hit(s, hits, k, h); }, dn, dt);
+}
+
+// One ray per warp, for calls of few rays (kz_intersect_closest / _any).
+constexpr int kFewWarps = 4;  // per block
+template <bool kAny>
+__global__ void __launch_bounds__(32 * kFewWarps) k_intersect_few(DevScene s, const kz_ray* __restrict__ rays,
+                                                                  uint32_t n, kz_hits hits, uint8_t* occ,
+                                                                  uint32_t* status) {
+    __shared__ uint2 stacks[kFewWarps][kWarpStack];
+    const uint32_t warp = threadIdx.x >> 5, k = blockIdx.x * kFewWarps + warp;
+    if (k >= n) return;
+    const float4* rp = reinterpret_cast<const float4*>(rays + k);
+    const float4 a = __ldg(rp), b = __ldg(rp + 1);
+    const TRay r = make_tray(mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), a.w);
+    uint2* stack = stacks[warp];
+    if (kAny) {
+        const int rc = warp_any(s, r, b.w, stack);
+        if (rc < 0) set_status(status, KZ_ERR_STACK);
+        if ((threadIdx.x & 31u) == 0) occ[k] = rc == 2 ? 1 : 0;
+    } else if (!warp_closest(s, r, b.w, stack, [&](const HitRec& h) { store_hit(s, hits, k, h); })) {
+        set_status(status, KZ_ERR_STACK);
+    }
 }
 
 template <bool kCount, bool kGuided>
@@ -258,16 +283,26 @@ void launch_pack_nodes(uint4* nodes, uint32_t n, cudaStream_t st) {
 void launch_intersect_closest(const DevScene& s, const kz_ray* rays, uint64_t n, kz_hits hits,
                               unsigned long long* next, uint32_t* status, cudaStream_t st) {
     if (!n) return;
+    if (n <= kFewRays) {
+        k_intersect_few<false><<<grid_for(n, kFewWarps), 32 * kFewWarps, 0, st>>>(s, rays, (uint32_t)n, hits, nullptr,
+                                                                                 status);
+        return;
+    }
     static const unsigned g = resident_grid(k_intersect_closest_persistent, 256);
-    k_intersect_closest_persistent<<<trace_grid(n, g), 256, 0, st>>>(s, rays, n, hits,
+    k_intersect_closest_persistent<<<trace_blocks(n, g), 256, 0, st>>>(s, rays, n, hits,
                                                                                                      next, status);
 }
 
 void launch_intersect_any(const DevScene& s, const kz_ray* rays, uint64_t n, uint8_t* occ,
                           unsigned long long* next, uint32_t* status, cudaStream_t st) {
     if (!n) return;
+    if (n <= kFewRays) {
+        k_intersect_few<true><<<grid_for(n, kFewWarps), 32 * kFewWarps, 0, st>>>(s, rays, (uint32_t)n, kz_hits{}, occ,
+                                                                                status);
+        return;
+    }
     static const unsigned g = resident_grid(k_intersect_any_persistent, 256);
-    k_intersect_any_persistent<<<trace_grid(n, g), 256, 0, st>>>(s, rays, n, occ,
+    k_intersect_any_persistent<<<trace_blocks(n, g), 256, 0, st>>>(s, rays, n, occ,
                                                                                                  next, status);
 }
 
@@ -289,10 +324,10 @@ void launch_trace_paths_dev(const DevScene& s, PathSoA p, uint32_t cap, const ui
     if (!cap) return;
     if (count) {
         static const unsigned g = resident_grid(k_trace_paths_persistent<true>, 256);
-        k_trace_paths_persistent<true><<<trace_grid(cap, g), 256, 0, st>>>(s, p, n_active, ctr);
+        k_trace_paths_persistent<true><<<stage_grid(cap, g), 256, 0, st>>>(s, p, n_active, ctr);
     } else {
         static const unsigned g = resident_grid(k_trace_paths_persistent<false>, 256);
-        k_trace_paths_persistent<false><<<trace_grid(cap, g), 256, 0, st>>>(s, p, n_active, ctr);
+        k_trace_paths_persistent<false><<<stage_grid(cap, g), 256, 0, st>>>(s, p, n_active, ctr);
     }
 }
 
@@ -302,11 +337,11 @@ void launch_trace_both(const DevScene& s, PathSoA p, uint32_t cap, const uint32_
     if (!cap) return;
     if (gs) {
         static const unsigned g = resident_grid(k_trace_both<true>, 256);
-        k_trace_both<true><<<trace_grid(cap, g), 256, 0, st>>>(
+        k_trace_both<true><<<stage_grid(cap, g), 256, 0, st>>>(
             s, p, n_active, ctr, sq, prev, film, film64, gs->recs, gs->nee, max_depth);
     } else {
         static const unsigned g = resident_grid(k_trace_both<false>, 256);
-        k_trace_both<false><<<trace_grid(cap, g), 256, 0, st>>>(s, p, n_active, ctr, sq, prev,
+        k_trace_both<false><<<stage_grid(cap, g), 256, 0, st>>>(s, p, n_active, ctr, sq, prev,
                                                                                     film, film64, nullptr, nullptr, 0);
     }
 }
@@ -316,15 +351,15 @@ void launch_trace_shadow_dev(const DevScene& s, ShadowSoA sq, uint32_t n_max, De
     if (!n_max) return;
     if (gs) {
         static const unsigned g = resident_grid(k_trace_shadow_persistent<false, true>, 256);
-        k_trace_shadow_persistent<false, true><<<trace_grid(n_max, g), 256, 0, st>>>(
+        k_trace_shadow_persistent<false, true><<<stage_grid(n_max, g), 256, 0, st>>>(
             s, sq, ctr, film, film64, gs->recs, gs->nee, max_depth);
     } else if (count) {
         static const unsigned g = resident_grid(k_trace_shadow_persistent<true, false>, 256);
-        k_trace_shadow_persistent<true, false><<<trace_grid(n_max, g), 256, 0, st>>>(
+        k_trace_shadow_persistent<true, false><<<stage_grid(n_max, g), 256, 0, st>>>(
             s, sq, ctr, film, film64, nullptr, nullptr, 0);
     } else {
         static const unsigned g = resident_grid(k_trace_shadow_persistent<false, false>, 256);
-        k_trace_shadow_persistent<false, false><<<trace_grid(n_max, g), 256, 0, st>>>(
+        k_trace_shadow_persistent<false, false><<<stage_grid(n_max, g), 256, 0, st>>>(
             s, sq, ctr, film, film64, nullptr, nullptr, 0);
     }
 }
@@ -358,13 +393,13 @@ void prepare_batch_wavefront() {
 void launch_trace_both_batch(const DevJob* jobs, PathSoA p, uint32_t cap, const uint32_t* n_active, DevCounters* ctr,
                              ShadowSoA sq, DevCounters* prev, cudaStream_t st) {
     if (!cap) return;
-    k_trace_both_batch<<<trace_grid(cap, grid_trace_batch()), 256, 0, st>>>(jobs, p, n_active,
+    k_trace_both_batch<<<stage_grid(cap, grid_trace_batch()), 256, 0, st>>>(jobs, p, n_active,
                                                                                                ctr, sq, prev);
 }
 
 void launch_trace_shadow_batch(const DevJob* jobs, ShadowSoA sq, uint32_t cap, DevCounters* ctr, cudaStream_t st) {
     if (!cap) return;
-    k_trace_shadow_batch<<<trace_grid(cap, grid_shadow_batch()), 256, 0, st>>>(jobs, sq, ctr);
+    k_trace_shadow_batch<<<stage_grid(cap, grid_shadow_batch()), 256, 0, st>>>(jobs, sq, ctr);
 }
 
 }  // namespace kz

@@ -779,14 +779,26 @@ constexpr uint32_t kAnyRefill = KZ_ANY_REFILL;
 // on the busy lanes returns true once the ray is finished and its result
 // written.
 //
-// Few rays are spread over the grid's warps: only the first ceil(n / warps)
-// lanes of each take rays then, the others help with the leaf tests. A launch
-// that does not fill the device takes as long as its longest ray, and a warp's
-// step is the shorter the fewer rays it steps.
+// A queue that does not fill the grid: blocks beyond its share leave at once
+// (256 rays a block, but 8 a block, one a warp, while that leaves SMs without
+// one), and of each warp only the first ceil(n / warps) lanes take rays; the
+// others help with the leaf tests. 64 rays through 20,000 triangles took 131 us
+// in one block and 114 in eight, but 65,537 Li rays 600 us over all resident
+// blocks against 540 over 257: there the warps' steps, not the longest ray, are
+// waited for.
+template <typename Ctr>
+__host__ __device__ __forceinline__ uint32_t trace_blocks(Ctr n, uint32_t most) {
+    const Ctr full = (n + 255) / 256, spread = n < 8 * 152 ? (n + 7) / 8 : 152;
+    const Ctr want = full > spread ? full : spread;
+    return want < most ? (uint32_t)want : most;
+}
+
 template <int K, typename Ctr, typename Start, typename Node, typename Leaves, typename Finish>
 __device__ __forceinline__ void persistent_rays_shared(Ctr n, Ctr* next, uint32_t refill, Start start, Node node,
                                                        Leaves leaves, Finish finish) {
-    const uint32_t lane = threadIdx.x & 31u, warps = gridDim.x * (blockDim.x >> 5);
+    const uint32_t blocks = trace_blocks(n, gridDim.x);
+    if (blockIdx.x >= blocks) return;
+    const uint32_t lane = threadIdx.x & 31u, warps = blocks * (blockDim.x >> 5);
     const uint32_t take = n >= (Ctr)warps * 32u ? 32u : (uint32_t)((n + (warps - 1u)) / warps);
     const uint32_t takers = 0xFFFFFFFFu >> (32u - (take ? take : 1u));
     refill = min(refill, take);
@@ -817,6 +829,187 @@ __device__ __forceinline__ void persistent_rays_shared(Ctr n, Ctr* next, uint32_
         }
         leaves(g);
         if (busy && finish(rc)) busy = false;
+    }
+}
+
+// ---- one ray per warp ------------------------------------------------------------
+//
+// A handful of rays cannot fill the device: the call takes as long as its
+// longest ray, and a ray of the loops above waits some 80 instructions of one
+// node's eight slots, one after the other, at every step. Here a warp takes
+// one ray: four nodes of its stack at a time, a lane per slot, and every lane
+// tests its own slot's triangles. The boxes, the triangle test and the order
+// of hits are the same, so the results are the same bits. 64 picked rays from
+// host memory through 20,000 triangles: 105 -> 39 us a call (with the copies gone,
+// kz_api.cu), 65,537 Li rays of depth 5, whose later iterations have few: 536 ->
+// 443 us.
+// Entries of a warp's stack; a ray that needs more falls back on the sequential
+// loop (a test build's small stack is small here too).
+constexpr int kWarpStack = kWideStack < kWideDepthCap ? kWideStack : 128;
+
+struct WarpRay {
+    float t;  // the lane's best, with its terms
+    float V, W, det;
+    uint32_t prim;
+    int32_t rec;
+};
+
+// Traverses one ray with the whole warp; `stack`: its kWarpStack entries of node
+// and entry distance, in shared memory. Returns 1 when it is complete (closest:
+// each lane holds the best of its own triangles; any hit: none found), 2 on a
+// hit (any hit), 0 if the stack was too small, -1 on an abort (as closest_step).
+template <bool kAny>
+__device__ __forceinline__ int warp_traverse(const DevScene& s, const TRay& r, float tmax, uint2* stack, WarpRay& h) {
+    const uint32_t lane = threadIdx.x & 31u, up = 3u - (lane >> 3), lt = (1u << lane) - 1u;
+    const uint32_t flip = 7u ^ ((r.inv.x < 0.f ? 1u : 0u) | (r.inv.y < 0.f ? 2u : 0u) | (r.inv.z < 0.f ? 4u : 0u));
+    const uint32_t slot = (lane & 7u) ^ flip;  // the nearest octant in the highest lane, pushed last
+    const TriRay q = tri_ray(r);
+    const WideDir dir = wide_dir(r);
+    h.t = tmax;
+    h.V = h.W = 0.f;
+    h.det = 1.f;
+    h.prim = KZ_INVALID_ID;
+    h.rec = -1;
+    float tcur = tmax;
+    uint32_t sp = 1, visits = 0;
+    if (lane == 0) stack[0] = make_uint2(0u, __float_as_uint(r.tmin));
+    __syncwarp();
+    while (sp) {
+        // one node at a time when the stack might not hold four nodes' children
+        const uint32_t n = (int)sp > kWarpStack - 32 && kWarpStack > 32 ? 1u : min(sp, 4u);
+        visits += n;
+        if (visits > s.n_nodes) return -1;
+        const uint2 e = up < n ? stack[sp - 1u - up] : make_uint2(0u, 0u);
+        bool alive = up < n && !(__uint_as_float(e.y) > tcur);
+        if (__any_sync(0xFFFFFFFFu, alive && e.x >= s.n_nodes)) return -1;
+        sp -= n;
+        __syncwarp();
+        uint32_t child = 0, tri = 0, leaf = 0;
+        float tn = 0.f;
+        bool inner = false;
+        if (alive) {
+            const uint4* np = s.nodes + (size_t)e.x * 5;
+            const uint4 h0 = __ldg(np), h1 = __ldg(np + 1);
+            const uint32_t* w = reinterpret_cast<const uint32_t*>(np + 2) + (slot >> 1);
+            const uint32_t odd = (slot & 1u) << 5;
+            const auto axis = [&](float p, float scale, float o, float inv, uint32_t word, uint32_t sel, float& lo,
+                                  float& hi) {
+                const WideAxis ax = wide_axis(p, scale, o, inv, make_uint4(0u, 0u, 0u, 0u));
+                lo = fmaf(__uint_as_float(__byte_perm(word, 0x3F800000u, sel | odd)), ax.A, ax.Bn);
+                hi = fmaf(__uint_as_float(__byte_perm(word, 0x3F800000u, (sel ^ 0x10u) | odd)), ax.A, ax.Bf);
+            };
+            float xn, xf, yn, yf, zn, zf;
+            axis(__uint_as_float(h0.x), __uint_as_float(h0.w << 16), r.o.x, r.inv.x, __ldg(w), dir.sx, xn, xf);
+            axis(__uint_as_float(h0.y), __uint_as_float(h0.w & 0xFFFF0000u), r.o.y, r.inv.y, __ldg(w + 4), dir.sy, yn,
+                 yf);
+            axis(__uint_as_float(h0.z), __uint_as_float(h1.w << 16), r.o.z, r.inv.z, __ldg(w + 8), dir.sz, zn, zf);
+            tn = fmaxf(fmaxf(fmaxf(xn, r.tmin), yn), zn);
+            const float tf = fminf(fminf(fminf(xf, tcur), yf), zf);
+            if (tn <= tf) {
+                inner = (h1.z >> (24 + slot)) & 1u;
+                child = h1.x + __popc((h1.z >> 24) & ((1u << slot) - 1u));
+                const uint32_t valid = h1.z & 0x00FFFFFFu;
+                leaf = (valid >> (3u * slot)) & 7u;
+                tri = leaf_record(h1.y, valid, 3u * slot);
+            }
+        }
+        const uint32_t in = __ballot_sync(0xFFFFFFFFu, inner);
+        if (sp + __popc(in) > (uint32_t)kWarpStack) return 0;
+        if (inner) stack[sp + __popc(in & lt)] = make_uint2(child, __float_as_uint(tn));
+        sp += __popc(in);
+        __syncwarp();
+        if (!__any_sync(0xFFFFFFFFu, leaf != 0)) continue;
+        bool hit = false, out = false;
+        for (; leaf; leaf &= leaf - 1u, ++tri) {  // a leaf's triangles are consecutive
+            if (tri >= s.n_tris) {
+                out = true;
+                break;
+            }
+            const float4* tp = s.tris + (size_t)tri * 3;
+            const float4 a = __ldg(tp), b = __ldg(tp + 1), c = __ldg(tp + 2);
+            float t, V, W, det;
+            if (!tri_test_t(q, a, b, c, t, V, W, det) || !(t > r.tmin)) continue;
+            if (kAny) {
+                hit |= t <= tmax;
+            } else {
+                const uint32_t prim = __float_as_uint(a.w);
+                if (t < h.t || (t == h.t && prim < h.prim)) {
+                    h.t = t;
+                    h.V = V;
+                    h.W = W;
+                    h.det = det;
+                    h.prim = prim;
+                    h.rec = (int32_t)tri;
+                }
+            }
+        }
+        if (__any_sync(0xFFFFFFFFu, out)) return -1;
+        if (kAny) {
+            if (__any_sync(0xFFFFFFFFu, hit)) return 2;
+        } else {
+            tcur = fminf(tcur, key_t((unsigned long long)__reduce_min_sync(
+                                         0xFFFFFFFFu, (uint32_t)(hit_key(h.t, 0u) >> 32)) << 32));
+        }
+    }
+    return 1;
+}
+
+// The best of the lanes' hits, in the lane that holds it; true there. (Both
+// reductions are taken by every lane, whether it holds a hit or not.)
+__device__ __forceinline__ bool warp_best(const WarpRay& h) {
+    const uint32_t o = h.rec >= 0 ? (uint32_t)(hit_key(h.t, 0u) >> 32) : 0xFFFFFFFFu;
+    const uint32_t o_min = __reduce_min_sync(0xFFFFFFFFu, o);
+    const bool first = h.rec >= 0 && o == o_min;
+    const uint32_t prim_min = __reduce_min_sync(0xFFFFFFFFu, first ? h.prim : KZ_INVALID_ID);
+    return first && h.prim == prim_min;
+}
+
+// Closest hit of one ray with the whole warp: calls store(hit) on one lane;
+// false on an abort (the hit is a miss then).
+template <typename Store>
+__device__ __forceinline__ bool warp_closest(const DevScene& s, const TRay& r, float tmax, uint2* stack,
+                                             Store store) {
+    WarpRay w;
+    const int rc = warp_traverse<false>(s, r, tmax, stack, w);
+    HitRec h{tmax, 0.f, 0.f, KZ_INVALID_ID, -1};
+    bool mine = (threadIdx.x & 31u) == 0, ok = rc >= 0;
+    if (rc == 1) {
+        const bool best = warp_best(w);
+        if (__any_sync(0xFFFFFFFFu, best)) mine = best;
+        if (best) h = HitRec{w.t, w.V / w.det, w.W / w.det, w.prim, w.rec};
+    } else if (rc == 0 && mine) {
+        uint32_t dn = 0, dt = 0;
+        ok = trace_closest<false>(s, r, tmax, h, dn, dt);
+    }
+    if (mine) store(h);
+    return __all_sync(0xFFFFFFFFu, ok);
+}
+
+// Any hit of one ray with the whole warp: 1 none, 2 a hit, -1 aborted.
+__device__ __forceinline__ int warp_any(const DevScene& s, const TRay& r, float tmax, uint2* stack) {
+    WarpRay w;
+    int rc = warp_traverse<true>(s, r, tmax, stack, w);
+    if (rc == 0) {
+        if ((threadIdx.x & 31u) == 0) {
+            uint32_t dn = 0, dt = 0;
+            bool overflow;
+            rc = trace_any<false>(s, r, tmax, overflow, dn, dt) ? 2 : overflow ? -1 : 1;
+        }
+        rc = __shfl_sync(0xFFFFFFFFu, rc, 0);
+    }
+    return rc;
+}
+
+// The warps of a persistent kernel take the rays [0, n) one at a time:
+// ray(k) runs on the whole warp.
+template <typename Ctr, typename Ray>
+__device__ __forceinline__ void warp_rays(Ctr n, Ctr* next, Ray ray) {
+    for (;;) {
+        Ctr k = 0;
+        if ((threadIdx.x & 31u) == 0) k = atomicAdd(next, (Ctr)1);
+        k = __shfl_sync(0xFFFFFFFFu, k, 0);
+        if (k >= n) break;
+        ray(k);
     }
 }
 

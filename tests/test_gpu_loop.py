@@ -36,7 +36,7 @@ def test_wavefront_sizes_agree(gpu, box, depth, size, flags):
         assert r.last_stats[k] == ref.last_stats[k], k
 
 
-@pytest.mark.parametrize("n", [1, 7, 8, 9, 1215, 1216, 1217, 38911, 38912, 38913])
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 1215, 1216, 1217, 16383, 16384, 16385, 38911, 38912, 38913])
 def test_few_rays_are_spread(gpu, oracle_mod, n):
     tv = scenes.triangle_soup(3000, seed=5)
     rays = scenes.soup_rays(n, seed=n)
