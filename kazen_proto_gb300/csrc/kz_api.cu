@@ -352,6 +352,13 @@ kz_status alloc_counters(kz_scene* s, size_t n) {
 // 8.1 / 8.7 ms a frame, 1 M-path box frame 0.82 / 0.86, 24 jobs in one batch
 // 6.2 / 6.4, 16 M-path slit room 23.3 / 23.0 and terrain 129.0 / 126.5.
 constexpr uint32_t kBothCap = 1u << 23;
+// Samples per pixel from which camera paths are traced in bundles of 32, four
+// pixels of a row or fewer. Frames with bundles / without: terrain 1080p, 64 spp
+// 115.5 / 126.1 ms, slit room 1024 x 1024, 16 spp 22.1 / 23.0, materials 641 x
+// 359, 16 spp 6.95 / 7.16, box 256 x 256, 16 spp 0.81 / 0.83, guided 512 x 512, 8
+// spp 4.90 / 5.02, but preview 97 x 65, 4 spp 0.75 / 0.69: eight pixels of so
+// small an image meet too many boxes.
+constexpr uint32_t kBundleSpp = 8;
 // The queue of split shading for wavefronts large enough for it (else none).
 kz_status alloc_heavy(kz_scene* s, uint32_t cap, kz::HeavyQueue& q) {
     if (cap < kz::split_shading_capacity()) return KZ_OK;
@@ -403,6 +410,7 @@ kz_status run_wavefront(kz_scene* s, const kz::DevCamera* cam, const kz_ray* ray
     const bool timing = (cfg->flags & KZ_RENDER_FLAG_TIMING) != 0;
     const bool count = (cfg->flags & KZ_RENDER_FLAG_COUNT) != 0;
     const bool both = !timing && !count && cap <= kBothCap;
+    const bool bundles = cam && !count && s->dev.n_tris && pp.spp >= kBundleSpp;
     const bool one_wave = total <= cap;
     // otherwise one batch covers the life of two waves of paths: the host waits
     // for the device once per batch, and fewer waits leave fewer idle gaps
@@ -444,20 +452,28 @@ kz_status run_wavefront(kz_scene* s, const kz::DevCamera* cam, const kz_ray* ray
             generated[it] = !one_wave || it == 0;
             if (generated[it]) {
                 const kz::IterSlots slots{cur, prev, last_gen, total, cap};
-                if (cam) kz::launch_generate_camera_dev(*cam, pp, A, slots, block, strm);
+                if (e && bundles) KZ_CUDA(cudaEventRecord(e[1], strm));  // generation counts as tracing then
+                if (bundles) kz::launch_camera_bundles(s->dev, *cam, pp, A, slots, strm);
+                else if (cam) kz::launch_generate_camera_dev(*cam, pp, A, slots, block, strm);
                 else kz::launch_generate_rays_dev(rays_dev, pp, A, slots, block, strm);
                 last_gen = cur;
                 n_active = &cur->n_active;
                 st.kernel_launches += 1;
             }
-            if (e) KZ_CUDA(cudaEventRecord(e[1], strm));
-            if (both)  // the first slot has no shadow rays
-                kz::launch_trace_both(s->dev, A, cap, n_active, cur, sq, prev, film, film64, gs, pp.max_depth, strm);
-            else
-                kz::launch_trace_paths_dev(s->dev, A, cap, n_active, cur, count, strm);
+            if (e && !(bundles && generated[it])) KZ_CUDA(cudaEventRecord(e[1], strm));
+            const uint32_t* n_trace = bundles ? &prev->queue.next : n_active;
+            if (bundles && first_batch && it == 0) {
+                // nothing but camera paths
+            } else if (both) {  // the first slot has no shadow rays
+                kz::launch_trace_both(s->dev, A, cap, n_trace, cur, sq, prev, film, film64, gs, pp.max_depth, strm);
+                st.kernel_launches += 1;
+            } else {
+                kz::launch_trace_paths_dev(s->dev, A, cap, n_trace, cur, count, strm);
+                st.kernel_launches += 1;
+            }
             if (gh) kz::launch_guide_infer_paths_dev(s->dev, A, cap, n_active, gh->gd, gh->raw, strm);
             if (e) KZ_CUDA(cudaEventRecord(e[2], strm));
-            st.kernel_launches += 1 + (gh ? 1 : 0) +
+            st.kernel_launches += (gh ? 1 : 0) +
                                   kz::launch_shade_dev(s->dev, pp, A, cap, B, sq, hq, cur, n_active, film, film64, gs,
                                                        block, strm);
             if (e) KZ_CUDA(cudaEventRecord(e[3], strm));

@@ -173,6 +173,7 @@ struct DevCounters {
     uint32_t gen_count, gen_slot;  // how many, and where in the buffer
     uint32_t trace_next;           // persistent kernels: next path / shadow ray to fetch
     uint32_t shadow_next;
+    uint32_t camera_next;          // camera bundles: next new path to fetch
     uint32_t heavy[kHeavyClasses], heavy_next;  // split shading: paths queued by class, fetch cursor
     uint32_t bar_count, bar_gen;   // grid barrier of the persistent batch kernel
     uint32_t bar_abort;            // set when a barrier wait ran out
@@ -279,6 +280,10 @@ void launch_scale(float* film, double* film64, uint64_t n, float sf, double sd, 
 // are sized for the capacity `cap`; threads beyond the count exit.
 void launch_generate_camera_dev(const DevCamera& cam, const PathParams& pp, PathSoA dst, const IterSlots& it,
                                 uint32_t block, cudaStream_t st);
+// Generates and traces an iteration's camera paths in bundles of 32; the
+// iteration's trace then takes the older paths only.
+void launch_camera_bundles(const DevScene& s, const DevCamera& cam, const PathParams& pp, PathSoA p,
+                           const IterSlots& it, cudaStream_t st);
 void launch_generate_rays_dev(const kz_ray* rays, const PathParams& pp, PathSoA dst, const IterSlots& it,
                               uint32_t block, cudaStream_t st);
 void launch_trace_paths_dev(const DevScene& s, PathSoA p, uint32_t cap, const uint32_t* n_active, DevCounters* ctr,

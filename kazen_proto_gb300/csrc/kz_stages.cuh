@@ -64,8 +64,11 @@ __device__ __forceinline__ void store_hit(const DevScene& s, kz_hits hits, uint6
 }
 
 // ------------------------------------------------------------------ wavefront stages
-__device__ __forceinline__ void generate_camera_path(const DevCamera& cam, const PathParams& pp, PathSoA dst,
-                                                     uint32_t k, uint64_t pid) {
+struct CameraPath {
+    f3 d;
+    unsigned long long rng;
+};
+__device__ __forceinline__ CameraPath camera_path(const DevCamera& cam, const PathParams& pp, uint64_t pid) {
     const uint64_t pix = pid / pp.spp;
     const uint32_t px = (uint32_t)(pix % cam.W), py = (uint32_t)(pix / cam.W);
     Pcg rng;
@@ -79,11 +82,18 @@ __device__ __forceinline__ void generate_camera_path(const DevCamera& cam, const
     const float ny = cam.flip * ((1.0f - 2.0f * sy) / cam.aspect);
     const float cx = nx * cam.tan_half;
     const float cy = ny * cam.tan_half;
-    const f3 d = normalize(ld3(cam.x) * cx + ld3(cam.y) * cy + ld3(cam.z) * (-1.0f));
+    return CameraPath{normalize(ld3(cam.x) * cx + ld3(cam.y) * cy + ld3(cam.z) * (-1.0f)), rng.state};
+}
+__device__ __forceinline__ void store_camera_path(const DevCamera& cam, PathSoA dst, uint32_t k, uint64_t pid,
+                                                  const CameraPath& c) {
     dst.o4[k] = make_float4(cam.eye[0], cam.eye[1], cam.eye[2], 0.f);
-    dst.d4[k] = make_float4(d.x, d.y, d.z, __uint_as_float(kSpecularFlag));
+    dst.d4[k] = make_float4(c.d.x, c.d.y, c.d.z, __uint_as_float(kSpecularFlag));
     dst.b4[k] = make_float4(1.f, 1.f, 1.f, __uint_as_float((uint32_t)pid));
-    dst.rng[k] = rng.state;
+    dst.rng[k] = c.rng;
+}
+__device__ __forceinline__ void generate_camera_path(const DevCamera& cam, const PathParams& pp, PathSoA dst,
+                                                     uint32_t k, uint64_t pid) {
+    store_camera_path(cam, dst, k, pid, camera_path(cam, pp, pid));
 }
 
 __device__ __forceinline__ void generate_ray_path(const kz_ray* __restrict__ rays, const PathParams& pp, PathSoA dst,

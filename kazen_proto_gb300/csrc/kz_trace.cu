@@ -170,6 +170,51 @@ __global__ void __launch_bounds__(256, KZ_TRACE_MINB) k_trace_paths_persistent(D
     if (kCount) warp_count(dn, dt, &ctr->fetch[0]);
 }
 
+// The new camera paths of an iteration: each warp takes 32 consecutive ones,
+// generates them and traces them as a bundle; one that reaches over the end of
+// an image row is traced as a bundle per row (as one it would be as wide as
+// the image).
+constexpr int kBundleWarps = 4;  // per block
+__global__ void __launch_bounds__(32 * kBundleWarps, 8)
+    k_camera_bundles(DevScene s, DevCamera cam, PathParams pp, PathSoA p, IterSlots it) {
+    __shared__ uint2 stacks[kBundleWarps][kWarpStack];
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    const NewPaths nw = new_paths(it, blockIdx.x * blockDim.x + threadIdx.x);
+    const uint32_t skip = (uint32_t)nw.first & 31u;  // bundles start at multiples of 32 path ids
+    for (;;) {
+        uint32_t j = 0;
+        if (lane == 0) j = atomicAdd(&it.cur->camera_next, 32u);
+        j = __shfl_sync(0xFFFFFFFFu, j, 0);
+        if (j >= nw.count + skip) break;
+        const bool live = j + lane >= skip && j + lane < nw.count + skip;
+        const uint32_t i = live ? j + lane - skip : 0u, k = nw.slot + i;
+        const uint64_t pid = nw.first + i;
+        const CameraPath c = camera_path(cam, pp, pid);
+        if (live) store_camera_path(cam, p, k, pid, c);
+        const uint32_t row = live ? (uint32_t)(pid / pp.spp / cam.W) : 0xFFFFFFFFu;
+        HitRec h{__int_as_float(0x7f800000), 0.f, 0.f, KZ_INVALID_ID, -1};
+        for (uint32_t todo = __ballot_sync(0xFFFFFFFFu, live); todo;) {
+            const uint32_t lead = __ffs(todo) - 1;
+            const bool mine = row == __shfl_sync(0xFFFFFFFFu, row, lead);
+            todo &= ~__ballot_sync(0xFFFFFFFFu, mine);
+            const f3 d = mk(__shfl_sync(0xFFFFFFFFu, c.d.x, lead), __shfl_sync(0xFFFFFFFFu, c.d.y, lead),
+                            __shfl_sync(0xFFFFFFFFu, c.d.z, lead));
+            const TRay r = make_tray(ld3(cam.eye), mine ? c.d : d, kRayEps);
+            WarpRay w;
+            bool aborted;
+            if (warp_bundle(s, r, mine, stacks[warp], w, aborted)) {
+                if (mine && !aborted && w.rec >= 0) h = HitRec{w.t, w.V / w.det, w.W / w.det, w.prim, w.rec};
+            } else if (mine) {
+                uint32_t dn = 0, dt = 0;
+                aborted = !trace_closest<false>(s, r, __int_as_float(0x7f800000), h, dn, dt);
+            }
+            if (mine && aborted) set_status(&it.cur->status, KZ_ERR_STACK);
+            __syncwarp();
+        }
+        if (live) p.hit[k] = make_float4(h.t, h.u, h.v, __int_as_float(h.rec));
+    }
+}
+
 // An iteration's closest hits and the shadow rays of the iteration before,
 // which depend on nothing of this one, in one launch: a warp that finds no
 // path left goes on to the shadow rays, so that one tail of long rays is
@@ -317,6 +362,13 @@ void launch_trace_paths(const DevScene& s, PathSoA p, uint32_t n, DevCounters* c
     if (!n) return;
     if (count) k_trace_paths<true><<<grid_for(n, block), block, 0, st>>>(s, p, n, ctr, nullptr);
     else k_trace_paths<false><<<grid_for(n, block), block, 0, st>>>(s, p, n, ctr, nullptr);
+}
+
+void launch_camera_bundles(const DevScene& s, const DevCamera& cam, const PathParams& pp, PathSoA p,
+                           const IterSlots& it, cudaStream_t st) {
+    if (!it.cap) return;
+    static const unsigned g = resident_grid(k_camera_bundles, 32 * kBundleWarps);
+    k_camera_bundles<<<std::min(g, grid_for(it.cap, 32 * kBundleWarps)), 32 * kBundleWarps, 0, st>>>(s, cam, pp, p, it);
 }
 
 void launch_trace_paths_dev(const DevScene& s, PathSoA p, uint32_t cap, const uint32_t* n_active, DevCounters* ctr,
