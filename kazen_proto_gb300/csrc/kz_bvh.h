@@ -70,15 +70,18 @@ struct WideBvhOutput {
 // relative SAH weights of a wide-node visit and of one triangle test
 // (KZ_BVH_TRI_COST).
 // Relative cost of one triangle test against a wide-node visit in the SAH
-// collapse. With the leaf tests shared by the warp (32 pairs per round), a
-// triangle is cheap next to an eight-slot node test: on the terrain frame
-// (1080p, 64 spp) the frame rate for 2.0 / 1.0 / 0.5 / 0.35 / 0.25 / 0.15
-// was 1,665 / 1,690 / 1,732 / 1,744 / 1,747 / 1,743 Mpaths*bounces/s.
+// collapse. With several nodes visited between two leaf rounds, and a round
+// cut into as many warp-wide steps as its pairs need, a triangle costs about
+// half a node. Over 0.10 / 0.15 / 0.25 / 0.40 / 0.50 / 0.65 / 0.80: 2^24
+// incoherent closest hits 8.63 / 8.58 / 8.38 / 8.26 / 8.24 / 8.25 / 8.26 ms,
+// any hits 5.51 / 5.48 / 5.34 / 5.26 / 5.25 / 5.28 / 5.31 ms, the terrain
+// frame (1080p, 64 spp) 116.1 / 115.7 / 115.0 / 114.2 / 113.9 / 113.9 / 114.0
+// ms. Hits do not depend on the tree: equal t goes to the smaller id.
 #ifndef KZ_BVH_BIN_LEAF
 #define KZ_BVH_BIN_LEAF 1
 #endif
 #ifndef KZ_BVH_TRI_COST
-#define KZ_BVH_TRI_COST 0.25f
+#define KZ_BVH_TRI_COST 0.5f
 #endif
 struct WideBuildOptions {
     bool sah_collapse = true;

@@ -462,8 +462,9 @@ __device__ bool trace_any(const DevScene& s, const TRay& r, float tmax, bool& ov
 // few visits more than it saves only from four on. Trace + shadow stages of
 // the terrain frame at 1 / 2 / 3 / 4 nodes a step: 132.6 / 105.0 / 102.2 /
 // 104.5 ms (135.7 before, with decoded slots and a searched pair list); any hit
-// on 2^24 incoherent rays at 2 / 3: 5.23 / 5.52 ms (6.31 before), closest hit
-// 8.63 at both (11.19 before).
+// on 2^24 incoherent rays at 2 / 3 now: 5.44 / 5.34 ms, the terrain frame's
+// shadow launches 22.75 / 22.09 ms; closest hit at 2 / 3 / 4: 8.55 / 8.39 /
+// 8.94 ms.
 //
 // Each lane publishes its ray (TriRay) in shared memory when it starts one.
 // The closest hit is exact and independent of which lane tested what:
@@ -475,7 +476,7 @@ __device__ bool trace_any(const DevScene& s, const TRay& r, float tmax, bool& ov
 #define KZ_CLOSEST_STEPS 3
 #endif
 #ifndef KZ_ANY_STEPS
-#define KZ_ANY_STEPS 2
+#define KZ_ANY_STEPS 3
 #endif
 constexpr int kClosestSteps = KZ_CLOSEST_STEPS, kAnySteps = KZ_ANY_STEPS;
 
