@@ -107,13 +107,13 @@ __device__ __forceinline__ void feature_afrag(uint32_t (&a)[4][4], f3 p0, f3 n0,
 }
 
 // Stage the BF16 weights into shared memory: W1..W3 [64][72], W4 [40][72]
-// and, when `transposed`, W2^T, W3^T [64][72] and W4^T [64][56].
+// and W2^T, W3^T [64][72] and W4^T [64][56].
 struct SmemW {
     __nv_bfloat16* w[4];
     __nv_bfloat16* wt[4];  // wt[1..3] used
 };
 
-__device__ void stage_weights(const __nv_bfloat16* __restrict__ Wg, __nv_bfloat16* smem, bool transposed, SmemW& s) {
+__device__ void stage_weights(const __nv_bfloat16* __restrict__ Wg, __nv_bfloat16* smem, SmemW& s) {
     s.w[0] = smem;
     s.w[1] = s.w[0] + 64 * kStrideW;
     s.w[2] = s.w[1] + 64 * kStrideW;
@@ -129,20 +129,18 @@ __device__ void stage_weights(const __nv_bfloat16* __restrict__ Wg, __nv_bfloat1
             const int o = i >> 6, k = i & 63;
             const __nv_bfloat16 v = Wg[offs[l] + i];
             s.w[l][o * kStrideW + k] = v;
-            if (transposed && l >= 1) {
+            if (l >= 1) {
                 if (l < 3) s.wt[l][k * kStrideW + o] = v;
                 else s.wt[3][k * kStrideW4T + o] = v;
             }
         }
-    if (transposed)
-        for (int i = threadIdx.x; i < 64 * 8; i += blockDim.x)  // W4^T columns 40..47 = 0
-            s.wt[3][(i >> 3) * kStrideW4T + 40 + (i & 7)] = __float2bfloat16_rn(0.f);
+    for (int i = threadIdx.x; i < 64 * 8; i += blockDim.x)  // W4^T columns 40..47 = 0
+        s.wt[3][(i >> 3) * kStrideW4T + 40 + (i & 7)] = __float2bfloat16_rn(0.f);
     __syncthreads();
 }
 
-constexpr size_t kSmemInfer = (size_t)(64 * 3 + 40) * kStrideW * 2;
-constexpr uint32_t kInferCtasPerSm = 6;  // 33 KB of weights each: six fit in shared memory
-constexpr size_t kSmemTrainW = kSmemInfer + (size_t)(64 * 2) * kStrideW * 2 + (size_t)64 * kStrideW4T * 2;
+constexpr size_t kSmemForward = (size_t)(64 * 3 + 40) * kStrideW * 2;
+constexpr size_t kSmemTrainW = kSmemForward + (size_t)(64 * 2) * kStrideW * 2 + (size_t)64 * kStrideW4T * 2;
 constexpr int kTrainWarps = 4;
 constexpr size_t kSmemTrain = kSmemTrainW + (size_t)kTrainWarps * 16 * 41 * 4;
 
@@ -161,78 +159,167 @@ __device__ __forceinline__ void forward_tile(const SmemW& s, const float* __rest
 }
 
 // ------------------------------------------------------------------ inference
+// A warp takes 32 rows, two 16-row tiles that share every weight fragment it
+// reads; the weights lie in shared memory in the order the lanes use them, 16
+// bytes for the two k-tiles of an 8-column block, so the 29 KB of fragments
+// are read once for 32 rows instead of twice, in a quarter as many loads. A
+// CTA's weights are copied as whole words: as single BF16 values the copy alone
+// took some 40 us a launch. Bound by the issue rate of products, conversions
+// and loads. Ten iterations of a 512 x 512 guided frame, 8 spp: 1.23 -> 0.71
+// ms (the first, 2.1M rows: 276 -> 187 us; the last: 52 -> 18 us); two, three
+// or four CTAs per SM are the same. The products of a row keep their order:
+// the outputs are the same bits.
+constexpr int kInferFrags = (8 * 3 + 5) * 2 * 32;  // uint4: 8-column block, pair of k-tiles, lane
+constexpr int kInferBias = 64 * 3 + 40;
+constexpr size_t kSmemInfer = (size_t)kInferFrags * 16 + kInferBias * 4;
+
+// Block b (8 columns of a layer): 0..23 the hidden layers, 24..28 the outputs.
+__device__ __forceinline__ void stage_fragments(const GuideDev& gd, uint4* frag, float* bias) {
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(gd.wbf);
+#pragma unroll 5
+    for (int i = threadIdx.x; i < kInferFrags; i += 128) {
+        const int b = i >> 6, q = (i >> 5) & 1, g = (i >> 2) & 7, t = i & 3;
+        const int layer = b >> 3;
+        const int off = layer == 0 ? kOffW1 : layer == 1 ? kOffW2 : layer == 2 ? kOffW3 : kOffW4;
+        const uint32_t* p = w + (off + (8 * (b & 7) + g) * 64 + 32 * q + 2 * t) / 2;
+        frag[i] = make_uint4(__ldg(p), __ldg(p + 4), __ldg(p + 8), __ldg(p + 12));
+    }
+    for (int i = threadIdx.x; i < kInferBias; i += 128) {
+        const int layer = i >> 6;
+        const int off = layer == 0 ? kOffB1 : layer == 1 ? kOffB2 : layer == 2 ? kOffB3 : kOffB4;
+        bias[i] = __ldg(gd.wf + off + (i & 63));
+    }
+    __syncthreads();
+}
+
+// warp_layer over two 16-row tiles, from fragments; the products of an
+// accumulator in the same order.
+template <int NT>
+__device__ __forceinline__ void infer_layer(float (&acc)[2][NT][4], const uint32_t (&a)[2][4][4], const uint4* frag,
+                                            const float* bias, int lane) {
+    const int t = lane & 3;
+#pragma unroll
+    for (int j = 0; j < NT; ++j) {
+        const float2 b = *reinterpret_cast<const float2*>(bias + 8 * j + 2 * t);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            acc[h][j][0] = acc[h][j][2] = b.x;
+            acc[h][j][1] = acc[h][j][3] = b.y;
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+#pragma unroll
+        for (int j = 0; j < NT; ++j) {
+            const uint4 w = frag[(2 * j + q) * 32 + lane];
+            mma16816(acc[0][j], a[0][2 * q], w.x, w.y);
+            mma16816(acc[1][j], a[1][2 * q], w.x, w.y);
+            mma16816(acc[0][j], a[0][2 * q + 1], w.z, w.w);
+            mma16816(acc[1][j], a[1][2 * q + 1], w.z, w.w);
+        }
+}
+
 // rows = points: pts[2i] = (p01.xyz, -), pts[2i+1] = (n.xyz, -); or, in path
 // mode, the hit of path i (position and geometric normal from the triangle
 // record). raw[i*40 ..] = network outputs.
 template <bool kPaths>
-__global__ void __launch_bounds__(128) k_guide_infer(DevScene sc, PathSoA ps, const float4* __restrict__ pts,
-                                                     uint32_t n, GuideDev gd, float* __restrict__ raw,
-                                                     const uint32_t* n_dev) {
+__global__ void __launch_bounds__(128, 3)
+    k_guide_infer(DevScene sc, PathSoA ps, const float4* __restrict__ pts, uint32_t n, GuideDev gd,
+                  float* __restrict__ raw, const uint32_t* n_dev) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     if (n_dev) n = *n_dev;
-    if ((n + 15) / 16 <= blockIdx.x * (blockDim.x >> 5)) return;  // no tile for this CTA
-    SmemW s;
-    stage_weights(gd.wbf, reinterpret_cast<__nv_bfloat16*>(smem_raw), false, s);
+    const uint32_t tiles = n / 32 + (n % 32 != 0), tstride = gridDim.x * 4u;
+    if (tiles <= blockIdx.x * 4u) return;  // no tile for this CTA
+    uint4* frag = reinterpret_cast<uint4*>(smem_raw);
+    float* bias = reinterpret_cast<float*>(frag + kInferFrags);
+    stage_fragments(gd, frag, bias);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane >> 2, t = lane & 3;
-    const uint32_t tiles = (n + 15) / 16;
-    const uint32_t tstride = gridDim.x * (blockDim.x >> 5);
-    // the hit records of the warp's next tile are loaded one tile ahead, so
-    // the triangle fetch that depends on them waits on one load, not two
-    float4 hit_next[2];
-    const uint32_t tile0 = blockIdx.x * (blockDim.x >> 5) + warp;
-    if (kPaths)
-        for (int h = 0; h < 2; ++h) {
-            const uint32_t r = tile0 * 16 + g + 8 * h;
-            hit_next[h] = r < n ? ps.hit[r] : make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
-        }
+    // a lane loads the row of its own number and hands it to the four lanes
+    // that build its features; the hit of its next row is loaded one tile
+    // ahead, so the triangle fetch that depends on it waits on one load
+    const auto hit_of = [&](uint32_t tile) {
+        const uint32_t r = tile * 32 + lane;
+        return kPaths && tile < tiles && r < n ? ps.hit[r] : make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
+    };
+    const uint32_t tile0 = blockIdx.x * 4u + warp;
+    float4 next = hit_of(tile0);
     for (uint32_t tile = tile0; tile < tiles; tile += tstride) {
-        f3 p[2], nn[2];
-        float4 hit_cur[2];
-        if (kPaths)
-            for (int h = 0; h < 2; ++h) {
-                hit_cur[h] = hit_next[h];
-                const uint32_t r = (tile + tstride) * 16 + g + 8 * h;
-                hit_next[h] = tile + tstride < tiles && r < n ? ps.hit[r] : make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
-            }
-        for (int h = 0; h < 2; ++h) {
-            const uint32_t r = tile * 16 + g + 8 * h;
-            p[h] = mk(0.5f, 0.5f, 0.5f);
-            nn[h] = mk(0.f, 1.f, 0.f);
-            if (r < n) {
-                if (kPaths) {
-                    const float4 hit = hit_cur[h];
-                    const int rec = __float_as_int(hit.w);
-                    if (rec >= 0) {
-                        const float4 o4 = ps.o4[r], d4 = ps.d4[r];
-                        const float4* tp = sc.tris + (size_t)rec * 3;
-                        const float4 ta = __ldg(tp), tb = __ldg(tp + 1), tc = __ldg(tp + 2);
-                        const f3 v0 = mk(ta.x, ta.y, ta.z), v1 = mk(tb.x, tb.y, tb.z), v2 = mk(tc.x, tc.y, tc.z);
-                        nn[h] = normalize(cross(v1 - v0, v2 - v0));
-                        const f3 P = mk(o4.x, o4.y, o4.z) + mk(d4.x, d4.y, d4.z) * hit.x;
-                        p[h] = hmul(P - mk(gd.box_lo.x, gd.box_lo.y, gd.box_lo.z),
-                                    mk(gd.box_inv.x, gd.box_inv.y, gd.box_inv.z));
-                    }
-                } else {
-                    const float4 a = pts[2 * (size_t)r], b = pts[2 * (size_t)r + 1];
-                    p[h] = mk(a.x, a.y, a.z);
-                    nn[h] = mk(b.x, b.y, b.z);
+        const uint32_t mine = tile * 32 + lane;
+        const float4 hit = next;
+        next = hit_of(tile + tstride);
+        f3 p = mk(0.5f, 0.5f, 0.5f), nn = mk(0.f, 1.f, 0.f);
+        if (mine < n) {
+            if (kPaths) {
+                const int rec = __float_as_int(hit.w);
+                if (rec >= 0) {
+                    const float4 o4 = ps.o4[mine], d4 = ps.d4[mine];
+                    const float4* tp = sc.tris + (size_t)rec * 3;
+                    const float4 ta = __ldg(tp), tb = __ldg(tp + 1), tc = __ldg(tp + 2);
+                    const f3 v0 = mk(ta.x, ta.y, ta.z), v1 = mk(tb.x, tb.y, tb.z), v2 = mk(tc.x, tc.y, tc.z);
+                    nn = normalize(cross(v1 - v0, v2 - v0));
+                    const f3 P = mk(o4.x, o4.y, o4.z) + mk(d4.x, d4.y, d4.z) * hit.x;
+                    p = hmul(P - mk(gd.box_lo.x, gd.box_lo.y, gd.box_lo.z),
+                             mk(gd.box_inv.x, gd.box_inv.y, gd.box_inv.z));
                 }
+            } else {
+                const float4 a = pts[2 * (size_t)mine], b = pts[2 * (size_t)mine + 1];
+                p = mk(a.x, a.y, a.z);
+                nn = mk(b.x, b.y, b.z);
             }
         }
-        uint32_t x[4][4], a1[4][4], a2[4][4], a3[4][4];
-        float h1[8][4], h2[8][4], h3[8][4], o[5][4];
-        feature_afrag(x, p[0], nn[0], p[1], nn[1], gd.band_scale, lane);
-        forward_tile(s, gd.wf, x, h1, h2, h3, o, a1, a2, a3, lane);
-        for (int h = 0; h < 2; ++h) {
-            const uint32_t r = tile * 16 + g + 8 * h;
+        const auto row_of = [&](f3 v, int r) {
+            return mk(__shfl_sync(0xFFFFFFFFu, v.x, r), __shfl_sync(0xFFFFFFFFu, v.y, r),
+                      __shfl_sync(0xFFFFFFFFu, v.z, r));
+        };
+        uint32_t a[2][4][4];
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+            feature_afrag(a[h], row_of(p, 16 * h + g), row_of(nn, 16 * h + g), row_of(p, 16 * h + g + 8),
+                          row_of(nn, 16 * h + g + 8), gd.band_scale, lane);
+#pragma unroll
+        for (int l = 0; l < 3; ++l) {
+            float c[2][8][4];
+            infer_layer<8>(c, a, frag + l * 512, bias + l * 64, lane);
+            to_afrag<8>(c[0], a[0], true);
+            to_afrag<8>(c[1], a[1], true);
+        }
+        float o[2][5][4];
+        infer_layer<5>(o, a, frag + 3 * 512, bias + 3 * 64, lane);
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+            const uint32_t r = tile * 32 + g + 8 * h;
             if (r >= n) continue;
 #pragma unroll
             for (int j = 0; j < 5; ++j)
                 *reinterpret_cast<float2*>(raw + (size_t)r * kGuideOut + 8 * j + 2 * t) =
-                    make_float2(o[j][2 * h], o[j][2 * h + 1]);
+                    make_float2(o[h >> 1][j][2 * (h & 1)], o[h >> 1][j][2 * (h & 1) + 1]);
         }
     }
+}
+
+int sm_count() {
+    static int n = 0;
+    if (!n) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        if (n <= 0) n = 1;
+    }
+    return n;
+}
+
+// Each CTA fills its 128 threads with rows before another one is used.
+template <bool kPaths>
+uint32_t infer_grid(uint32_t n) {
+    static const uint32_t resident = [] {
+        int per_sm = 1;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_guide_infer<kPaths>, 128, kSmemInfer) !=
+                cudaSuccess || per_sm < 1)
+            per_sm = 1;
+        return (uint32_t)(per_sm * sm_count());
+    }();
+    return min(n / 128 + 1, resident);
 }
 
 // ------------------------------------------------------------------ training: forward + loss + backward (data)
@@ -247,7 +334,7 @@ __global__ void __launch_bounds__(kTrainWarps * 32) k_guide_train_fb(const float
                                                                      float* __restrict__ loss) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     SmemW s;
-    stage_weights(gd.wbf, reinterpret_cast<__nv_bfloat16*>(smem_raw), true, s);
+    stage_weights(gd.wbf, reinterpret_cast<__nv_bfloat16*>(smem_raw), s);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane >> 2, t = lane & 3;
     float* so = reinterpret_cast<float*>(smem_raw + kSmemTrainW) + warp * 16 * 41;
@@ -475,17 +562,6 @@ __global__ void k_guide_to_bf16(const float* __restrict__ w, __nv_bfloat16* __re
     if (i < n) wbf[i] = __float2bfloat16_rn(w[i]);
 }
 
-int sm_count() {
-    static int n = 0;
-    if (!n) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        if (n <= 0) n = 1;
-    }
-    return n;
-}
-
 }  // namespace
 
 cudaError_t guide_kernel_setup() {
@@ -505,18 +581,14 @@ cudaError_t guide_kernel_setup() {
 void launch_guide_infer_paths_dev(const DevScene& s, PathSoA p, uint32_t cap, const uint32_t* n_active,
                                   const GuideDev& gd, float* raw, cudaStream_t st) {
     if (!cap) return;
-    const uint32_t tiles = (cap + 15) / 16;
-    const uint32_t grid = min((tiles + 3) / 4, (uint32_t)sm_count() * kInferCtasPerSm);
-    k_guide_infer<true><<<grid, 128, kSmemInfer, st>>>(s, p, nullptr, cap, gd, raw, n_active);
+    k_guide_infer<true><<<infer_grid<true>(cap), 128, kSmemInfer, st>>>(s, p, nullptr, cap, gd, raw, n_active);
 }
 
 void launch_guide_infer_points(const float4* pts, uint32_t n, const GuideDev& gd, float* raw, cudaStream_t st) {
     if (!n) return;
     DevScene none;
     PathSoA np{};
-    const uint32_t tiles = (n + 15) / 16;
-    const uint32_t grid = min((tiles + 3) / 4, (uint32_t)sm_count() * kInferCtasPerSm);
-    k_guide_infer<false><<<grid, 128, kSmemInfer, st>>>(none, np, pts, n, gd, raw, nullptr);
+    k_guide_infer<false><<<infer_grid<false>(n), 128, kSmemInfer, st>>>(none, np, pts, n, gd, raw, nullptr);
 }
 
 int guide_train_mode() {
