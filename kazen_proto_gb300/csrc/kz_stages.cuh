@@ -1066,8 +1066,8 @@ __global__ void __launch_bounds__(256, kGuided ? KZ_SHADE_GUIDED_MIN_BLOCKS : KZ
 // makes ten times slower than the rest. Both wait on dependent loads; the
 // plain pass moves about 230 bytes a path, the heavy one is left with the lobe
 // switch and FP64. Shade stage, one kernel before / two: terrain 1080p 30.8 /
-// 23.6 ms (11.7 of it plain), slit room 12.1 / 6.9 ms, 641 x 359 frame of
-// mixed materials 16.3 / 3.0 ms, box room 0.59 / 0.45 ms.
+// 18.8 ms, slit room 12.1 / 6.2 ms, 641 x 359 frame of mixed materials 16.3 /
+// 2.8 ms, box room 0.59 / 0.36 ms.
 // Blocks per SM, terrain + materials shade: plain (256 threads) 4 / 5 / 6 / 8:
 // 27.5 / 27.6 / 28.1 / 32.8 ms; heavy (128 threads) 4 / 6 / 8 / 12: 27.8 /
 // 27.6 / 27.4 / 28.3 ms.
@@ -1078,6 +1078,17 @@ __global__ void __launch_bounds__(256, kGuided ? KZ_SHADE_GUIDED_MIN_BLOCKS : KZ
 #define KZ_HEAVY_MIN_BLOCKS 8
 #endif
 constexpr int kHeavyThreads = 128;
+// Paths a thread classifies between two rounds of shading. The plain ones are
+// listed per block and shaded 256 at a time: where most bounces leave the scene,
+// ten of 32 lanes were active otherwise. Two independent hit -> triangle ->
+// class chains a thread also hide half of their waits. Shade stage, a path per
+// lane / 2 / 4 / 8 a thread with the list: terrain 22.7 / 18.8 / 18.9 / 19.4 ms,
+// slit room 6.47 / 6.21 / 6.21 / 6.41, mixed materials 2.92 / 2.82 / 2.84 / 2.92.
+#ifndef KZ_PLAIN_CHUNK
+#define KZ_PLAIN_CHUNK 2
+#endif
+constexpr uint32_t kPlainChunk = KZ_PLAIN_CHUNK;
+static_assert(kPlainChunk * 32u <= 256u, "ranks within a warp are kept in a byte");
 
 // Queue place of the k-th path of a heavy class: two arrays of the wavefront's
 // capacity, each filled from both ends (a path is in one class only).
@@ -1091,40 +1102,55 @@ __global__ void __launch_bounds__(256, KZ_PLAIN_MIN_BLOCKS)
     k_shade_plain(DevScene scene, PathParams params, const DevJob* __restrict__ jobs, PathSoA in, PathSoA out,
                   ShadowSoA sq, HeavyQueue hq, DevCounters* ctr, const uint32_t* n_active, float* film,
                   double* film64) {
-    // per warp: appended paths and shadow rays, then the four heavy classes; double buffered over the rounds
-    __shared__ unsigned long long s_app[2][8];
-    __shared__ uint32_t s_heavy[2][kHeavyClasses][8];
+    __shared__ uint32_t s_list[256 * (kPlainChunk + 1)];  // plain paths found and not yet shaded
+    __shared__ uint32_t s_heavy[kHeavyClasses][8], s_plain[9];
+    __shared__ unsigned long long s_app[2][8];  // per warp: appended paths and shadow rays; double buffered
     const uint32_t n = *n_active, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, lt = (1u << lane) - 1u;
-    uint32_t buf = 0;
-    for (uint32_t base = blockIdx.x * 256u; base < n; base += gridDim.x * 256u, buf ^= 1u) {
-        const uint32_t i = base + threadIdx.x;
-        ShadeOut so;
-        uint32_t heavy = kHeavyClasses;  // none
-        if (i < n) {
-            const float4 hit = in.hit[i], d4 = in.d4[i];
-            const DevJob* J = kJobs ? jobs + (__float_as_uint(d4.w) >> kJobShift) : nullptr;
-            const DevScene& s = kJobs ? J->scene : scene;
-            const PathParams& pp = kJobs ? J->pp : params;
-            const uint32_t kind = shade_kind(s, hit);
-            if (kind == 1u + kPlainClass) shade_plain<kAttr>(s, pp, hit, in.o4[i], d4, in.b4[i], in.rng[i], so);
-            else if (kind) heavy = kind - 2u;
-            else if (s.has_env) shade_miss(s, pp, d4, in.b4[i], so);
-            if (!is_zero(so.Lsum)) film_add(kJobs ? J->film : film, kJobs ? nullptr : film64, so.film_idx, so.Lsum);
-        }
-        // one atomic per queue and block, not per warp
-        const uint32_t bc = __ballot_sync(0xFFFFFFFFu, so.cont), bs = __ballot_sync(0xFFFFFFFFu, so.shadow);
-        uint32_t bh = 0;  // this lane's class among the warp's
+    // every block has paths before one takes several per thread
+    const uint32_t per = min((uint32_t)kPlainChunk, n / (gridDim.x * 256u) + 1u);
+    uint32_t found = 0, buf = 0;  // the list's length, the same in every thread
+    for (uint32_t base = blockIdx.x * 256u * per; base < n; base += gridDim.x * 256u * per) {
+        // ---- classify: misses are finished, the others listed or queued
+        uint32_t mark[kPlainChunk];  // class << 8 | rank among the warp's; class 0 plain, c + 1 heavy c
+        uint32_t cnt[1 + kHeavyClasses] = {};
 #pragma unroll
-        for (uint32_t c = 0; c < kHeavyClasses; ++c) {
-            const uint32_t b = __ballot_sync(0xFFFFFFFFu, heavy == c);
-            if (heavy == c) bh = b;
-            if (lane == 0) s_heavy[buf][c][warp] = __popc(b);
+        for (uint32_t k = 0; k < kPlainChunk; ++k) {
+            const uint32_t i = base + k * 256u + threadIdx.x;
+            mark[k] = ~0u;
+            if (k >= per) continue;  // uniform over the block
+            uint32_t cls = ~0u;
+            if (i < n) {
+                const float4 hit = in.hit[i];
+                const DevJob* J = kJobs ? jobs + (__float_as_uint(in.d4[i].w) >> kJobShift) : nullptr;
+                const DevScene& s = kJobs ? J->scene : scene;
+                const uint32_t kind = shade_kind(s, hit);
+                if (kind) {
+                    cls = kind - 1u;  // kPlainClass is 0
+                } else if (s.has_env) {
+                    ShadeOut so;
+                    shade_miss(s, kJobs ? J->pp : params, in.d4[i], in.b4[i], so);
+                    if (!is_zero(so.Lsum))
+                        film_add(kJobs ? J->film : film, kJobs ? nullptr : film64, so.film_idx, so.Lsum);
+                }
+            }
+            const uint32_t classes = __any_sync(0xFFFFFFFFu, cls != ~0u && cls) ? 1u + kHeavyClasses : 1u;
+#pragma unroll
+            for (uint32_t c = 0; c < 1u + kHeavyClasses; ++c) {
+                if (c >= classes) break;
+                const uint32_t m = __ballot_sync(0xFFFFFFFFu, cls == c);
+                if (cls == c) mark[k] = c << 8 | (cnt[c] + __popc(m & lt));
+                cnt[c] += __popc(m);
+            }
         }
-        if (lane == 0) s_app[buf][warp] = ((unsigned long long)__popc(bs) << 32) | (unsigned)__popc(bc);
+        if (lane == 0) {
+            s_plain[warp] = cnt[0];
+#pragma unroll
+            for (uint32_t c = 0; c < kHeavyClasses; ++c) s_heavy[c][warp] = cnt[1 + c];
+        }
         __syncthreads();
-        if (warp == 0) {  // lanes 8 c + w: warp w of class c
+        if (warp == 0) {  // lanes 8 c + w: warp w of class c; one atomic per class and block
             const uint32_t c = lane >> 3, w = lane & 7u;
-            const uint32_t v = s_heavy[buf][c][w];
+            const uint32_t v = s_heavy[c][w];
             uint32_t incl = v;
 #pragma unroll
             for (uint32_t o = 1; o < 8; o <<= 1) {
@@ -1133,22 +1159,63 @@ __global__ void __launch_bounds__(256, KZ_PLAIN_MIN_BLOCKS)
             }
             uint32_t first = 0;
             if (w == 7 && incl) first = atomicAdd(&ctr->heavy[c], incl);
-            s_heavy[buf][c][w] = __shfl_sync(0xFFFFFFFFu, first, 7, 8) + incl - v;
+            s_heavy[c][w] = __shfl_sync(0xFFFFFFFFu, first, 7, 8) + incl - v;
         } else if (warp == 1 && lane < 8) {
-            const unsigned long long v = s_app[buf][lane];
-            unsigned long long incl = v, first = 0;
+            const uint32_t v = s_plain[lane];
+            uint32_t incl = v;
 #pragma unroll
             for (uint32_t o = 1; o < 8; o <<= 1) {
-                const unsigned long long x = __shfl_up_sync(0xFFu, incl, o);
+                const uint32_t x = __shfl_up_sync(0xFFu, incl, o);
                 if (lane >= o) incl += x;
             }
-            if (lane == 7 && incl) first = atomicAdd(&ctr->n_append, incl);
-            s_app[buf][lane] = __shfl_sync(0xFFu, first, 7) + incl - v;
+            s_plain[lane] = found + incl - v;
+            if (lane == 7) s_plain[8] = found + incl;
         }
         __syncthreads();
-        const unsigned long long at = s_app[buf][warp];
-        store_next(out, sq, so, AppendSlots{(uint32_t)at + __popc(bc & lt), (uint32_t)(at >> 32) + __popc(bs & lt)});
-        if (heavy < kHeavyClasses) *heavy_slot(hq, heavy, s_heavy[buf][heavy][warp] + __popc(bh & lt)) = i;
+#pragma unroll
+        for (uint32_t k = 0; k < kPlainChunk; ++k) {
+            if (mark[k] == ~0u) continue;
+            const uint32_t i = base + k * 256u + threadIdx.x, c = mark[k] >> 8, r = mark[k] & 0xFFu;
+            if (c == 0) s_list[s_plain[warp] + r] = i;
+            else *heavy_slot(hq, c - 1u, s_heavy[c - 1u][warp] + r) = i;
+        }
+        found = s_plain[8];
+        __syncthreads();
+        // ---- shade full blocks of plain paths; what is left once no path follows
+        const bool last = n - base <= gridDim.x * 256u * per;
+        for (; found >= 256u || (last && found); buf ^= 1u) {
+            const uint32_t take = min(found, 256u);
+            found -= take;
+            ShadeOut so;
+            if (threadIdx.x < take) {
+                const uint32_t i = s_list[found + threadIdx.x];
+                const float4 d4 = in.d4[i];
+                const DevJob* J = kJobs ? jobs + (__float_as_uint(d4.w) >> kJobShift) : nullptr;
+                shade_plain<kAttr>(kJobs ? J->scene : scene, kJobs ? J->pp : params, in.hit[i], in.o4[i], d4, in.b4[i],
+                                   in.rng[i], so);
+                if (!is_zero(so.Lsum))
+                    film_add(kJobs ? J->film : film, kJobs ? nullptr : film64, so.film_idx, so.Lsum);
+            }
+            // one atomic per block, not per warp
+            const uint32_t bc = __ballot_sync(0xFFFFFFFFu, so.cont), bs = __ballot_sync(0xFFFFFFFFu, so.shadow);
+            if (lane == 0) s_app[buf][warp] = ((unsigned long long)__popc(bs) << 32) | (unsigned)__popc(bc);
+            __syncthreads();
+            if (warp == 0 && lane < 8) {
+                const unsigned long long v = s_app[buf][lane];
+                unsigned long long incl = v, first = 0;
+#pragma unroll
+                for (uint32_t o = 1; o < 8; o <<= 1) {
+                    const unsigned long long x = __shfl_up_sync(0xFFu, incl, o);
+                    if (lane >= o) incl += x;
+                }
+                if (lane == 7 && incl) first = atomicAdd(&ctr->n_append, incl);
+                s_app[buf][lane] = __shfl_sync(0xFFu, first, 7) + incl - v;
+            }
+            __syncthreads();
+            const unsigned long long at = s_app[buf][warp];
+            store_next(out, sq, so, AppendSlots{(uint32_t)at + __popc(bc & lt), (uint32_t)(at >> 32) + __popc(bs & lt)});
+        }
+        if (last) break;
     }
 }
 
