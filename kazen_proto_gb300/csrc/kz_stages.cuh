@@ -1097,11 +1097,10 @@ __device__ __forceinline__ uint32_t* heavy_slot(const HeavyQueue& q, uint32_t cl
     return (cls & 1u) ? a + (q.cap - 1u - k) : a + k;
 }
 
-template <bool kAttr, bool kJobs>
+template <bool kAttr>
 __global__ void __launch_bounds__(256, KZ_PLAIN_MIN_BLOCKS)
-    k_shade_plain(DevScene scene, PathParams params, const DevJob* __restrict__ jobs, PathSoA in, PathSoA out,
-                  ShadowSoA sq, HeavyQueue hq, DevCounters* ctr, const uint32_t* n_active, float* film,
-                  double* film64) {
+    k_shade_plain(DevScene s, PathParams pp, PathSoA in, PathSoA out, ShadowSoA sq, HeavyQueue hq, DevCounters* ctr,
+                  const uint32_t* n_active, float* film, double* film64) {
     __shared__ uint32_t s_list[256 * (kPlainChunk + 1)];  // plain paths found and not yet shaded
     __shared__ uint32_t s_heavy[kHeavyClasses][8], s_plain[9];
     __shared__ unsigned long long s_app[2][8];  // per warp: appended paths and shadow rays; double buffered
@@ -1120,17 +1119,13 @@ __global__ void __launch_bounds__(256, KZ_PLAIN_MIN_BLOCKS)
             if (k >= per) continue;  // uniform over the block
             uint32_t cls = ~0u;
             if (i < n) {
-                const float4 hit = in.hit[i];
-                const DevJob* J = kJobs ? jobs + (__float_as_uint(in.d4[i].w) >> kJobShift) : nullptr;
-                const DevScene& s = kJobs ? J->scene : scene;
-                const uint32_t kind = shade_kind(s, hit);
+                const uint32_t kind = shade_kind(s, in.hit[i]);
                 if (kind) {
                     cls = kind - 1u;  // kPlainClass is 0
                 } else if (s.has_env) {
                     ShadeOut so;
-                    shade_miss(s, kJobs ? J->pp : params, in.d4[i], in.b4[i], so);
-                    if (!is_zero(so.Lsum))
-                        film_add(kJobs ? J->film : film, kJobs ? nullptr : film64, so.film_idx, so.Lsum);
+                    shade_miss(s, pp, in.d4[i], in.b4[i], so);
+                    if (!is_zero(so.Lsum)) film_add(film, film64, so.film_idx, so.Lsum);
                 }
             }
             const uint32_t classes = __any_sync(0xFFFFFFFFu, cls != ~0u && cls) ? 1u + kHeavyClasses : 1u;
@@ -1189,12 +1184,8 @@ __global__ void __launch_bounds__(256, KZ_PLAIN_MIN_BLOCKS)
             ShadeOut so;
             if (threadIdx.x < take) {
                 const uint32_t i = s_list[found + threadIdx.x];
-                const float4 d4 = in.d4[i];
-                const DevJob* J = kJobs ? jobs + (__float_as_uint(d4.w) >> kJobShift) : nullptr;
-                shade_plain<kAttr>(kJobs ? J->scene : scene, kJobs ? J->pp : params, in.hit[i], in.o4[i], d4, in.b4[i],
-                                   in.rng[i], so);
-                if (!is_zero(so.Lsum))
-                    film_add(kJobs ? J->film : film, kJobs ? nullptr : film64, so.film_idx, so.Lsum);
+                shade_plain<kAttr>(s, pp, in.hit[i], in.o4[i], in.d4[i], in.b4[i], in.rng[i], so);
+                if (!is_zero(so.Lsum)) film_add(film, film64, so.film_idx, so.Lsum);
             }
             // one atomic per block, not per warp
             const uint32_t bc = __ballot_sync(0xFFFFFFFFu, so.cont), bs = __ballot_sync(0xFFFFFFFFu, so.shadow);
@@ -1216,6 +1207,75 @@ __global__ void __launch_bounds__(256, KZ_PLAIN_MIN_BLOCKS)
             store_next(out, sq, so, AppendSlots{(uint32_t)at + __popc(bc & lt), (uint32_t)(at >> 32) + __popc(bs & lt)});
         }
         if (last) break;
+    }
+}
+
+// The plain pass over jobs of several scenes: a path per lane. Listed, a path
+// would look its job and that job's scene up twice, one dependent load after
+// another: 24 jobs 5.82 ms a path per lane, 5.85 listed; 256 uneven jobs 563 and
+// 565 ms.
+template <bool kAttr>
+__global__ void __launch_bounds__(256, KZ_PLAIN_MIN_BLOCKS)
+    k_shade_plain_jobs(const DevJob* __restrict__ jobs, PathSoA in, PathSoA out, ShadowSoA sq, HeavyQueue hq,
+                       DevCounters* ctr, const uint32_t* n_active) {
+    // per warp: appended paths and shadow rays, then the four heavy classes; double buffered over the rounds
+    __shared__ unsigned long long s_app[2][8];
+    __shared__ uint32_t s_heavy[2][kHeavyClasses][8];
+    const uint32_t n = *n_active, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, lt = (1u << lane) - 1u;
+    uint32_t buf = 0;
+    for (uint32_t base = blockIdx.x * 256u; base < n; base += gridDim.x * 256u, buf ^= 1u) {
+        const uint32_t i = base + threadIdx.x;
+        ShadeOut so;
+        uint32_t heavy = kHeavyClasses;  // none
+        if (i < n) {
+            const float4 hit = in.hit[i], d4 = in.d4[i];
+            const DevJob* J = jobs + (__float_as_uint(d4.w) >> kJobShift);
+            const DevScene& s = J->scene;
+            const PathParams& pp = J->pp;
+            const uint32_t kind = shade_kind(s, hit);
+            if (kind == 1u + kPlainClass) shade_plain<kAttr>(s, pp, hit, in.o4[i], d4, in.b4[i], in.rng[i], so);
+            else if (kind) heavy = kind - 2u;
+            else if (s.has_env) shade_miss(s, pp, d4, in.b4[i], so);
+            if (!is_zero(so.Lsum)) film_add(J->film, nullptr, so.film_idx, so.Lsum);
+        }
+        // one atomic per queue and block, not per warp
+        const uint32_t bc = __ballot_sync(0xFFFFFFFFu, so.cont), bs = __ballot_sync(0xFFFFFFFFu, so.shadow);
+        uint32_t bh = 0;  // this lane's class among the warp's
+#pragma unroll
+        for (uint32_t c = 0; c < kHeavyClasses; ++c) {
+            const uint32_t b = __ballot_sync(0xFFFFFFFFu, heavy == c);
+            if (heavy == c) bh = b;
+            if (lane == 0) s_heavy[buf][c][warp] = __popc(b);
+        }
+        if (lane == 0) s_app[buf][warp] = ((unsigned long long)__popc(bs) << 32) | (unsigned)__popc(bc);
+        __syncthreads();
+        if (warp == 0) {  // lanes 8 c + w: warp w of class c
+            const uint32_t c = lane >> 3, w = lane & 7u;
+            const uint32_t v = s_heavy[buf][c][w];
+            uint32_t incl = v;
+#pragma unroll
+            for (uint32_t o = 1; o < 8; o <<= 1) {
+                const uint32_t x = __shfl_up_sync(0xFFFFFFFFu, incl, o, 8);
+                if (w >= o) incl += x;
+            }
+            uint32_t first = 0;
+            if (w == 7 && incl) first = atomicAdd(&ctr->heavy[c], incl);
+            s_heavy[buf][c][w] = __shfl_sync(0xFFFFFFFFu, first, 7, 8) + incl - v;
+        } else if (warp == 1 && lane < 8) {
+            const unsigned long long v = s_app[buf][lane];
+            unsigned long long incl = v, first = 0;
+#pragma unroll
+            for (uint32_t o = 1; o < 8; o <<= 1) {
+                const unsigned long long x = __shfl_up_sync(0xFFu, incl, o);
+                if (lane >= o) incl += x;
+            }
+            if (lane == 7 && incl) first = atomicAdd(&ctr->n_append, incl);
+            s_app[buf][lane] = __shfl_sync(0xFFu, first, 7) + incl - v;
+        }
+        __syncthreads();
+        const unsigned long long at = s_app[buf][warp];
+        store_next(out, sq, so, AppendSlots{(uint32_t)at + __popc(bc & lt), (uint32_t)(at >> 32) + __popc(bs & lt)});
+        if (heavy < kHeavyClasses) *heavy_slot(hq, heavy, s_heavy[buf][heavy][warp] + __popc(bh & lt)) = i;
     }
 }
 
@@ -1261,8 +1321,11 @@ struct SplitGrids {
 };
 template <bool kAttr, bool kJobs>
 static SplitGrids split_grids() {
-    static const SplitGrids g{resident_grid(k_shade_plain<kAttr, kJobs>, 256),
-                              resident_grid(k_shade_heavy<kAttr, kJobs>, kHeavyThreads)};
+    static const SplitGrids g = [] {
+        const unsigned heavy = resident_grid(k_shade_heavy<kAttr, kJobs>, kHeavyThreads);
+        if constexpr (kJobs) return SplitGrids{resident_grid(k_shade_plain_jobs<kAttr>, 256), heavy};
+        else return SplitGrids{resident_grid(k_shade_plain<kAttr>, 256), heavy};
+    }();
     return g;
 }
 template <bool kAttr, bool kJobs>
@@ -1270,8 +1333,11 @@ static int launch_split_shading(const DevScene& s, const PathParams& pp, const D
                                 PathSoA out, ShadowSoA sq, HeavyQueue hq, DevCounters* ctr,
                                 const uint32_t* n_active, float* film, double* film64, bool heavy, cudaStream_t st) {
     const SplitGrids g = split_grids<kAttr, kJobs>();
-    k_shade_plain<kAttr, kJobs><<<std::min(g.plain, grid_for(cap, 256)), 256, 0, st>>>(s, pp, jobs, in, out, sq, hq, ctr,
-                                                                                n_active, film, film64);
+    const unsigned plain = std::min(g.plain, grid_for(cap, 256));
+    if constexpr (kJobs)
+        k_shade_plain_jobs<kAttr><<<plain, 256, 0, st>>>(jobs, in, out, sq, hq, ctr, n_active);
+    else
+        k_shade_plain<kAttr><<<plain, 256, 0, st>>>(s, pp, in, out, sq, hq, ctr, n_active, film, film64);
     if (!heavy) return 1;
     k_shade_heavy<kAttr, kJobs><<<std::min(g.heavy, grid_for(cap, kHeavyThreads)), kHeavyThreads, 0, st>>>(
         s, pp, jobs, in, out, sq, hq, ctr, film, film64);
