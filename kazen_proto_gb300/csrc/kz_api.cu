@@ -357,7 +357,8 @@ constexpr uint32_t kBothCap = 1u << 23;
 // 115.5 / 126.1 ms, slit room 1024 x 1024, 16 spp 22.1 / 23.0, materials 641 x
 // 359, 16 spp 6.95 / 7.16, box 256 x 256, 16 spp 0.81 / 0.83, guided 512 x 512, 8
 // spp 4.90 / 5.02, but preview 97 x 65, 4 spp 0.75 / 0.69: eight pixels of so
-// small an image meet too many boxes.
+// small an image meet too many boxes. What bundles lose in small images of fine
+// scenes at more samples is bounded by kBundleWork (kz_traverse.cuh).
 constexpr uint32_t kBundleSpp = 8;
 // The queue of split shading for wavefronts large enough for it (else none).
 kz_status alloc_heavy(kz_scene* s, uint32_t cap, kz::HeavyQueue& q) {

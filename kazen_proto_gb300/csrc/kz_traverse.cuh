@@ -966,6 +966,21 @@ __device__ __forceinline__ int warp_traverse(const DevScene& s, const TRay& r, f
 // the results are the same bits. Camera rays of the 1080p terrain frame, 64 spp:
 // 15 nodes and 7 triangles a bundle in 6 steps, where each ray alone visits 11
 // and tests 4; 22.5 -> 15.8 ms, of which some 3 write the paths' state.
+//
+// That holds while the rays of a bundle stay together. In an image whose pixels
+// are coarse against the scene (a small image, or a scene seen from afar) a
+// bundle's beam covers thousands of triangles, of which each ray meets a few; so
+// a bundle that has taken kBundleWork steps and triangle tests gives up, and its
+// rays are traced each on its own lane. Frames of depth 5 through the 2.2 M
+// triangle terrain, ms, without a limit / 32 / 64 / 128 / without bundles: 64 x
+// 64, 8 spp 13.41 / 0.39 / 0.40 / 0.42 / 0.34, 256 x 256, 64 spp 8.35 / 3.06 / 3.14
+// / 3.20 / 2.92, 960 x 540, 8 spp from 200 times as far 257.6 / 0.59 / 0.60 / 0.64
+// / 0.54, 1080p, 64 spp 101.9 / 102.9 / 101.4 / 101.2 / 112.3.
+
+#ifndef KZ_BUNDLE_WORK
+#define KZ_BUNDLE_WORK 64
+#endif
+constexpr uint32_t kBundleWork = KZ_BUNDLE_WORK;
 
 // Smallest and largest of a float over the warp (no NaN).
 __device__ __forceinline__ float warp_min(float v) {
@@ -979,8 +994,8 @@ __device__ __forceinline__ float warp_max(float v) {
 
 // Closest hits of the warp's rays, all from r.o with r.tmin, unbounded. Lanes
 // without a ray pass live = false and a copy of another lane's ray. False if
-// the stack was too small (nothing is set then); on an abort (as closest_step)
-// the rays miss and *aborted is set.
+// the bundle gave up or the stack was too small (nothing is set then); on an
+// abort (as closest_step) the rays miss and *aborted is set.
 __device__ __forceinline__ bool warp_bundle(const DevScene& s, const TRay& r, bool live, uint2* stack, WarpRay& h,
                                             bool& aborted) {
     const uint32_t lane = threadIdx.x & 31u, up = 3u - (lane >> 3), lt = (1u << lane) - 1u;
@@ -1005,10 +1020,11 @@ __device__ __forceinline__ bool warp_bundle(const DevScene& s, const TRay& r, bo
     h.rec = -1;
     aborted = false;
     float tcur = inf;
-    uint32_t sp = 1, visits = 0;
+    uint32_t sp = 1, visits = 0, work = 0;
     if (lane == 0) stack[0] = make_uint2(0u, __float_as_uint(r.tmin));
     __syncwarp();
     while (sp) {
+        if (++work > kBundleWork) return false;
         const uint32_t n = (int)sp > kWarpStack - 32 && kWarpStack > 32 ? 1u : min(sp, 4u);
         visits += n;
         const uint2 e = up < n ? stack[sp - 1u - up] : make_uint2(0u, 0u);
@@ -1070,6 +1086,7 @@ __device__ __forceinline__ bool warp_bundle(const DevScene& s, const TRay& r, bo
                 aborted = true;
                 break;
             }
+            work += count;
             for (uint32_t k = first; k < first + count; ++k) {
                 const float4* tp = s.tris + (size_t)k * 3;
                 const float4 a = __ldg(tp), b = __ldg(tp + 1), c = __ldg(tp + 2);
