@@ -246,7 +246,9 @@ namespace {
 
 // A host call of so few rays goes through mapped pinned memory: the kernel reads
 // the rays and writes the hits there itself, in place of a copy from pageable
-// memory and up to five back to it, each of which the host waits for.
+// memory and up to five back to it, each of which the host waits for. A call that
+// fails leaves the caller's arrays alone: what lies in the buffer then may be an
+// earlier call's (a stack overflow is none: its rays are stored as misses).
 constexpr uint64_t kFewHost = 1024;
 constexpr size_t kFewBytes = sizeof(kz_ray) + 5 * 4;  // ray, t, prim, geom, u, v
 static_assert(kFewHost <= kz::kFewRays, "few host rays take the kernel that needs no fetch counter");
@@ -1095,6 +1097,7 @@ kz_status kz_intersect_closest(kz_scene* s, const kz_ray* rays, uint64_t n, kz_h
                                      s->status.as<uint32_t>(), st);
         KZ_CUDA(cudaGetLastError());
         const kz_status rc = sync_and_status(s);
+        if (rc != KZ_OK && rc != KZ_ERR_STACK) return rc;
         void* to[5] = {hits.t, hits.prim_id, hits.geom_id, hits.u, hits.v};
         for (int k = 0; k < 5; ++k)
             if (to[k]) std::memcpy(to[k], s->few_host + at + k * step, step);
@@ -1151,6 +1154,7 @@ kz_status kz_intersect_any(kz_scene* s, const kz_ray* rays, uint64_t n, uint8_t*
                                  s->status.as<uint32_t>(), st);
         KZ_CUDA(cudaGetLastError());
         const kz_status rc = sync_and_status(s);
+        if (rc != KZ_OK && rc != KZ_ERR_STACK) return rc;
         std::memcpy(occluded, s->few_host + at, n);
         return rc;
     }
