@@ -180,7 +180,8 @@ typedef struct kz_render_config {
     uint32_t spp;            /* samples per pixel                              */
     uint32_t max_depth;      /* maximum number of shaded path vertices         */
     uint64_t seed;           /* PCG32 seed; stream = pixel * spp + sample      */
-    uint32_t wavefront_size; /* paths in flight; 0 = KZ_RENDER_DEFAULT_WAVEFRONT */
+    uint32_t wavefront_size; /* paths in flight at most; 0 = KZ_RENDER_DEFAULT_WAVEFRONT
+                              * (kz_render_guided: see there)               */
     uint32_t rr_min_depth;   /* first vertex index that plays roulette (ref: 3) */
     uint32_t block_size;     /* threads per block of the stage kernels: 0 (= 256)
                               * or a multiple of 32 up to 256 (the kernels are
@@ -400,7 +401,12 @@ kz_status kz_guide_forward(kz_guide* guide, const float* points, uint64_t n, flo
 kz_status kz_guide_train_step(kz_guide* guide, const float* samples, uint64_t n, float learning_rate,
                               int32_t apply, float* out_loss, float* out_grad, int32_t mem);
 /* Guided render (same film contract as kz_render). cfg->spp is the target;
- * gcfg->time_budget_ms may stop it earlier (gstats->spp_done says where). */
+ * gcfg->time_budget_ms may stop it earlier (gstats->spp_done says where).
+ * cfg->wavefront_size 0: a pass (width * height * spp_per_pass paths) is in
+ * flight at once, up to KZ_RENDER_DEFAULT_WAVEFRONT paths; with the network
+ * frozen, up to 2^22 paths of several spp where a pass has fewer. A path in
+ * flight takes 352 bytes of device memory (192 of state, 160 of network
+ * outputs), 1.5 GB for 2^22. */
 kz_status kz_render_guided(kz_scene* scene, kz_guide* guide, const kz_camera* camera,
                            const kz_film_desc* film, const kz_render_config* cfg,
                            const kz_guide_config* gcfg, float* out_rgb, double* out_rgb64,

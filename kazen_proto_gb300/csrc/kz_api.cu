@@ -1622,11 +1622,15 @@ kz_status kz_guide_train_step(kz_guide* g, const float* samples, uint64_t n, flo
     return KZ_OK;
 }
 
-// Paths in flight of a guided render by default: each holds the network's 40
-// outputs (160 bytes) besides its path state. Frozen passes used to hold one
-// spp of the frame; at 512 x 512, 8 spp, depth 10 that is eight waves of 2^18,
-// 44 iterations and 8.1 ms, against one of 2^21, 10 iterations and 5.1 ms (4.5
-// with camera bundles and the present inference).
+// Paths in flight of a guided render by default: a pass is one wave up to
+// KZ_RENDER_DEFAULT_WAVEFRONT paths, and a frozen render fills a wave of
+// kGuidedWavefront with several spp where its own pass is smaller. Each path
+// holds the network's 40 outputs (160 bytes) besides its state of 192 bytes, so
+// a full wave of 2^22 takes 1.5 GB. At 512 x 512, 8 spp, depth 10, one spp at a
+// time is eight waves of 2^18, 44 iterations and 8.1 ms, one of 2^21 takes 10
+// iterations and 5.1 ms (4.5 with camera bundles and the present inference). A
+// pass above 2^22 paths as one wave / cut into waves of 2^22: 2304 x 2048, depth 6,
+// one frozen spp 12.1 / 12.5 ms, two training passes of one spp 30.2 / 31.1 ms.
 constexpr uint64_t kGuidedWavefront = 1ull << 22;
 
 kz_status kz_render_guided(kz_scene* s, kz_guide* g, const kz_camera* camera, const kz_film_desc* fd,
@@ -1674,7 +1678,9 @@ kz_status kz_render_guided(kz_scene* s, kz_guide* g, const kz_camera* camera, co
     }
     KZ_CUDA(cudaMemsetAsync(film, 0, npix * 12, strm));
     if (film64) KZ_CUDA(cudaMemsetAsync(film64, 0, npix * 24, strm));
-    const uint64_t want = cfg->wavefront_size ? cfg->wavefront_size : kGuidedWavefront;
+    const uint64_t want = cfg->wavefront_size ? cfg->wavefront_size
+                                              : std::min<uint64_t>(KZ_RENDER_DEFAULT_WAVEFRONT,
+                                                                   std::max(kGuidedWavefront, per_pass));
     const uint64_t n_recs = per_pass * cfg->max_depth;
     if (gc.train) {
         KZ_TRY(g->recs.ensure(n_recs * sizeof(kz::VRec)));
