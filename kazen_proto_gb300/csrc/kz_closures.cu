@@ -17,6 +17,13 @@
 // take 1.8 us a thousand, of the others 0.07). The lobes themselves stay out of
 // the tile: with them in it two blocks fit an SM instead of four, and fewer
 // searches were in flight (717 us; 860 with the searches last).
+//
+// A tile of one kind is not sorted, and its results go straight to memory. A
+// batch of one kind then takes as long as in an ungrouped kernel up to 311,296
+// queries, and 1.05 to 1.25 times as long above (plain ones 0.8 to 0.95 times):
+// the tile's barriers and staging, and four queries a thread. GGX glass, 262,144
+// queries, both calls: 105 -> 83 us (80 ungrouped); principled specular, 4,000,000:
+// 483 -> 461 (395).
 #include "kz_stages.cuh"
 
 namespace kz {
@@ -60,9 +67,10 @@ __device__ __forceinline__ bool next_queries(Tile& t, uint32_t m, uint32_t& k) {
     return first < m;
 }
 
-// Loads the tile's m queries and groups them by kind.
+// Loads the tile's m queries and groups them by kind; false if all are of one
+// kind, whose order is then not written.
 template <int kItems>
-__device__ __forceinline__ void load_tile(ClosureTile<kItems>& t, const kz_lobe* lobes, const float* a, const float* b,
+__device__ __forceinline__ bool load_tile(ClosureTile<kItems>& t, const kz_lobe* lobes, const float* a, const float* b,
                                           uint64_t first, uint32_t m) {
     const uint32_t tid = threadIdx.x;
     for (uint32_t k = tid; k < 3 * m; k += kClosureThreads) {
@@ -73,15 +81,18 @@ __device__ __forceinline__ void load_tile(ClosureTile<kItems>& t, const kz_lobe*
     if (tid == 0) t.next = 0u;
     __syncthreads();
     uint32_t kind[kItems], rank[kItems];
+    const uint32_t kind0 = closure_kind(lobes[first].closure_id, lobes[first].params[0]);
+    bool same = true;
 #pragma unroll
     for (int j = 0; j < kItems; ++j) {
         const uint32_t q = tid + j * kClosureThreads;
         if (q < m) {
             kind[j] = closure_kind(lobes[first + q].closure_id, lobes[first + q].params[0]);
             rank[j] = atomicAdd(&t.count[kind[j]], 1u);
+            same &= kind[j] == kind0;
         }
     }
-    __syncthreads();
+    if (__syncthreads_and(same)) return false;
     if (tid < kKinds) {  // exclusive prefix over the kinds (the first warp)
         const uint32_t c = t.count[tid];
         uint32_t incl = c;
@@ -99,6 +110,7 @@ __device__ __forceinline__ void load_tile(ClosureTile<kItems>& t, const kz_lobe*
         if (q < m) t.order[t.count[kind[j]] + rank[j]] = (uint16_t)q;
     }
     __syncthreads();
+    return true;
 }
 
 __device__ __forceinline__ void put3(float* p, f3 v) {
@@ -116,7 +128,18 @@ __global__ void __launch_bounds__(kClosureThreads, kClosureBlocks) k_closure_eva
     ClosureTile<kItems>& t = *reinterpret_cast<ClosureTile<kItems>*>(smem_raw);
     const uint64_t first = (uint64_t)blockIdx.x * t.kN;
     const uint32_t m = (uint32_t)min((uint64_t)t.kN, n - first);
-    load_tile(t, lobes, wi, wo, first, m);
+    if (!load_tile(t, lobes, wi, wo, first, m)) {
+#pragma unroll 1
+        for (uint32_t q = threadIdx.x; q < m; q += kClosureThreads) {
+            const uint64_t i = first + q;
+            const kz_lobe& l = lobes[i];
+            const f3 a = ld3(t.a + 3 * q), b = ld3(t.b + 3 * q);
+            const LobeEval e = conv == KZ_CONVENTION_REFERENCE ? lobe_eval_reference<true>(l, a, b) : lobe_eval(l, a, b);
+            put3(f + 3 * i, e.f);
+            pdf[i] = e.pdf;
+        }
+        return;
+    }
     for (uint32_t k; next_queries(t, m, k);) {
         if (k >= m) continue;
         const uint32_t q = t.order[k];
@@ -140,7 +163,19 @@ __global__ void __launch_bounds__(kClosureThreads, kClosureBlocks) k_closure_sam
     ClosureTile<kItems>& t = *reinterpret_cast<ClosureTile<kItems>*>(smem_raw);
     const uint64_t first = (uint64_t)blockIdx.x * t.kN;
     const uint32_t m = (uint32_t)min((uint64_t)t.kN, n - first);
-    load_tile(t, lobes, wi, u, first, m);
+    if (!load_tile(t, lobes, wi, u, first, m)) {
+#pragma unroll 1
+        for (uint32_t q = threadIdx.x; q < m; q += kClosureThreads) {
+            const uint64_t i = first + q;
+            const kz_lobe& l = lobes[i];
+            const LobeSample s = lobe_sample(l, ld3(t.a + 3 * q), t.b[3 * q], t.b[3 * q + 1], t.b[3 * q + 2]);
+            put3(wo + 3 * i, s.wo);
+            put3(weight + 3 * i, s.weight);
+            pdf[i] = s.pdf;
+            flags[i] = (uint8_t)((s.valid ? 1 : 0) | (s.delta ? 2 : 0));
+        }
+        return;
+    }
     for (uint32_t k; next_queries(t, m, k);) {
         if (k >= m) continue;
         const uint32_t q = t.order[k];
@@ -162,14 +197,25 @@ __global__ void __launch_bounds__(kClosureThreads, kClosureBlocks) k_closure_sam
     }
 }
 
-// Queries per thread, 1, 2 or 4: a tile of 1,024 holds about 45 of each of 23
-// kinds, more than a warp, but a batch should also spread over the SMs.
-// Evaluation and sampling of 21 kinds / of five principled ones at 1 / 2 / 4
-// (and ungrouped): 16,000 queries 119 / 118 / 119 (168) and 40 / 41 / 50 us
-// (41), 80,000: 158 / 151 / 143 (463) and 43 / 43 / 50 (48), 320,000: 432 / 262
-// / 203 (1,591) and 70 / 61 / 56 (84), 1,000,000: 1,528 / 954 / 483 (5,453) and
-// 152 / 123 / 113 (185).
-int items_per_thread(uint64_t n) { return n < (1u << 16) ? 1 : n < (1u << 18) ? 2 : 4; }
+// Queries per thread, 1, 2 or 4: as few as keep all tiles of a batch resident at
+// once (kClosureBlocks an SM), four above that. A larger tile holds more of each
+// kind, but leaves fewer warps to wait for their lobes, which is all that a batch
+// of one kind does. Evaluation and sampling at 1 / 2 / 4 (and ungrouped), us a pair
+// of calls: 21 kinds, 65,536 queries 169 / 150 / 139 (408), 100,000 170 / 170 / 156
+// (541), 200,000 287 / 195 / 191 (1,027), 262,144 342 / 212 / 200 (1,265), 600,000
+// 858 / 514 / 272 (3,161); one kind (GGX glass) 100,000 55 / 68 / 94 (59), 262,144
+// 77 / 83 / 102 (80), 600,000 120 / 125 / 127 (121); five principled kinds 100,000
+// 51 / 53 / 56 (62), 600,000 100 / 80 / 73 (131). (Lines at 2^16 and 2^18 queries
+// made batches of one kind up to 1.3 times as slow as ungrouped.)
+int items_per_thread(uint64_t n) {
+    static const uint64_t wave = [] {
+        int dev = 0, sms = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        return (uint64_t)(sms > 0 ? sms : 1) * kClosureBlocks * kClosureThreads;
+    }();
+    return n <= wave ? 1 : n <= 2 * wave ? 2 : 4;
+}
 
 template <int kItems>
 void run_eval(const kz_lobe* lobes, const float* wi, const float* wo, uint64_t n, int conv, float* f, float* pdf,

@@ -1,0 +1,70 @@
+"""Closure batches whose tiles hold one kind: such a tile is not sorted. Every
+query's result is the one it has among queries of other kinds (a sorted tile),
+bit for bit: batches of one kind, with one other query at a tile's first, last
+and middle place, at the sizes where the tile grows (one query a thread while
+all tiles are resident, then two, then four: 155,648 and 311,296 queries on 152
+SMs). And a batch of one kind takes no longer, against a smaller one, than it
+is larger; with four queries a thread from 2^18 on it did."""
+import time
+
+import numpy as np
+import pytest
+
+from kazen_proto_gb300 import _native as N
+from kazen_proto_gb300 import api
+from test_gpu_closures import N_KINDS, dirs, lobe_grid
+
+pytestmark = pytest.mark.gpu
+
+
+def results(lobes, wi, wo, u):
+    return [*api.closure_eval(lobes, wi, wo, N.KZ_CONVENTION_INTEGRATOR),
+            *api.closure_eval(lobes, wi, wo, N.KZ_CONVENTION_REFERENCE), *api.closure_sample(lobes, wi, u)]
+
+
+@pytest.mark.parametrize("n", [1, 33, 256, 257, 155648, 155649, 311296, 311297])
+@pytest.mark.parametrize("other", [None, 0, 255, 256, -1])
+@pytest.mark.parametrize("kind", [0, 4, 6])
+def test_one_kind_matches_mixed(gpu, n, other, kind):
+    rng = np.random.default_rng(n)
+    base = lobe_grid(rng, 40 * N_KINDS)
+    lobes = base[kind::N_KINDS][rng.integers(0, 40, n)]
+    if other is not None and other < n:
+        lobes[other] = base[(kind + 1) % N_KINDS]
+    wi, wo, u = dirs(rng, n), dirs(rng, n), rng.random((n, 3)).astype(np.float32)
+    whole = results(lobes, wi, wo, u)
+    at = np.unique(np.concatenate([np.arange(0, n, max(1, n // 300)), [min(255, n - 1), min(256, n - 1), n - 1]]))
+    for k in range(0, len(at), 100):
+        p = at[k:k + 100]
+        more = rng.integers(0, len(base), len(p))  # as many of other kinds, in between
+        mix = np.empty(2 * len(p), base.dtype)
+        mix[0::2], mix[1::2] = lobes[p], base[more]
+        piece = results(mix, np.repeat(wi[p], 2, 0), np.repeat(wo[p], 2, 0), np.repeat(u[p], 2, 0))
+        for a, b in zip(whole, piece):
+            assert a[p].tobytes() == b[0::2].tobytes()
+
+
+def test_time_of_one_kind_follows_its_size(gpu):
+    import ctypes as C
+
+    import torch
+    rng = np.random.default_rng(1)
+    n = 1 << 18
+    one = np.repeat(api.microfacet("ggx", 0.3, eta=1.5, refract=1)[None], n)
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a).view(np.float32).reshape(n, -1)).cuda()  # noqa: E731
+    lobes, wi, u = dev(one), dev(dirs(rng, n)), dev(rng.random((n, 3)).astype(np.float32))
+    wo, w, pdf, fl = (torch.empty(n * k, device="cuda") for k in (3, 3, 1, 1))
+    p = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
+
+    def us(m):
+        t = []
+        for _ in range(60):
+            torch.cuda.synchronize()
+            t0 = time.perf_counter()
+            N.check(N.lib().kz_closure_sample_batch(p(lobes), p(wi), p(u), m, p(wo), p(w), p(pdf), p(fl),
+                                                    N.KZ_MEM_DEVICE))
+            torch.cuda.synchronize()
+            t.append(time.perf_counter() - t0)
+        return sorted(t)[len(t) // 4] * 1e6
+
+    assert us(n) <= us(200000) * n / 200000
