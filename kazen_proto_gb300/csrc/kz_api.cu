@@ -210,13 +210,14 @@ struct kz_scene {
     std::vector<float> point_lights;  // 6 floats each: position, radiance
     DevBuf d_tri_uv, d_mat_tex, d_textures, d_texels, d_tri_nrm;
     kz::DevScene dev;
-    DevBuf status;        // uint32 device status word for batch calls
+    DevBuf status;        // uint32 device status word for batch calls; the fetch counter of calls on rays behind it
     uint32_t* status_host = nullptr;  // pinned; the few-ray buffer lies behind it
     unsigned char* few_host = nullptr;  // kFewHost rays and their results (host pointer, and the device's)
     unsigned char* few_dev = nullptr;
 
     // batch scratch (host-memory calls)
-    DevBuf s_rays, s_t, s_prim, s_geom, s_u, s_v, s_occ, s_ctr, s_next;
+    DevBuf s_rays, s_t, s_prim, s_geom, s_u, s_v, s_occ, s_ctr;
+    unsigned long long* fetch_counter() const { return status.as<unsigned long long>() + 16; }
 
     // wavefront buffers
     DevBuf pa[5], pb[5], sh[3], heavy, ctr, film, film64;
@@ -230,7 +231,7 @@ struct kz_scene {
         cudaSetDevice(device);
         if (stream) cudaStreamSynchronize(stream);
         DevBuf* all[] = {&nodes, &tris, &geom_offset, &geom_light, &mats, &mat_class, &mat_plain, &lights, &light_cdf,
-                         &light_tris, &status, &s_rays, &s_t, &s_prim, &s_geom, &s_u, &s_v, &s_occ, &s_ctr, &s_next,
+                         &light_tris, &status, &s_rays, &s_t, &s_prim, &s_geom, &s_u, &s_v, &s_occ, &s_ctr,
                          &heavy, &ctr, &film, &film64, &d_tri_uv, &d_mat_tex, &d_textures, &d_texels, &d_tri_nrm};
         for (DevBuf* b : all) b->release();
         for (auto& b : pa) b.release();
@@ -251,7 +252,7 @@ namespace {
 // earlier call's (a stack overflow is none: its rays are stored as misses).
 constexpr uint64_t kFewHost = 1024;
 constexpr size_t kFewBytes = sizeof(kz_ray) + 5 * 4;  // ray, t, prim, geom, u, v
-static_assert(kFewHost <= kz::kFewRays, "few host rays take the kernel that needs no fetch counter");
+static_assert(kFewHost <= kz::kFewRaysTiny, "few host rays take the kernel that needs no fetch counter");
 
 template <typename T>
 kz_status upload(DevBuf& b, const std::vector<T>& v, cudaStream_t st) {
@@ -532,7 +533,7 @@ kz_status init_cuda(kz_scene* s) {
     KZ_CUDA(cudaHostGetDevicePointer((void**)&s->few_dev, s->status_host, 0));
     s->few_dev += 64;
     if (!s->stream) s->stream = s->own_stream;
-    KZ_TRY(s->status.ensure(sizeof(uint32_t)));
+    KZ_TRY(s->status.ensure(256));
     KZ_CUDA(cudaMemset(s->status.ptr, 0, sizeof(uint32_t)));
     return KZ_OK;
 }
@@ -1103,12 +1104,9 @@ kz_status kz_intersect_closest(kz_scene* s, const kz_ray* rays, uint64_t n, kz_h
             if (to[k]) std::memcpy(to[k], s->few_host + at + k * step, step);
         return rc;
     }
-    if (n > kz::kFewRays) {
-        KZ_TRY(s->s_next.ensure(sizeof(unsigned long long)));
-        KZ_CUDA(cudaMemsetAsync(s->s_next.ptr, 0, sizeof(unsigned long long), st));
-    }
+    if (n > kz::few_rays(s->dev)) KZ_CUDA(cudaMemsetAsync(s->fetch_counter(), 0, sizeof(unsigned long long), st));
     if (mem == KZ_MEM_DEVICE) {
-        kz::launch_intersect_closest(s->dev, rays, n, hits, s->s_next.as<unsigned long long>(),
+        kz::launch_intersect_closest(s->dev, rays, n, hits, s->fetch_counter(),
                                      s->status.as<uint32_t>(), st);
         KZ_CUDA(cudaGetLastError());
         return KZ_OK;
@@ -1122,7 +1120,7 @@ kz_status kz_intersect_closest(kz_scene* s, const kz_ray* rays, uint64_t n, kz_h
     KZ_CUDA(cudaMemcpyAsync(s->s_rays.ptr, rays, n * sizeof(kz_ray), cudaMemcpyHostToDevice, st));
     kz_hits dh{s->s_t.as<float>(), s->s_prim.as<uint32_t>(), hits.geom_id ? s->s_geom.as<uint32_t>() : nullptr,
                hits.u ? s->s_u.as<float>() : nullptr, hits.v ? s->s_v.as<float>() : nullptr};
-    kz::launch_intersect_closest(s->dev, s->s_rays.as<kz_ray>(), n, dh, s->s_next.as<unsigned long long>(),
+    kz::launch_intersect_closest(s->dev, s->s_rays.as<kz_ray>(), n, dh, s->fetch_counter(),
                                  s->status.as<uint32_t>(), st);
     KZ_CUDA(cudaGetLastError());
     KZ_CUDA(cudaMemcpyAsync(hits.t, dh.t, n * 4, cudaMemcpyDeviceToHost, st));
@@ -1158,12 +1156,9 @@ kz_status kz_intersect_any(kz_scene* s, const kz_ray* rays, uint64_t n, uint8_t*
         std::memcpy(occluded, s->few_host + at, n);
         return rc;
     }
-    if (n > kz::kFewRays) {
-        KZ_TRY(s->s_next.ensure(sizeof(unsigned long long)));
-        KZ_CUDA(cudaMemsetAsync(s->s_next.ptr, 0, sizeof(unsigned long long), st));
-    }
+    if (n > kz::few_rays(s->dev)) KZ_CUDA(cudaMemsetAsync(s->fetch_counter(), 0, sizeof(unsigned long long), st));
     if (mem == KZ_MEM_DEVICE) {
-        kz::launch_intersect_any(s->dev, rays, n, occluded, s->s_next.as<unsigned long long>(),
+        kz::launch_intersect_any(s->dev, rays, n, occluded, s->fetch_counter(),
                                  s->status.as<uint32_t>(), st);
         KZ_CUDA(cudaGetLastError());
         return KZ_OK;
@@ -1172,7 +1167,7 @@ kz_status kz_intersect_any(kz_scene* s, const kz_ray* rays, uint64_t n, uint8_t*
     KZ_TRY(s->s_occ.ensure(n));
     KZ_CUDA(cudaMemcpyAsync(s->s_rays.ptr, rays, n * sizeof(kz_ray), cudaMemcpyHostToDevice, st));
     kz::launch_intersect_any(s->dev, s->s_rays.as<kz_ray>(), n, s->s_occ.as<uint8_t>(),
-                             s->s_next.as<unsigned long long>(), s->status.as<uint32_t>(), st);
+                             s->fetch_counter(), s->status.as<uint32_t>(), st);
     KZ_CUDA(cudaGetLastError());
     KZ_CUDA(cudaMemcpyAsync(occluded, s->s_occ.ptr, n, cudaMemcpyDeviceToHost, st));
     return sync_and_status(s);
@@ -1813,7 +1808,7 @@ extern "C" kz_status kz_scene_release_scratch(kz_scene* s) {
     if (!s->cuda_ready) return KZ_OK;
     KZ_CUDA(cudaSetDevice(s->device));
     KZ_CUDA(cudaStreamSynchronize(s->stream));
-    DevBuf* all[] = {&s->s_rays, &s->s_t, &s->s_prim, &s->s_geom, &s->s_u, &s->s_v, &s->s_occ, &s->s_ctr, &s->s_next,
+    DevBuf* all[] = {&s->s_rays, &s->s_t, &s->s_prim, &s->s_geom, &s->s_u, &s->s_v, &s->s_occ, &s->s_ctr,
                      &s->heavy, &s->film, &s->film64};
     for (DevBuf* b : all) b->release();
     for (auto& b : s->pa) b.release();

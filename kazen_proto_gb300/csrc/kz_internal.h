@@ -210,6 +210,14 @@ struct BatchCounters {
 // 4,000 51 / 127, 16,000 88 / 127, 32,000 138 / 152; through 2,000 triangles 27 /
 // 41, 27 / 40, 43 / 42, 63 / 44.
 constexpr uint64_t kFewRays = 16384;
+// Calls on rays through a handful of triangles: there a lane's ray takes a few
+// steps, and all rays up to 20,000 the same time. Closest hits, a warp a ray / a
+// lane a ray, calls back to back: 36 triangles, 4,000 rays 8.3 / 10.2 us, 8,192 12.4
+// / 14.6, 12,288 14.5 / 14.7, 16,384 18.6 / 11.4; 12 triangles 8,192 8.5 / 8.5, 16,384
+// 12.5 / 8.4; 100 triangles 16,384 16.0 / 12.4, but 300 triangles 18.6 / 16.5.
+constexpr uint64_t kFewRaysTiny = 8192;
+constexpr uint32_t kTinyScene = 128;  // triangles
+inline uint64_t few_rays(const DevScene& s) { return s.n_tris <= kTinyScene ? kFewRaysTiny : kFewRays; }
 // Nodes as the builder writes them to the layout the traversal reads, in place.
 void launch_pack_nodes(uint4* nodes, uint32_t n, cudaStream_t st);
 // `next` is a zeroed 64-bit fetch counter for the persistent kernel.

@@ -328,7 +328,7 @@ void launch_pack_nodes(uint4* nodes, uint32_t n, cudaStream_t st) {
 void launch_intersect_closest(const DevScene& s, const kz_ray* rays, uint64_t n, kz_hits hits,
                               unsigned long long* next, uint32_t* status, cudaStream_t st) {
     if (!n) return;
-    if (n <= kFewRays) {
+    if (n <= few_rays(s)) {
         k_intersect_few<false><<<grid_for(n, kFewWarps), 32 * kFewWarps, 0, st>>>(s, rays, (uint32_t)n, hits, nullptr,
                                                                                  status);
         return;
@@ -341,7 +341,7 @@ void launch_intersect_closest(const DevScene& s, const kz_ray* rays, uint64_t n,
 void launch_intersect_any(const DevScene& s, const kz_ray* rays, uint64_t n, uint8_t* occ,
                           unsigned long long* next, uint32_t* status, cudaStream_t st) {
     if (!n) return;
-    if (n <= kFewRays) {
+    if (n <= few_rays(s)) {
         k_intersect_few<true><<<grid_for(n, kFewWarps), 32 * kFewWarps, 0, st>>>(s, rays, (uint32_t)n, kz_hits{}, occ,
                                                                                 status);
         return;
