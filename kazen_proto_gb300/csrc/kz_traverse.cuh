@@ -783,13 +783,18 @@ constexpr uint32_t kAnyRefill = KZ_ANY_REFILL;
 // A queue that does not fill the grid: blocks beyond its share leave at once
 // (256 rays a block, but 8 a block, one a warp, while that leaves SMs without
 // one), and of each warp only the first ceil(n / warps) lanes take rays; the
-// others help with the leaf tests. 64 rays through 20,000 triangles took 131 us
-// in one block and 114 in eight, but 65,537 Li rays 600 us over all resident
-// blocks against 540 over 257: there the warps' steps, not the longest ray, are
-// waited for.
+// others help with the leaf tests. Reached by calls of more rays than take a warp
+// each, by stage timing and fetch counting, and by wavefronts above 2^23 paths.
+// With / without the spread: 16,385 closest hits through 250,000 triangles 148 / 169
+// us, 20,000 through a 525,000-triangle terrain 73 / 83, through 36 triangles 28 / 34
+// (any hits, 12,288); 32 x 32 x 4 paths of depth 5 with stage timing 0.49 / 0.57 ms,
+// counted 0.52 / 0.72. Rays over all resident blocks instead: 65,537 Li rays 600 us
+// against 540 over 257 blocks, since the warps' steps, not the longest ray, are
+// waited for there.
+constexpr uint32_t kSpreadBlocks = 152;  // the SMs of a GB300: a rule of speed only
 template <typename Ctr>
 __host__ __device__ __forceinline__ uint32_t trace_blocks(Ctr n, uint32_t most) {
-    const Ctr full = (n + 255) / 256, spread = n < 8 * 152 ? (n + 7) / 8 : 152;
+    const Ctr full = (n + 255) / 256, spread = n < 8 * kSpreadBlocks ? (n + 7) / 8 : kSpreadBlocks;
     const Ctr want = full > spread ? full : spread;
     return want < most ? (uint32_t)want : most;
 }
