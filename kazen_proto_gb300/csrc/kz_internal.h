@@ -232,8 +232,6 @@ void launch_closure_eval(const kz_lobe* lobes, const float* wi, const float* wo,
 void launch_closure_sample(const kz_lobe* lobes, const float* wi, const float* u, uint64_t n,
                            float* wo, float* weight, float* pdf, uint8_t* flags, cudaStream_t st);
 
-void launch_generate_camera(const DevCamera& cam, const PathParams& pp, PathSoA dst, uint32_t dst_offset,
-                            uint64_t first_path, uint32_t n_new, uint32_t block, cudaStream_t st);
 void launch_generate_rays(const kz_ray* rays, const PathParams& pp, PathSoA dst, uint32_t dst_offset,
                           uint64_t first_path, uint32_t n_new, uint32_t block, cudaStream_t st);
 void launch_trace_paths(const DevScene& s, PathSoA p, uint32_t n, DevCounters* ctr, bool count, uint32_t block,

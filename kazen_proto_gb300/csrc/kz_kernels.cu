@@ -8,13 +8,6 @@
 namespace kz {
 namespace {
 
-__global__ void k_generate_camera(DevCamera cam, PathParams pp, PathSoA dst, uint32_t dst_offset,
-                                  uint64_t first_path, uint32_t n_new) {
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n_new) return;
-    generate_camera_path(cam, pp, dst, dst_offset + j, first_path + j);
-}
-
 __global__ void k_generate_rays(const kz_ray* __restrict__ rays, PathParams pp, PathSoA dst, uint32_t dst_offset,
                                 uint64_t first_path, uint32_t n_new) {
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
@@ -93,11 +86,6 @@ __global__ void k_scale(float* film, double* film64, uint64_t n, float sf, doubl
 
 }  // namespace
 
-void launch_generate_camera(const DevCamera& cam, const PathParams& pp, PathSoA dst, uint32_t dst_offset,
-                            uint64_t first_path, uint32_t n_new, uint32_t block, cudaStream_t st) {
-    if (!n_new) return;
-    k_generate_camera<<<grid_for(n_new, block), block, 0, st>>>(cam, pp, dst, dst_offset, first_path, n_new);
-}
 void launch_generate_rays(const kz_ray* rays, const PathParams& pp, PathSoA dst, uint32_t dst_offset,
                           uint64_t first_path, uint32_t n_new, uint32_t block, cudaStream_t st) {
     if (!n_new) return;

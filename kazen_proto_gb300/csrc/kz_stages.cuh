@@ -931,8 +931,6 @@ __device__ __forceinline__ void plan_iteration(DevCounters* c, uint32_t cap, boo
     c->n_append = 0;
     c->trace_next = 0;
     c->shadow_next = 0;
-    c->heavy_next = 0;
-    for (int k = 0; k < kHeavyClasses; ++k) c->heavy[k] = 0;
     if (c->n_active) {
         c->iterations += 1;
         c->path_bounces += c->n_active;

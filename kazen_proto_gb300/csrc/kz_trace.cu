@@ -90,10 +90,8 @@ __global__ void k_intersect_stats(DevScene s, const kz_ray* __restrict__ rays, u
 }
 
 template <bool kCount>
-__global__ void __launch_bounds__(256) k_trace_paths(DevScene s, PathSoA p, uint32_t n, DevCounters* ctr,
-                                                     const uint32_t* n_dev) {
+__global__ void __launch_bounds__(256) k_trace_paths(DevScene s, PathSoA p, uint32_t n, DevCounters* ctr) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n_dev) n = *n_dev;
     uint32_t dn = 0, dt = 0;
     if (i < n) {
         const float4 o = p.o4[i], d = p.d4[i];
@@ -268,9 +266,9 @@ __global__ void __launch_bounds__(32 * kFewWarps) k_intersect_few(DevScene s, co
     }
 }
 
-template <bool kCount, bool kGuided>
+template <bool kCount>
 __global__ void __launch_bounds__(256) k_trace_shadow(DevScene s, ShadowSoA sq, DevCounters* ctr, float* film,
-                                                      double* film64, VRec* recs, NRec* nee, uint32_t max_depth) {
+                                                      double* film64) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t dn = 0, dt = 0;
     if (i < ctr->queue.shadow) {
@@ -279,16 +277,7 @@ __global__ void __launch_bounds__(256) k_trace_shadow(DevScene s, ShadowSoA sq, 
         bool overflow;
         const bool occluded = trace_any<kCount>(s, r, o.w, overflow, dn, dt);
         if (overflow) set_status(&ctr->status, KZ_ERR_STACK);
-        if (!occluded && !overflow) {
-            const float4 c = sq.c4[i];
-            film_add(film, film64, __float_as_uint(d.w), xyz(c));
-            if (kGuided && recs) {
-                const uint32_t tag = __float_as_uint(c.w);
-                const uint64_t rb = (uint64_t)(tag >> 4) * max_depth;
-                propagate(recs, rb, tag & 15u, xyz(c));
-                if (nee) nee[rb + (tag & 15u)].n.w = 1.f;
-            }
-        }
+        if (!occluded && !overflow) film_add(film, film64, __float_as_uint(d.w), xyz(sq.c4[i]));
     }
     if (kCount) warp_count(dn, dt, &ctr->fetch[2]);
 }
@@ -360,8 +349,8 @@ void launch_intersect_stats(const DevScene& s, const kz_ray* rays, uint64_t n, u
 void launch_trace_paths(const DevScene& s, PathSoA p, uint32_t n, DevCounters* ctr, bool count, uint32_t block,
                         cudaStream_t st) {
     if (!n) return;
-    if (count) k_trace_paths<true><<<grid_for(n, block), block, 0, st>>>(s, p, n, ctr, nullptr);
-    else k_trace_paths<false><<<grid_for(n, block), block, 0, st>>>(s, p, n, ctr, nullptr);
+    if (count) k_trace_paths<true><<<grid_for(n, block), block, 0, st>>>(s, p, n, ctr);
+    else k_trace_paths<false><<<grid_for(n, block), block, 0, st>>>(s, p, n, ctr);
 }
 
 void launch_camera_bundles(const DevScene& s, const DevCamera& cam, const PathParams& pp, PathSoA p,
@@ -419,12 +408,8 @@ void launch_trace_shadow_dev(const DevScene& s, ShadowSoA sq, uint32_t n_max, De
 void launch_trace_shadow(const DevScene& s, ShadowSoA sq, uint32_t n_max, DevCounters* ctr, bool count, float* film,
                          double* film64, uint32_t block, cudaStream_t st) {
     if (!n_max) return;
-    if (count)
-        k_trace_shadow<true, false><<<grid_for(n_max, block), block, 0, st>>>(s, sq, ctr, film, film64, nullptr,
-                                                                              nullptr, 0);
-    else
-        k_trace_shadow<false, false><<<grid_for(n_max, block), block, 0, st>>>(s, sq, ctr, film, film64, nullptr,
-                                                                               nullptr, 0);
+    if (count) k_trace_shadow<true><<<grid_for(n_max, block), block, 0, st>>>(s, sq, ctr, film, film64);
+    else k_trace_shadow<false><<<grid_for(n_max, block), block, 0, st>>>(s, sq, ctr, film, film64);
 }
 
 static unsigned grid_trace_batch() {
