@@ -977,13 +977,14 @@ __device__ __forceinline__ int warp_traverse(const DevScene& s, const TRay& r, f
 // bundle's beam covers thousands of triangles, of which each ray meets a few; so
 // a bundle that has taken kBundleWork steps and triangle tests gives up, and its
 // rays are traced each on its own lane. Frames of depth 5 through the 2.2 M
-// triangle terrain, ms, without a limit / 32 / 64 / 128 / without bundles: 64 x
-// 64, 8 spp 13.41 / 0.39 / 0.40 / 0.42 / 0.34, 256 x 256, 64 spp 8.35 / 3.06 / 3.14
-// / 3.20 / 2.92, 960 x 540, 8 spp from 200 times as far 257.6 / 0.59 / 0.60 / 0.64
-// / 0.54, 1080p, 64 spp 101.9 / 102.9 / 101.4 / 101.2 / 112.3.
-
+// triangle terrain, ms, without a limit / 64 / 128 / 192 / without bundles: 8 x 8, 8
+// spp 234 / 0.29 / 0.33 / 0.34 / 0.22, 64 x 64, 8 spp 13.41 / 0.40 / 0.42 / 0.46 / 0.34,
+// 512 x 512, 8 spp 2.70 / 1.93 / 2.00 / 2.02 / 1.79, 960 x 540, 8 spp from 200 times as
+// far 257.6 / 0.60 / 0.64 / 0.67 / 0.54, 1080p, 8 spp 13.46 / 13.62 / 13.50 / 13.45 /
+// 14.65, 64 spp 101.9 / 101.4 / 101.2 / 100.8 / 112.3. 641 x 359, 16 spp of mixed
+// materials: 7.46 / 7.49 / 7.46 / 7.46.
 #ifndef KZ_BUNDLE_WORK
-#define KZ_BUNDLE_WORK 64
+#define KZ_BUNDLE_WORK 192
 #endif
 constexpr uint32_t kBundleWork = KZ_BUNDLE_WORK;
 
