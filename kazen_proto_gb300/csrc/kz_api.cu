@@ -383,12 +383,14 @@ struct GuideHooks {
 // host enqueues batches of iterations (generate, trace, [infer], shade) and
 // synchronises once per batch. An iteration's shadow rays are traced beside
 // the next one's paths, in one launch, in wavefronts up to kBothCap; in larger
-// ones, and with stage timing or fetch counts, they have their own. Contributions are summed into film (and film64) on the device.
+// ones, and with stage timing or fetch counts, they have their own. Contributions
+// are summed into film (and film64) on the device.
 //
 // When all paths fit into the wavefront at once, only the first iteration
 // generates, a path has at most max_depth vertices, and so max_depth iterations
 // are enough: one batch, one synchronisation. The 256 x 256, 16 spp box frame
-// of depth 5 takes 18 launches and 0.82 ms; with two waves' worth of iterations
+// of depth 5 takes 16 launches (bundles, four joint traces, five times two shading
+// kernels, the last shadow rays) and 0.82 ms; with two waves' worth of iterations
 // and planning kernels between them it took 84 and 1.20 ms.
 kz_status run_wavefront(kz_scene* s, const kz::DevCamera* cam, const kz_ray* rays_dev, uint64_t total,
                         const kz_render_config* cfg, float* film, double* film64, kz_render_stats* stats,
@@ -446,7 +448,10 @@ kz_status run_wavefront(kz_scene* s, const kz::DevCamera* cam, const kz_ray* ray
     std::vector<uint8_t> generated(batch);
     for (bool first_batch = true;; first_batch = false) {
         const NvtxRange batch_range("wavefront batch");
-        if (!first_batch) kz::launch_carry(ctr, batch + 1, ctr + batch, ctr + batch, strm);
+        if (!first_batch) {
+            kz::launch_carry(ctr, batch + 1, ctr + batch, ctr + batch, strm);
+            st.kernel_launches += 1;
+        }
         const kz::DevCounters* last_gen = ctr;
         for (uint32_t it = 0; it < batch; ++it) {
             cudaEvent_t* e = timing ? &ev[5 * (size_t)it] : nullptr;
