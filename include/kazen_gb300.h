@@ -190,7 +190,13 @@ typedef struct kz_render_config {
 } kz_render_config;
 
 /* Record CUDA events around every stage launch (on the scene stream) and
- * report per-stage device time in kz_render_stats. */
+ * report per-stage device time in kz_render_stats. Stages have launches of
+ * their own then: a wavefront of up to 2^23 paths, whose shadow rays are
+ * otherwise traced beside the next iteration's paths in one launch, takes one
+ * launch more per iteration and traces few rays a lane each, not a warp each
+ * (a frame of 1,000 to 40,000 paths then takes 1.2 to 2.7 times as long); larger
+ * wavefronts run as they do without the flag. Where camera paths are generated
+ * and traced in one kernel (8 samples per pixel or more), both count as tracing. */
 #define KZ_RENDER_FLAG_TIMING 1u
 /* Trace with the fetch-counting traversal variant and report BVH node and
  * triangle fetches (slower; for roofline accounting, not for timing). */
@@ -209,7 +215,7 @@ typedef struct kz_render_stats {
     uint64_t shadow_rays;    /* any-hit rays traced for next-event estimation  */
     uint64_t iterations;     /* wavefront iterations                           */
     uint64_t paths;          /* camera paths started                           */
-    uint64_t kernel_launches;/* kernels launched by the call                   */
+    uint64_t kernel_launches;/* kernels launched by the path loop (the film's scaling not counted) */
     /* KZ_RENDER_FLAG_COUNT: fetches of 80-byte nodes / 48-byte triangles */
     uint64_t closest_node_fetches, closest_tri_fetches;
     uint64_t shadow_node_fetches, shadow_tri_fetches;
@@ -497,9 +503,10 @@ kz_status kz_scene_release_scratch(kz_scene* scene);
  *     returns after the work has finished on the scene stream.
  *   - The host waits for the stream after every wavefront iteration (it
  *     reads the queue counts to size the next launches), where kz_li_batch
- *     lets the device drive the loop and waits once per 2 x (max_depth + 1)
- *     iterations: for the same rays this call is slower, more so for small
- *     batches whose iterations are short. */
+ *     lets the device drive the loop and waits once for rays that fit its
+ *     wavefront, else once per 2 x (max_depth + 1) iterations: for the same
+ *     rays this call is slower, more so for small batches whose iterations
+ *     are short. */
 #define KZ_LI_NOALLOC_MAX_WAVEFRONT 16384u
 kz_status kz_li_batch_noalloc(kz_scene* scene, const kz_ray* rays, uint64_t n,
                               const kz_render_config* cfg, float* out_rgb,
