@@ -751,14 +751,21 @@ def run_ours(args):
         e2e_bounces += r.last_stats["path_bounces"]
     e_units, e_secs = aggregate(e2e_bounces, e2e_s, dist)
 
-    # fetch counts for the roofline: one counted frame at reduced spp (untimed,
-    # after the timed region so profiler launch indices are unaffected)
-    cnt = api.Renderer(spp=max(1, w["spp"] // 16), max_depth=w["max_depth"], seed=seed,
-                       wavefront_size=w["wavefront"], flags=N.KZ_RENDER_FLAG_COUNT)
-    cnt.render(s, desc.camera, W, H, device_out=(rgb, None))
-    cs = cnt.last_stats
-    nodes_per_ray = cs["closest_node_fetches"] / max(1, cs["path_bounces"])
-    tris_per_ray = cs["closest_tri_fetches"] / max(1, cs["path_bounces"])
+    # The roofline's kernel traces the rays after the camera's: those are traced
+    # in bundles, by a kernel that also generates them. Its time is the trace
+    # stage's less that of frames of depth 1, its fetches those of a counted frame
+    # at reduced spp less those of depth 1 (untimed, after the timed region so
+    # profiler launch indices are unaffected).
+    def stats_of(**kw):
+        k = api.Renderer(seed=seed, wavefront_size=w["wavefront"], **kw)
+        k.render(s, desc.camera, W, H, device_out=(rgb, None))
+        return k.last_stats
+    camera_ms = min(stats_of(spp=w["spp"], max_depth=1, flags=N.KZ_RENDER_FLAG_TIMING)["trace_ms"] for _ in range(3))
+    cs, c1 = (stats_of(spp=max(1, w["spp"] // 16), max_depth=d, flags=N.KZ_RENDER_FLAG_COUNT)
+              for d in (w["max_depth"], 1))
+    counted_rays = max(1, cs["path_bounces"] - c1["path_bounces"])
+    nodes_per_ray = (cs["closest_node_fetches"] - c1["closest_node_fetches"]) / counted_rays
+    tris_per_ray = (cs["closest_tri_fetches"] - c1["closest_tri_fetches"]) / counted_rays
 
     sections = {}
 
@@ -795,8 +802,8 @@ def run_ours(args):
     if rank != 0:
         return
     peak, peak_kind = measured_peaks()
-    trace_ms_frame = stage["trace_ms"] / args.steps
-    rays_frame = bounces / args.steps
+    trace_ms_frame = stage["trace_ms"] / args.steps - camera_ms
+    rays_frame = bounces / args.steps - W * H * w["spp"]
     alg_bytes_ray = 32 + 16 + NODE_BYTES * nodes_per_ray + 48 * tris_per_ray
     alg_bytes_frame = alg_bytes_ray * rays_frame
     achieved = alg_bytes_frame / (trace_ms_frame / 1e3) / 1e9
@@ -835,9 +842,11 @@ def run_ours(args):
                      "peak_source": peak_kind + " (MEASURED_PEAKS.json hbm_gbs)" if peak_kind == "measured" else peak_kind,
                      "alg_bytes_per_ray": round(alg_bytes_ray, 1),
                      "node_fetches_per_ray": round(nodes_per_ray, 2), "tri_fetches_per_ray": round(tris_per_ray, 2),
-                     "note": "achieved/frac count algorithmic bytes = 32 B ray + 16 B hit + 80 B per 8-wide node fetch "
-                             "+ 48 B per triangle fetch; node/triangle fetches are served mostly from L1/L2, so the "
-                             "kernel is issue- and divergence-bound (see limiter), not HBM-bound"},
+                     "note": "rays after the camera's (camera rays are traced in bundles by a kernel of their own; "
+                             "its time, from frames of depth 1, is taken off the trace stage); achieved/frac count "
+                             "algorithmic bytes = 32 B ray + 16 B hit + 80 B per 8-wide node fetch + 48 B per "
+                             "triangle fetch; node/triangle fetches are served mostly from L1/L2, so the kernel is "
+                             "issue- and divergence-bound (see limiter), not HBM-bound"},
         "stages_ms_per_frame": {k: round(v / args.steps, 3) for k, v in stage.items()},
         "mrays_per_s": round((bounces + shadow) / (total_ms / 1e3) / 1e6, 2),
         "gpu_launches": launches,
