@@ -11,12 +11,14 @@
 // query's own inputs. Values are those of the ungrouped kernel, bit for bit.
 //
 // 1,000,003 queries over 21 kinds (221 bytes each over both calls, 33 us at
-// the measured copy rate), evaluation and sampling: 5,450 -> 480 us, 110 of it
-// evaluation. Bound by FP64: the Beckmann slope search of one query in ten, on
-// an FP64 rate of two lanes a clock and SM (queries of Beckmann lobes alone
-// take 1.8 us a thousand, of the others 0.07). The lobes themselves stay out of
-// the tile: with them in it two blocks fit an SM instead of four, and fewer
-// searches were in flight (717 us; 860 with the searches last).
+// the measured copy rate), evaluation and sampling: 5,450 -> 490 us, 87 of it
+// evaluation. Bound by instruction fetch (21 branches, a few warps in each at a
+// time: 13 % of the issue slots busy in sampling) and by the wait of every tile
+// for its Beckmann slope searches, one query in ten; not by FP64 throughput, nor
+// by memory: Beckmann queries alone (1.8 us a thousand) and the others alone
+// (0.07) add up to some 235 us. The lobes themselves stay out of the tile: with
+// them in it two blocks fit an SM instead of four, and fewer searches were in
+// flight (717 us; 860 with the searches last).
 //
 // A tile of one kind is not sorted, and its results go straight to memory. A
 // batch of one kind then takes as long as in an ungrouped kernel up to 311,296
