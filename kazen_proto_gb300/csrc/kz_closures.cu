@@ -20,12 +20,12 @@
 // them in it two blocks fit an SM instead of four, and fewer searches were in
 // flight (717 us; 860 with the searches last).
 //
-// A tile of one kind is not sorted, and its results go straight to memory. A
-// batch of one kind then takes as long as in an ungrouped kernel up to 311,296
-// queries, and 1.05 to 1.25 times as long above (plain ones 0.8 to 0.95 times):
-// the tile's barriers and staging, and four queries a thread. GGX glass, 262,144
-// queries, both calls: 105 -> 83 us (80 ungrouped); principled specular, 4,000,000:
-// 483 -> 461 (395).
+// A tile of one kind, or of few queries, is not sorted, and its results go
+// straight to memory. A batch of one kind then takes as long as in an ungrouped
+// kernel up to 311,296 queries, and 1.1 to 1.25 times as long above a million
+// (diffuse ones 0.85 to 0.95 times): the tile's barriers and staging, and four
+// queries a thread. GGX glass, 262,144 queries, both calls: 105 -> 82 us (80
+// ungrouped); principled specular, 4,000,000: 484 -> 463 (395).
 #include "kz_stages.cuh"
 
 namespace kz {
@@ -55,7 +55,7 @@ struct ClosureTile {
     float a[kN * 3], b[kN * 3], pdf[kN];
     uint16_t order[kN];
     uint8_t flags[kN];
-    uint32_t count[kKinds], next;
+    uint32_t count[kKinds], start[kKinds], kind0, next;
 };
 
 // The warps of a block take the sorted queries 32 at a time; returns the
@@ -69,12 +69,18 @@ __device__ __forceinline__ bool next_queries(Tile& t, uint32_t m, uint32_t& k) {
     return first < m;
 }
 
-// Loads the tile's m queries and groups them by kind; false if all are of one
-// kind, whose order is then not written.
+// Loads the tile's m queries and groups them by kind. False, with no order
+// written, if they are all of one kind or at most kUnsorted: three warps are too
+// few to hold a kind each, and a short call is as long as its barriers. Evaluation
+// and sampling of 21 kinds sorted / unsorted (and in an ungrouped kernel): 48
+// queries 137 / 114 us (115), 65 129 / 116 (118), 96 131 / 121 (124), but six
+// microfacet kinds and diffuse 112 112 / 127 (129), 128 108 / 131 (133).
+constexpr uint32_t kUnsorted = 96;
 template <int kItems>
 __device__ __forceinline__ bool load_tile(ClosureTile<kItems>& t, const kz_lobe* lobes, const float* a, const float* b,
                                           uint64_t first, uint32_t m) {
     const uint32_t tid = threadIdx.x;
+    uint32_t kind[kItems], rank[kItems];
     for (uint32_t k = tid; k < 3 * m; k += kClosureThreads) {
         t.a[k] = __ldg(a + 3 * first + k);
         t.b[k] = __ldg(b + 3 * first + k);
@@ -82,19 +88,18 @@ __device__ __forceinline__ bool load_tile(ClosureTile<kItems>& t, const kz_lobe*
     if (tid < kKinds) t.count[tid] = 0u;
     if (tid == 0) t.next = 0u;
     __syncthreads();
-    uint32_t kind[kItems], rank[kItems];
-    const uint32_t kind0 = closure_kind(lobes[first].closure_id, lobes[first].params[0]);
-    bool same = true;
+    if (m <= kUnsorted) return false;
 #pragma unroll
     for (int j = 0; j < kItems; ++j) {
         const uint32_t q = tid + j * kClosureThreads;
         if (q < m) {
             kind[j] = closure_kind(lobes[first + q].closure_id, lobes[first + q].params[0]);
             rank[j] = atomicAdd(&t.count[kind[j]], 1u);
-            same &= kind[j] == kind0;
         }
     }
-    if (__syncthreads_and(same)) return false;
+    if (tid == 0) t.kind0 = kind[0];
+    __syncthreads();
+    if (t.count[t.kind0] == m) return false;
     if (tid < kKinds) {  // exclusive prefix over the kinds (the first warp)
         const uint32_t c = t.count[tid];
         uint32_t incl = c;
@@ -103,13 +108,13 @@ __device__ __forceinline__ bool load_tile(ClosureTile<kItems>& t, const kz_lobe*
             const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, o);
             if (tid >= o) incl += v;
         }
-        t.count[tid] = incl - c;
+        t.start[tid] = incl - c;
     }
     __syncthreads();
 #pragma unroll
     for (int j = 0; j < kItems; ++j) {
         const uint32_t q = tid + j * kClosureThreads;
-        if (q < m) t.order[t.count[kind[j]] + rank[j]] = (uint16_t)q;
+        if (q < m) t.order[t.start[kind[j]] + rank[j]] = (uint16_t)q;
     }
     __syncthreads();
     return true;
