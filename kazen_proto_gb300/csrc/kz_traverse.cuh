@@ -975,14 +975,16 @@ __device__ __forceinline__ int warp_traverse(const DevScene& s, const TRay& r, f
 // That holds while the rays of a bundle stay together. In an image whose pixels
 // are coarse against the scene (a small image, or a scene seen from afar) a
 // bundle's beam covers thousands of triangles, of which each ray meets a few; so
-// a bundle that has taken kBundleWork steps and triangle tests gives up, and its
-// rays are traced each on its own lane. Frames of depth 5 through the 2.2 M
-// triangle terrain, ms, without a limit / 64 / 128 / 192 / without bundles: 8 x 8, 8
-// spp 234 / 0.29 / 0.33 / 0.34 / 0.22, 64 x 64, 8 spp 13.41 / 0.40 / 0.42 / 0.46 / 0.34,
-// 512 x 512, 8 spp 2.70 / 1.93 / 2.00 / 2.02 / 1.79, 960 x 540, 8 spp from 200 times as
-// far 257.6 / 0.60 / 0.64 / 0.67 / 0.54, 1080p, 8 spp 13.46 / 13.62 / 13.50 / 13.45 /
-// 14.65, 64 spp 101.9 / 101.4 / 101.2 / 100.8 / 112.3. 641 x 359, 16 spp of mixed
-// materials: 7.46 / 7.49 / 7.46 / 7.46.
+// a bundle gives up, and its rays are traced each on its own lane, once its steps
+// and triangle tests and four times the entries on its stack exceed kBundleWork
+// (a wide beam is told by its stack before it has spent the work). Frames of depth
+// 5, ms, without a limit / work alone up to 64 / up to 192 / this / without bundles:
+// 2.2 M triangle terrain 8 x 8, 8 spp 230 / 0.29 / 0.35 / 0.32 / 0.22, 64 x 64, 8 spp
+// 13.6 / 0.40 / 0.46 / 0.43 / 0.35, 512 x 512, 8 spp 2.65 / 1.93 / 2.03 / 2.00 / 1.79,
+// 960 x 540, 8 spp from 20 times as far 18.0 / 0.67 / 0.73 / 0.66 / 0.59, 1080p, 8 spp
+// 13.44 / 13.63 / 13.49 / 13.49 / 14.64, 64 spp of depth 8 98.2 / 98.8 / 98.5 / 98.5 /
+// 109.5; slit room 64 x 64, 8 spp 0.463 / - / 0.473 / 0.465 / 0.400; mixed materials
+// 641 x 359, 16 spp 7.46 / 7.50 / 7.46 / 7.46 / 7.74.
 #ifndef KZ_BUNDLE_WORK
 #define KZ_BUNDLE_WORK 192
 #endif
@@ -1030,7 +1032,7 @@ __device__ __forceinline__ bool warp_bundle(const DevScene& s, const TRay& r, bo
     if (lane == 0) stack[0] = make_uint2(0u, __float_as_uint(r.tmin));
     __syncwarp();
     while (sp) {
-        if (++work > kBundleWork) return false;
+        if (++work + 4u * sp > kBundleWork) return false;
         const uint32_t n = (int)sp > kWarpStack - 32 && kWarpStack > 32 ? 1u : min(sp, 4u);
         visits += n;
         const uint2 e = up < n ? stack[sp - 1u - up] : make_uint2(0u, 0u);
